@@ -10,7 +10,7 @@
 // small islands are short of parallel work, so islands overlap). Then either
 // form screens them:
 //
-// * pruned (every island admits the tensor-core pruning bound and clears the
+// * pruned (every island admits the pruning bound and clears the
 //   pruning floor): each island's pruning screen (csx_prune.cuh) runs over the
 //   whole GPU in turn, with its own shared memory and grid, waiting only for
 //   its own island's items, and writes its CTA lists into the island's area;
@@ -384,12 +384,14 @@ struct IslandBufs {
     uint64_t *ck = nullptr;
     SegOut *so = nullptr;
     uint32_t *off = nullptr;
+    PairBufs pairs;  // pruned batch
 };
 
 struct BatchLayout {
     int n = 0;
     std::vector<Plan> pl;
     std::vector<csx_cfg> cfg;
+    std::vector<csx_model> model;
     std::vector<int> ne;
     std::vector<IslandBufs> b;
     bool fast = true, filter = true;
@@ -427,6 +429,7 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
     L->n = n;
     L->pl.assign(n, Plan{});
     L->cfg.assign(cfgs, cfgs + n);
+    L->model.assign(models, models + n);
     L->ne.assign(n_elites, n_elites + n);
     L->b.assign(n, IslandBufs{});
     int ne_max = 0;
@@ -453,22 +456,21 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
                            tune ? tune->seg_cands : 0);
         if (rc) return rc;
         items_sum += L->pl[i].items_cap;
-        L->prune = L->prune && L->pl[i].prune_ok && L->pl[i].prune_tc;
+        L->prune = L->prune && L->pl[i].prune_ok;
     }
     if (items_sum >= 0xFFFFFFFFull) return CSX_ERR_LIMIT;
 
     int per_sm = 0;
     const int cap = tune && tune->ctas_per_sm > 0 ? static_cast<int>(tune->ctas_per_sm) : 3;
     if (L->prune) {
-        // every island's pruning screen with the tensor-core bound, one after
-        // another, each with its own shared memory and up to three CTAs per SM
+        // every island's pruning screen, one after another, each with its own shared memory and up to three CTAs per SM
         // (as the single screen); the lists are laid out for the widest grid
         L->smem = 0;
         for (int i = 0; i < n; ++i) {
             if (cfgs[i].lambda == 0) continue;
             Plan &pl = L->pl[i];
-            pl.el_smem = prune_el_smem(pl.sort_n, n_elites[i], pl.nb, cx.num_sms, true, cx.max_smem);
-            pl.smem = prune_smem(pl.sort_n, n_elites[i], pl.nb, cx.num_sms, true, pl.el_smem);
+            pl.el_smem = prune_el_smem(pl.sort_n, n_elites[i], cx.num_sms, cx.max_smem);
+            pl.smem = prune_smem(pl.sort_n, n_elites[i], cx.num_sms, pl.el_smem);
             if (pl.smem + 1024 > cx.max_smem) return CSX_ERR_LIMIT;
             const int fit = std::min(cap, std::max(1, static_cast<int>((228u << 10) / (pl.smem + 1024))));
             pl.grid = fit * cx.num_sms;
@@ -476,9 +478,9 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
             per_sm = std::max(per_sm, fit);
         }
         per_sm = std::max(per_sm, 1);
-        for (int nb : {16, kNtot})
-            CSX_CUDA(cudaFuncSetAttribute(screen_p_fn(nb, true, true, false),
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L->smem)));
+        for (bool tail : {false, true})
+            CSX_CUDA(cudaFuncSetAttribute(screen_p_fn(tail, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(L->smem)));
     } else {
         L->smem = screen_smem(L->sort_n, ne_max, L->filter);
         if (L->smem + 2048 > cx.max_smem) return CSX_ERR_LIMIT;
@@ -521,6 +523,8 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
             b.ids = cv.take<unsigned long long>(static_cast<size_t>(n_elites[i]));
             b.tribes = cv.take<unsigned int>(static_cast<size_t>(n_elites[i]));
             if (cfgs[i].lambda == 0) continue;
+            if (L->prune)
+                b.pairs = pair_bufs(cv.take<unsigned char>(pair_bytes(n_elites[i], pl.tail)), n_elites[i], pl.tail);
             b.items = cv.take<Item>(pl.items_cap);
             if (!pl.short_path) {
                 b.recs = cv.take<SegRec>(pl.g.n_seg);
@@ -574,14 +578,9 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
             if (cfgs[i].lambda == 0) continue;
             const Plan &pl = L->pl[i];
             const IslandBufs &b = L->b[i];
-            PruneArgs &P = L->pargs[i];
-            static_cast<ScreenArgs &>(P) = screen_args(cfgs[i], models[i], make_synth(cfgs[i], n_elites[i]), pl,
-                                                       b.tab, b.items, b.ctrl, b.la);
-            P.pc = pl.pc;
-            P.tc = pl.ptc;
-            P.pub = L->pub;
-            P.sel_cap = 8u * static_cast<uint32_t>(cx.num_sms);
-            P.el_smem = pl.el_smem ? 1u : 0u;
+            L->pargs[i] = prune_args(screen_args(cfgs[i], models[i], make_synth(cfgs[i], n_elites[i]), pl, b.tab,
+                                                 b.items, b.ctrl, b.la),
+                                     pl, b.pairs, L->pub, cx.num_sms);
         }
     }
     return CSX_OK;
@@ -613,6 +612,10 @@ int batch_enqueue(Context &cx, const BatchLayout &L, cudaStream_t st, bool captu
         ++nk;
         if (L.cfg[i].lambda > 0) {
             const SynthConst sc = make_synth(L.cfg[i], ne);
+            if (L.prune) {
+                const int rc = enqueue_pairs(L.model[i], pl.pc, pl.lam, ne, pl.tail, b.tab, b.pairs, a, &nk);
+                if (rc) return rc;
+            }
             const int rc = enqueue_items(sc, pl, b.recs, b.ck, b.so, b.off, b.items, b.ctrl, a, &nk);
             if (rc) return rc;
         }
@@ -627,7 +630,7 @@ int batch_enqueue(Context &cx, const BatchLayout &L, cudaStream_t st, bool captu
             if (L.cfg[i].lambda == 0) continue;
             const Plan &pl = L.pl[i];
             CSX_CUDA(cudaMemsetAsync(L.pub, 0, static_cast<size_t>(kPruneMs) * pl.grid * sizeof(uint32_t), st));
-            screen_p_fn(pl.nb, true, true, false)<<<pl.grid, kThreads, pl.smem, st>>>(L.pargs[i]);
+            screen_p_fn(pl.tail, false)<<<pl.grid, kThreads, pl.smem, st>>>(L.pargs[i]);
             CSX_CUDA(cudaGetLastError());
             ++nk;
         }

@@ -85,7 +85,7 @@ struct Context {
     bool timed = false;
     csx_run_info info{};
     DevBuf genomes, tab, ids, tribes, recs, ck, segout, off, items, lists_a, lists_b, ctrl, surv,
-        result, pub, tie_hits, tie_count, tie_streams, tie_out;
+        result, pub, pairs, tie_hits, tie_count, tie_streams, tie_out;
     // batched islands
     DevBuf batch, b_genomes, b_surv, b_result;
     void *pinned = nullptr;         // host staging of the island descriptors (page-locked)
@@ -150,11 +150,10 @@ struct Plan {
     JumpBound jb{};  // widening of err for a candidate with a jump (filter mode)
     bool prune = false;     // the pruning screen (csx_prune.cuh)
     bool prune_ok = false;  // its bound is certifiable for this call (the batch decides for itself)
-    bool prune_tc = false;  // its bound's gradient on the tensor cores
-    int nb = 16;            // crossover genes its bound draws
+    bool tail = false;      // some linear weight past gene 15 is nonzero
     bool el_smem = false;   // its elite table in shared memory (prune_el_smem)
+    uint64_t lam = 0;       // candidates of the streams this call screens
     PruneConst pc{};
-    PruneTc ptc{};
 };
 
 int context_init(Context &cx, int dev) {
@@ -285,15 +284,11 @@ void screen_shape(const csx_cfg &cfg, const csx_model &model, bool full, Plan *p
     pl->filter = !full && !(cfg.flags & CSX_FLAG_EXACT_ALL) && pl->err > 0.0f;
     // the pruning screen: the filter form's conditions, the fast delta form
     // (its mutation is within |sigma| of the parent gene by construction) and
-    // a certifiable bound. The precision form (TC flags) prunes with its tile
-    // format's bound and ranks in FP64; without a tensor-core bound it keeps
-    // its own unpruned kernel.
-    const uint32_t tcf = cfg.flags & (CSX_FLAG_TC_BF16 | CSX_FLAG_TC_FP16);
+    // a certifiable bound. The precision form (TC flags) prunes likewise and
+    // ranks in FP64; without a certifiable bound it keeps its own unpruned
+    // kernel.
     pl->prune = pl->filter && pl->fast_delta && !(cfg.flags & CSX_FLAG_NO_PRUNE) &&
-                make_prune(model, cfg.sigma, &pl->pc, &pl->nb);
-    pl->prune_tc = pl->prune && (tcf != 0 || !(cfg.flags & CSX_FLAG_PRUNE_FFMA)) &&
-                   make_prune_tc(model, pl->pc, tcf != CSX_FLAG_TC_BF16, &pl->ptc);
-    if (tcf && !pl->prune_tc) pl->prune = false;
+                make_prune(model, cfg.sigma, &pl->pc, &pl->tail);
     pl->kpad = list_kpad(cfg.keep);
     pl->sort_n = pow2_at_least(pl->kpad + 4ull * kThreads);
     pl->buf_cap = pl->sort_n - pl->kpad;
@@ -357,6 +352,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     const uint64_t my_max = std::max(g.per, g.my_last);
     const bool has_last = g.t0 + g.nT == g.T;
     const uint64_t lam_range = (g.nT - (has_last ? 1 : 0)) * g.per + (has_last ? g.my_last : 0);
+    pl->lam = lam_range;
     screen_shape(cfg, model, full != nullptr, pl);
     const uint32_t tcf = cfg.flags & (CSX_FLAG_TC_BF16 | CSX_FLAG_TC_FP16);
     if (tcf == (CSX_FLAG_TC_BF16 | CSX_FLAG_TC_FP16)) return CSX_ERR_BAD_ARGS;
@@ -373,8 +369,8 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     pl->prune_ok = pl->prune && lam_range >= min_prune;
     if (pl->prune_ok && grid_override == 0) {
         // the selection scratch holds one key per CTA: at most 8 CTAs of 256 threads per SM
-        pl->el_smem = prune_el_smem(pl->sort_n, ne, pl->nb, cx.num_sms, pl->prune_tc, cx.max_smem);
-        pl->smem = prune_smem(pl->sort_n, ne, pl->nb, cx.num_sms, pl->prune_tc, pl->el_smem);
+        pl->el_smem = prune_el_smem(pl->sort_n, ne, cx.num_sms, cx.max_smem);
+        pl->smem = prune_smem(pl->sort_n, ne, cx.num_sms, pl->el_smem);
         pl->prune = pl->smem + 1024 <= cx.max_smem;
     } else {
         pl->prune = false;
@@ -387,18 +383,8 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     if (grid_override > 0) {
         pl->grid = grid_override;
     } else if (pl->prune) {
-        int rc = screen_occupancy(screen_p_fn(pl->nb, pl->prune_tc, pl->fp16 || !pl->tc, pl->tc), cx.num_sms,
-                                  pl->smem, &pl->grid);
+        int rc = screen_occupancy(screen_p_fn(pl->tail, pl->tc), cx.num_sms, pl->smem, &pl->grid);
         if (rc) return rc;
-        // The occupancy query reports one CTA per SM for the tensor-core form;
-        // its registers (80 at three CTAs), shared memory (~65 KB each) and
-        // TMEM (32 columns each) hold three, which run 9% faster than two
-        // (measured). The screen is persistent with dynamic work, so any grid
-        // is correct.
-        if (pl->prune_tc) {
-            const int fit = static_cast<int>((228u << 10) / (pl->smem + 1024));  // 228 KB of shared memory per SM
-            pl->grid = std::max(pl->grid, std::min(3, std::max(1, fit)) * cx.num_sms);
-        }
     } else if (pl->tc) {
         // The occupancy query reports one CTA per SM for this kernel, yet three
         // are resident and run faster (80 registers, ~50 KB of shared memory,
@@ -552,6 +538,56 @@ int enqueue_merge(Entry *cur, Entry *nxt, uint32_t nl, uint32_t kpad, cudaStream
     return CSX_OK;
 }
 
+// Device scratch of the pair bounds: boxes, then u0, then (with a tail) tmax.
+struct PairBufs {
+    uint32_t *box = nullptr;
+    float *u0 = nullptr, *tmax = nullptr;
+};
+
+size_t pair_bytes(int ne, bool tail) {
+    const size_t n = static_cast<size_t>(ne);
+    return (n * 16 + n * n * (tail ? 2 : 1)) * sizeof(float);
+}
+
+PairBufs pair_bufs(void *base, int ne, bool tail) {
+    const size_t n = static_cast<size_t>(ne);
+    PairBufs b;
+    b.box = static_cast<uint32_t *>(base);
+    b.u0 = reinterpret_cast<float *>(b.box + n * 16);
+    b.tmax = tail ? b.u0 + n * n : nullptr;
+    return b;
+}
+
+int enqueue_pairs(const csx_model &m, const PruneConst &pc, uint64_t lambda, int ne, bool tail, const float *tab,
+                  const PairBufs &b, cudaStream_t st, uint32_t *launches) {
+    prune_box_kernel<<<(ne * 16 + 127) / 128, 128, 0, st>>>(tab, ne, pc.s, b.box);
+    CSX_CUDA(cudaGetLastError());
+    const PairArgs P = make_pair_args(m, pc, lambda, ne, tail, tab, b.box, b.u0, b.tmax);
+    const uint64_t threads = (static_cast<uint64_t>(ne) * ne) << P.tpp_log2;
+    pair_bound_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(P);
+    CSX_CUDA(cudaGetLastError());
+    *launches += 2;
+    return CSX_OK;
+}
+
+// The pruning screen's arguments past the plain screen's.
+PruneArgs prune_args(const ScreenArgs &A, const Plan &pl, const PairBufs &b, uint32_t *pub, int num_sms) {
+    PruneArgs P;
+    static_cast<ScreenArgs &>(P) = A;
+    P.pc = pl.pc;
+    P.box = b.box;
+    P.u0 = b.u0;
+    P.tmax = b.tmax;
+    P.pub = pub;
+    P.sel_cap = 8u * static_cast<uint32_t>(num_sms);
+    P.el_smem = pl.el_smem ? 1u : 0u;
+    P.bm_words = prune_bm_words(static_cast<int>(A.sc.ne));
+    // a rebuild reads the whole table once per CTA: every 8 rounds for 64
+    // elites (128 words), less often in proportion for more
+    P.bm_period = std::max<uint32_t>(8, pow2_at_least(P.bm_words / 16));
+    return P;
+}
+
 // Enqueue the whole pipeline on `st`. Device inputs: genomes (csx_genome x ne).
 int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_genome *d_genomes,
                    int ne, csx_survivor *d_out, unsigned long long *d_result, cudaStream_t st,
@@ -571,7 +607,12 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     const uint32_t nl = static_cast<uint32_t>(pl.grid);
     CSX_CUDA(cx.lists_a.ensure(static_cast<size_t>(nl) * pl.kpad * sizeof(Entry)));
     CSX_CUDA(cx.lists_b.ensure(static_cast<size_t>((nl + 1) / 2) * pl.kpad * sizeof(Entry)));
-    if (pl.prune) CSX_CUDA(cx.pub.ensure(static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t)));
+    PairBufs pairs;
+    if (pl.prune) {
+        CSX_CUDA(cx.pub.ensure(static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t)));
+        CSX_CUDA(cx.pairs.ensure(pair_bytes(ne, pl.tail)));
+        pairs = pair_bufs(cx.pairs.p, ne, pl.tail);
+    }
     if (!pl.short_path) {
         CSX_CUDA(cx.recs.ensure(g.n_seg * sizeof(SegRec)));
         CSX_CUDA(cx.ck.ensure(g.n_seg * g.ckcap * sizeof(uint64_t)));
@@ -601,6 +642,10 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
         d_genomes, ne, tab, ids, tribes);
     CSX_CUDA(cudaGetLastError());
     ++launches;
+    if (pl.prune) {
+        rc = enqueue_pairs(model, pl.pc, pl.lam, ne, pl.tail, tab, pairs, st, &launches);
+        if (rc) return rc;
+    }
     CSX_CUDA(mark(1));
 
     Item *items = static_cast<Item *>(cx.items.p);
@@ -617,14 +662,8 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
 
     const ScreenArgs A = screen_args(cfg, model, sc, pl, tab, items, ctrl, static_cast<Entry *>(cx.lists_a.p));
     if (pl.prune) {
-        PruneArgs P;
-        static_cast<ScreenArgs &>(P) = A;
-        P.pc = pl.pc;
-        P.tc = pl.ptc;
-        P.pub = static_cast<uint32_t *>(cx.pub.p);
-        P.sel_cap = 8u * static_cast<uint32_t>(cx.num_sms);
-        P.el_smem = pl.el_smem ? 1u : 0u;
-        screen_p_fn(pl.nb, pl.prune_tc, pl.fp16 || !pl.tc, pl.tc)<<<pl.grid, kThreads, pl.smem, st>>>(P);
+        const PruneArgs P = prune_args(A, pl, pairs, static_cast<uint32_t *>(cx.pub.p), cx.num_sms);
+        screen_p_fn(pl.tail, pl.tc)<<<pl.grid, kThreads, pl.smem, st>>>(P);
     } else if (pl.tc) {
         TcScreenArgs P;
         P.A = A;

@@ -142,36 +142,6 @@ struct TcGroup {
     bool issuer;
 };
 
-// Row `row` (0..127) of the group's X tile <- packed x; one MMA for the group;
-// y <- this thread's row of X L^T. All 128 threads of the group must call it.
-// Returns false when the MMA's completion wait gave up (y is then garbage).
-__device__ __forceinline__ bool tc_round(TcGroup &g, const uint32_t (&pk)[8], uint32_t row, float (&y)[16]) {
-    const uint32_t a = g.xs + (row >> 3) * 256u + (row & 7u) * 16u;
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
-                 : "memory");
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 128u), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]),
-                 "r"(pk[7])
-                 : "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc_fence_before();
-    // literal barrier ids: a register id makes ptxas reserve all 16 named barriers,
-    // which limits how many CTAs an SM holds
-    if (g.bar_id == 1)
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-    else
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-    if (g.issuer) {
-        tc_fence_after();
-        tc_mma(g.tmem_d, g.adesc, g.bdesc, g.idesc);
-        tc_commit(g.mbar);
-    }
-    const bool ok = mbar_wait(g.mbar, g.phase);
-    g.phase ^= 1u;
-    tc_fence_after();
-    tc_ld16(g.tmem_ld, y);
-    return ok;
-}
-
 }  // namespace csx
 
 namespace csx {
@@ -199,8 +169,11 @@ __device__ __forceinline__ void synth_tc(const TcModel &T, const SynthConst &C, 
     for (int j = 0; j < 8; ++j) pk[j] = pack2(x[2 * j], x[2 * j + 1], kFp16);
 }
 
-// One tensor-core round of a 128-thread group (tc_round with a give-up path
-// that keeps the group in step). gbad is the group's flag in
+// One tensor-core round of a 128-thread group: row `row` (0..127) of the
+// group's X tile <- packed x, one MMA for the group, y <- this thread's row of
+// X L^T. All 128 threads of the group must call it. The barrier ids are
+// literals: a register id makes ptxas reserve all 16 named barriers, which
+// limits how many CTAs an SM holds. gbad is the group's flag in
 // shared memory, written only by the group's threads, after their wait of a
 // round and before the next round's barrier: every thread of the group reads
 // the same value after that barrier, so once a wait has given up the whole

@@ -57,25 +57,25 @@ enum {
 #define CSX_FLAG_STAGE_TIMES 0x10u /* record per-stage device times (csx_last_run_info) */
 #define CSX_FLAG_TC_BF16 0x20u     /* precision form: survivors ranked by their FP64 score (rounded
                                       to f32): the FP64 top-K, genes bit-exact. By default the
-                                      pruning bound runs on BF16 tensor cores and the candidates it
-                                      cannot rule out are filtered by FFMA and scored in FP64; with
+                                      candidates the pruning bound cannot rule out are filtered by
+                                      FFMA and scored in FP64; with
                                       CSX_FLAG_NO_PRUNE the quadratic block of every candidate runs
                                       on the tensor cores and candidates within max(1e-3 relative,
                                       the form's certified error bound) of the K-th score are
                                       rescored in FP64. csx_screen / csx_screen_device */
 #define CSX_FLAG_TC_FP16 0x40u     /* the same with FP16 tiles (unpruned: x' = 2g - 1) */
 #define CSX_FLAG_NO_PRUNE 0x80u    /* score every candidate's full synthesis (the filter form)
-                                      instead of skipping, by a certified bound taken after the
-                                      crossover bits, candidates that cannot reach the top-K.
+                                      instead of skipping, by certified bounds taken from the parent
+                                      pair and after the crossover bits, candidates that cannot
+                                      reach the top-K.
                                       Results are identical either way; only speed differs.
                                       Without the flag the library prunes generations of at least
                                       400 candidates per screen thread (3 CTAs x 256 threads per
                                       SM: 4.67e7 on 152 SMs; below, the unpruned kernel is
                                       faster); the environment variable CSX_PRUNE_MIN_CANDS sets
                                       that floor in candidates */
-#define CSX_FLAG_PRUNE_FFMA 0x100u /* the pruning bound's gradient by FP32 FMA instead of the
-                                      tensor cores (FP16 tcgen05.mma with a certified error
-                                      share). Results are identical either way */
+#define CSX_FLAG_PRUNE_FFMA 0x100u /* the pruning bound's gradient by FP32 FMA: accepted, and what
+                                      the library does without it as well */
 
 /* Model: the flat weight layout of src/screen.zig:23-27. */
 typedef struct csx_model {
@@ -252,7 +252,7 @@ int csx_last_run_info(csx_run_info *out);
  * running brain/evolve.py with its own seed, elites and surrogate,
  * .github/workflows/arena.yml:56-92) in one pipeline: every island's work
  * items are built on its own forked stream; then, when every island's
- * surrogate admits the tensor-core pruning bound and every island is above
+ * surrogate admits the pruning bound and every island is above
  * the pruning floor (CSX_FLAG_NO_PRUNE), each island's pruning screen runs
  * over the whole GPU in turn, else (or when any island carries
  * CSX_FLAG_NO_PRUNE) ONE unpruned persistent screen launch consumes all
