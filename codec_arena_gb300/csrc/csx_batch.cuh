@@ -524,7 +524,8 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
             b.tribes = cv.take<unsigned int>(static_cast<size_t>(n_elites[i]));
             if (cfgs[i].lambda == 0) continue;
             if (L->prune)
-                b.pairs = pair_bufs(cv.take<unsigned char>(pair_bytes(n_elites[i], pl.tail)), n_elites[i], pl.tail);
+                b.pairs = pair_bufs(cv.take<unsigned char>(pair_bytes(pl.lam, n_elites[i], pl.tail)), pl.lam,
+                                    n_elites[i], pl.tail);
             b.items = cv.take<Item>(pl.items_cap);
             if (!pl.short_path) {
                 b.recs = cv.take<SegRec>(pl.g.n_seg);
@@ -580,7 +581,7 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
             const IslandBufs &b = L->b[i];
             L->pargs[i] = prune_args(screen_args(cfgs[i], models[i], make_synth(cfgs[i], n_elites[i]), pl, b.tab,
                                                  b.items, b.ctrl, b.la),
-                                     pl, b.pairs, L->pub, cx.num_sms);
+                                     models[i], pl, b.pairs, L->pub, cx.num_sms);
         }
     }
     return CSX_OK;
@@ -613,7 +614,7 @@ int batch_enqueue(Context &cx, const BatchLayout &L, cudaStream_t st, bool captu
         if (L.cfg[i].lambda > 0) {
             const SynthConst sc = make_synth(L.cfg[i], ne);
             if (L.prune) {
-                const int rc = enqueue_pairs(L.model[i], pl.pc, pl.lam, ne, pl.tail, b.tab, b.pairs, a, &nk);
+                const int rc = enqueue_pairs(L.model[i], pl.pc, ne, pl.tail, b.tab, b.pairs, a, &nk);
                 if (rc) return rc;
             }
             const int rc = enqueue_items(sc, pl, b.recs, b.ck, b.so, b.off, b.items, b.ctrl, a, &nk);

@@ -59,6 +59,9 @@ struct PruneArgs : ScreenArgs {
     PruneConst pc;
     const uint32_t *box;  // ne x 16: each elite gene's mutation box, half2 (centre, radius)
     const float *u0;      // ne x ne: pair_bound_kernel's bound of every mask of a parent pair
+    const float *t1;      // its bounds of the masks that agree on k1 genes: pair_index x 2^k1
+    uint64_t goff[8];     // draw offset (x kGolden) of those genes' crossover bits
+    uint32_t k1;
     const float *tmax;    // ne x ne: the linear tail's largest value over a pair (null without a tail)
     uint32_t *pub;        // kPruneMs x gridDim.x: okey of each CTA's 1st / 2nd / 4th best entry
     uint32_t sel_cap;     // entries of the selection scratch in shared memory (>= gridDim.x)
@@ -158,17 +161,21 @@ __global__ void prune_box_kernel(const float *__restrict__ tab, int ne, float s,
     box[i] = *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// u0[a * ne + b]: an upper bound of the real score of every crossover
-// candidate of parents a, b (any mask, no jump), with its own f32 rounding
-// added. The genes are taken in the order `perm` (the ones that matter most
-// first); the masks of the first n_enum are enumerated and the others take
-// the hull of both parents' boxes, so
-//   u0 = max over masks of [f(c) + sum |grad_k f(c)| r_k] + q(r) + tail,
-// q(r) = sum max(Q_ii, 0) r_i^2 + sum |Q_ij| r_i r_j. A pair and its mirror
-// have the same masks, so a <= b is evaluated once. Each thread takes some
-// values of the enumerated genes past the fifth, and walks the first five in
-// Gray order: a flip updates the gradient by 16 FMAs and the value by two.
-constexpr int kPairGray = 5;  // genes walked in Gray order per thread
+// Upper bounds of the real score of the crossover candidates of parents a, b
+// (no jump), their own f32 rounding added: t1 over the masks that agree on the
+// first k1 genes, u0 over all masks. The genes are taken in the order `perm`
+// (the ones that matter most first); the masks of the first n_enum are
+// enumerated and the others take the hull of both parents' boxes:
+//   max over masks of [f(c) + sum |grad_k f(c)| r_k] + q(r) + tail.
+// A pair and its mirror have the same masks (complemented), so a <= b is
+// evaluated once. A group of 2^(k1 - 5) x 16 threads takes a pair: each thread
+// fixes genes 5..k1-1, takes every 16th value of the enumerated genes from k1
+// on, and walks the first five in Gray order, where a flip updates the
+// gradient by 16 FMAs and the value by two; its 32 maxima meet the other
+// threads' in shared memory.
+constexpr int kPairGray = 5;   // genes walked in Gray order per thread
+constexpr int kPairUps = 16;   // threads that share the enumerated genes from k1 on
+constexpr int kMaxMaskGenes = 8;
 
 struct PairArgs {
     float qs[16][16];  // Qs in `perm` order
@@ -177,21 +184,39 @@ struct PairArgs {
     float w16, s, err;
     const float *tab;
     const uint32_t *box;
-    float *u0, *tmax;
-    int ne, n_enum, tpp_log2;  // threads per pair (a power of two)
+    float *u0, *t1, *tmax;
+    int ne, n_enum, k1, tail;
     uint8_t perm[16];
 };
 
-__global__ void __launch_bounds__(128, 4) pair_bound_kernel(const __grid_constant__ PairArgs A) {
-    const uint64_t gt = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t pair = gt >> A.tpp_log2;
-    const uint32_t sub = static_cast<uint32_t>(gt) & ((1u << A.tpp_log2) - 1u);
-    const uint64_t ne = static_cast<uint64_t>(A.ne);
-    // a mirrored pair, and what lies past the last pair, has no masks to take
-    // but joins its warp's shuffles
-    uint32_t a = static_cast<uint32_t>(pair / ne), b = static_cast<uint32_t>(pair - a * ne);
-    const bool mine = a < A.ne && a <= b;
-    if (!mine) a = b = 0;
+// Index of the unordered pair {a, b} among a <= b.
+__host__ __device__ __forceinline__ uint32_t pair_index(uint32_t a, uint32_t b) {
+    const uint32_t lo = min(a, b), hi = max(a, b);
+    return hi * (hi + 1) / 2 + lo;
+}
+
+__global__ void __launch_bounds__(128, 3) pair_bound_kernel(const __grid_constant__ PairArgs A) {
+    __shared__ uint32_t s_best[(128 / kPairUps) << kPairGray];  // okey of each pair's 2^k1 entries
+    __shared__ uint32_t s_top[128 / kPairUps];
+    const uint32_t tid = threadIdx.x;
+    const uint32_t low_log2 = static_cast<uint32_t>(A.k1 - kPairGray);
+    const uint32_t g_log2 = low_log2 + 4;  // threads per pair: 2^low x kPairUps
+    const uint32_t slot = tid >> g_log2, sub = tid & ((1u << g_log2) - 1u);
+    const uint32_t low = sub & ((1u << low_log2) - 1u), up = sub >> low_log2;
+    const uint32_t n_slots = 128u >> g_log2;
+    for (uint32_t i = tid; i < (n_slots << A.k1); i += 128) s_best[i] = 0u;
+    if (tid < n_slots) s_top[tid] = 0u;
+    __syncthreads();
+    const uint32_t n_pairs = static_cast<uint32_t>(A.ne) * (A.ne + 1) / 2;
+    const uint32_t pair = blockIdx.x * n_slots + slot;
+    const bool mine = pair < n_pairs;
+    uint32_t a = 0, b = 0;  // pair = b (b + 1) / 2 + a, a <= b
+    if (mine) {
+        b = static_cast<uint32_t>((sqrt(8.0 * pair + 1.0) - 1.0) * 0.5);
+        while (b * (b + 1) / 2 > pair) --b;
+        while ((b + 1) * (b + 2) / 2 <= pair) ++b;
+        a = pair - b * (b + 1) / 2;
+    }
     float c[16], r[16], d[16];  // centre under parent a (or the hull's), radius, centre of b minus centre of a
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
@@ -210,9 +235,12 @@ __global__ void __launch_bounds__(128, 4) pair_bound_kernel(const __grid_constan
             r[q] = fmaxf(__fsub_ru(hi, c[q]), __fsub_ru(c[q], lo));
         }
     }
-    float best = -INFINITY;
-    const uint32_t n_hi = mine ? 1u << (A.n_enum - kPairGray) : 0u;
-    for (uint32_t hi = sub; hi < n_hi; hi += 1u << A.tpp_log2) {
+    float best[1 << kPairGray];  // by the first five genes' mask
+#pragma unroll
+    for (int i = 0; i < (1 << kPairGray); ++i) best[i] = -INFINITY;
+    const uint32_t n_up = mine ? 1u << (A.n_enum - A.k1) : 0u;
+    for (uint32_t u = up; u < n_up; u += kPairUps) {
+        const uint32_t hi = (u << low_log2) | low;  // genes 5.. of the mask
         float x[16], g[16];
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
@@ -241,12 +269,20 @@ __global__ void __launch_bounds__(128, 4) pair_bound_kernel(const __grid_constan
             float v = f;
 #pragma unroll
             for (int q = 0; q < 16; ++q) v = __fmaf_rn(fabsf(g[q]), r[q], v);
-            best = fmaxf(best, v);
+            best[st ^ (st >> 1)] = fmaxf(best[st ^ (st >> 1)], v);
         }
     }
-    // the largest over the pair's threads (tpp <= 32: within a warp)
-    for (int o = 1; o < (1 << A.tpp_log2); o <<= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (sub != 0 || !mine) return;
+    if (up < n_up) {
+        float top = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < (1 << kPairGray); ++i) {
+            top = fmaxf(top, best[i]);
+            atomicMax(&s_best[(slot << A.k1) + (low << kPairGray) + i], score_okey(best[i]));
+        }
+        atomicMax(&s_top[slot], score_okey(top));
+    }
+    __syncthreads();
+    if (!mine) return;
     float q2 = 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -256,7 +292,7 @@ __global__ void __launch_bounds__(128, 4) pair_bound_kernel(const __grid_constan
         q2 = __fmaf_rn(t, r[i], q2);
     }
     float tl = 0.0f;
-    if (A.tmax) {
+    if (A.tail) {
 #pragma unroll
         for (int k = 16; k < kNtot; ++k) {
             const float ya = fmaxf(fminf(A.tab[a * kNtot + k], 1.0f), 0.0f);
@@ -266,22 +302,30 @@ __global__ void __launch_bounds__(128, 4) pair_bound_kernel(const __grid_constan
                                       : fmaxf(__fsub_rd(fminf(ya, yb), A.s), 0.0f);
             tl = __fmaf_ru(w, y, tl);
         }
-        A.tmax[a * ne + b] = tl;
-        A.tmax[b * ne + a] = tl;
     }
-    const float u = best + q2 + tl + A.err;
-    A.u0[a * ne + b] = u;
-    A.u0[b * ne + a] = u;
+    const float add = q2 + tl + A.err;
+    for (uint32_t i = sub; i < (1u << A.k1); i += 1u << g_log2)
+        A.t1[(static_cast<size_t>(pair) << A.k1) + i] = okey_score(s_best[(slot << A.k1) + i]) + add;
+    if (sub == 0) {
+        const float v = okey_score(s_top[slot]) + add;
+        A.u0[a * A.ne + b] = v;
+        A.u0[b * A.ne + a] = v;
+        if (A.tail) {
+            A.tmax[a * A.ne + b] = tl;
+            A.tmax[b * A.ne + a] = tl;
+        }
+    }
 }
 
 // ---- the pruning screen ------------------------------------------------------------
 
-// Per-warp queue of candidates whose parent pair the table cannot rule out.
+// Per-warp queues: candidates whose parent pair the table cannot rule out,
+// and those whose first k1 crossover bits cannot either (or that jump).
 constexpr uint32_t kWqCap = 64;
 struct WarpQueue {
     uint64_t st[kWqCap];  // splitmix64 state of the candidate's first draw
-    uint32_t item[kWqCap], dcand[kWqCap], ddraw[kWqCap];
-    uint32_t meta[kWqCap];  // ea | eb << 11 | immigrant << 30 | jump << 31
+    uint4 q1[kWqCap];     // item, candidate, draw offset, ea | eb << 11 | immigrant << 30 | jump << 31
+    uint4 q2[kWqCap];     // the same
 };
 
 // The bound of one queued candidate from its 16 crossover bits (and its jump):
@@ -399,9 +443,22 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     };
     next_item();
     unsigned int gk = 0;
-    uint32_t round = 0, nq = 0;
-    bool has_def = false;  // holds a candidate the full queue could not take; its warp pauses until the flush
-    Pend def{0u, 0u, 0u};
+    uint32_t round = 0, n1 = 0, n2 = 0;  // n1, n2: the warp's queue lengths
+    const uint32_t lt = (1u << lane) - 1u;
+    // candidates the CTA's full queue could not take (one from either warp
+    // queue); the warp pauses until the flush
+    uint32_t n_def = 0;
+    Pend def[2] = {{0u, 0u, 0u}, {0u, 0u, 0u}};
+    auto push = [&](const Pend &q) {
+        const unsigned int ps = atomicAdd(&s_pend_n, 1u);
+        if (ps < kPendCap) {
+            pend[ps] = q;
+        } else {
+            if (n_def == 0) def[0] = q;
+            else def[1] = q;
+            ++n_def;
+        }
+    };
 
     auto rescore = [&](const Pend &q, unsigned long long t1, unsigned long long t2, float ts) {
         const Item it = A.items[q.item];
@@ -421,12 +478,12 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     for (;;) {
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
-        const int any = __syncthreads_or(valid || has_def || nq > 0);
-        const int any_def = __syncthreads_or(has_def);
+        const int any = __syncthreads_or(valid || n_def > 0 || n1 + n2 > 0);
+        const int any_def = __syncthreads_or(n_def > 0);
         // the queue is evaluated once it can employ every thread (or a thread
-        // waits on it, or the work is done); a flush appends <= pn + 256 <= 768
+        // waits on it, or the work is done); a flush appends <= pn + 2 x 256 <= 1024
         if (pn >= kThreads || any_def || (!any && pn > 0)) {
-            if (s_buf_n + kPendCap + kThreads > A.buf_cap) merge();  // make room first
+            if (s_buf_n + kPendCap + 2 * kThreads > A.buf_cap) merge();  // make room first
             unsigned long long t1 = s_t1, t2 = s_t2;
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
@@ -436,10 +493,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                 ts = okey_score(g);
             }
             for (uint32_t i = tid; i < pn; i += kThreads) rescore(pend[i], t1, t2, ts);
-            if (has_def) {
-                rescore(def, t1, t2, ts);
-                has_def = false;
-            }
+            for (uint32_t i = 0; i < n_def; ++i) rescore(i == 0 ? def[0] : def[1], t1, t2, ts);
+            n_def = 0;
             __syncthreads();
             if (tid == 0) s_pend_n = 0;
             __syncthreads();
@@ -469,8 +524,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
 #pragma unroll 1
         for (int rr = 0; rr < kRounds; ++rr) {
             bool pass = false;
-            uint64_t s0 = st;
-            uint32_t meta = 0, dc = dcand, dd = ddraw, itm = item;
+            const uint64_t s0 = st;
+            uint4 e = make_uint4(item, dcand, ddraw, 0u);
             if (valid) {
                 const uint32_t ea = fastmod_u32(draw_hi(s0), A.sc.ne_magic, A.sc.ne);
                 const uint32_t eb = fastmod_u32(draw_hi(s0 + kGolden), A.sc.ne_magic, A.sc.ne);
@@ -479,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                 const uint32_t pi = ea * A.sc.ne + eb;
                 const bool on = A.bm_words ? ((bm[pi >> 5] >> (pi & 31u)) & 1u) != 0u : !(A.u0[pi] < tlo);
                 pass = imm || jump || on;
-                meta = ea | (eb << 11) | (imm ? 1u << 30 : 0u) | (jump && !imm ? 1u << 31 : 0u);
+                e.w = ea | (eb << 11) | (imm ? 1u << 30 : 0u) | (jump && !imm ? 1u << 31 : 0u);
                 const uint32_t len = (imm ? 33u : 62u) + (jump ? 2u : 0u);
                 st += static_cast<uint64_t>(len) * kGolden;
                 ddraw += len;
@@ -488,36 +543,55 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
             }
             const uint32_t m = __ballot_sync(0xffffffffu, pass);
             if (pass) {
-                const uint32_t slot = nq + __popc(m & ((1u << lane) - 1u));
+                const uint32_t slot = n1 + __popc(m & lt);
                 wq.st[slot] = s0;
-                wq.item[slot] = itm;
-                wq.dcand[slot] = dc;
-                wq.ddraw[slot] = dd;
-                wq.meta[slot] = meta;
+                wq.q1[slot] = e;
             }
-            nq += __popc(m);
-            if (nq >= 32 || (nq > 0 && !__any_sync(0xffffffffu, valid))) {
-                __syncwarp();
-                const uint32_t nb = min(nq, 32u);
-                nq -= nb;
+            n1 += __popc(m);
+            if (n1 < 32 && (n1 + n2 == 0 || __any_sync(0xffffffffu, valid))) continue;
+            // a warp's worth (or, without work left, the rest) of the first queue: the first k1 bits
+            __syncwarp();
+            {
+                const uint32_t nb = min(n1, 32u);
+                n1 -= nb;
+                bool to2 = false, imm = false;
+                uint4 q = make_uint4(0u, 0u, 0u, 0u);
                 if (lane < nb) {
-                    const uint32_t slot = nq + lane;
-                    const uint32_t mt = wq.meta[slot];
-                    const float b = prune_bound<kTail>(A, bx, wq.st[slot], mt);
-                    // immigrants are always scored; a NaN bound is never trusted
-                    if ((mt & (1u << 30)) || !(b < tlo)) {
-                        const Pend q{wq.item[slot], wq.dcand[slot], wq.ddraw[slot]};
-                        const unsigned int ps = atomicAdd(&s_pend_n, 1u);
-                        if (ps < kPendCap) {
-                            pend[ps] = q;
-                        } else {
-                            has_def = true;
-                            def = q;
-                        }
+                    q = wq.q1[n1 + lane];
+                    const uint64_t sq = wq.st[n1 + lane];
+                    const uint32_t ea = q.w & 2047u, eb = (q.w >> 11) & 2047u;
+                    imm = (q.w & (1u << 30)) != 0u;
+                    bool jump = (q.w >> 31) != 0u;
+                    if (jump && !kTail) {  // a jump past gene 15 leaves the score as it is
+                        jump = draw_hi(sq + 62 * kGolden) % 29u < 16u;
+                        if (!jump) q.w &= 0x7fffffffu;
                     }
+                    uint32_t mask = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < kMaxMaskGenes; ++k)
+                        if (k < A.k1) mask |= (draw_bitword(sq + A.goff[k]) >> 31) << k;
+                    if (ea > eb) mask ^= (1u << A.k1) - 1u;
+                    const float b1 = A.t1[(static_cast<size_t>(pair_index(ea, eb)) << A.k1) + mask];
+                    to2 = !imm && (jump || !(b1 < tlo));
                 }
-                if (__any_sync(0xffffffffu, has_def)) break;
+                if (imm) push(Pend{q.x, q.y, q.z});  // immigrants are always scored
+                const uint32_t m2 = __ballot_sync(0xffffffffu, to2);
+                if (to2) wq.q2[n2 + __popc(m2 & lt)] = q;
+                n2 += __popc(m2);
             }
+            // the second queue: each candidate's own bound
+            if (n2 >= 32 || (n2 > 0 && n1 == 0 && !__any_sync(0xffffffffu, valid))) {
+                __syncwarp();
+                const uint32_t nb = min(n2, 32u);
+                n2 -= nb;
+                if (lane < nb) {
+                    const uint4 q = wq.q2[n2 + lane];
+                    const Item it = A.items[q.x];
+                    const uint64_t sq = stream_seed(A.seed, it.stream) + (it.draw0 + q.z + 1) * kGolden;
+                    if (!(prune_bound<kTail>(A, bx, sq, q.w) < tlo)) push(Pend{q.x, q.y, q.z});  // NaN: scored
+                }
+            }
+            if (__any_sync(0xffffffffu, n_def > 0)) break;
         }
     }
     Entry *out = A.lists + static_cast<size_t>(blockIdx.x) * A.kpad;
@@ -551,12 +625,12 @@ inline uint32_t prune_bm_words(int ne) {
 
 // Shared memory of the pruning screen: the sort buffer, the warps' queues, the
 // CTA's queue, the box table, the pair bitmap and the selection scratch of the
-// published keys (one per CTA, at most 8 CTAs per SM), with el_smem the elite
+// published keys (one per CTA, at most 3 CTAs per SM), with el_smem the elite
 // table.
 size_t prune_smem(uint32_t sort_n, int ne, int num_sms, bool el_smem) {
     return static_cast<size_t>(sort_n) * sizeof(Entry) + (kThreads / 32) * sizeof(WarpQueue) +
            kPendCap * sizeof(Pend) + static_cast<size_t>(ne) * 17 * sizeof(uint32_t) +
-           prune_bm_words(ne) * sizeof(uint32_t) + 8ull * num_sms * sizeof(uint32_t) +
+           prune_bm_words(ne) * sizeof(uint32_t) + 3ull * num_sms * sizeof(uint32_t) +
            (el_smem ? static_cast<size_t>(ne + 1) * kNtot * sizeof(float) : 0);
 }
 
@@ -627,20 +701,43 @@ inline int pair_enum(uint64_t lambda, int ne) {
     return k;
 }
 
-// The pair table's arguments: the genes in descending order of their influence
-// (the mean gradient over the unit box times 1, the box's width, stands in for
-// the elites' spread), the model in that order, and the table's own rounding.
-PairArgs make_pair_args(const csx_model &m, const PruneConst &pc, uint64_t lambda, int ne, bool tail,
-                        const float *tab, const uint32_t *box, float *u0, float *tmax) {
-    PairArgs P{};
-    double infl[16], qsum = 0.0, lsum = 0.0;
+// Genes of the mask table: the enumerated ones but four (a pair's group of
+// threads shares those), at most eight, fewer where the table would pass 64 MB.
+inline int pair_k1(int n_enum, int ne) {
+    const uint64_t pairs = static_cast<uint64_t>(ne) * (ne + 1) / 2;
+    int k = std::min(kMaxMaskGenes, std::max(kPairGray, n_enum - 4));
+    while (k > kPairGray && (pairs << (k + 2)) > (64ull << 20)) --k;
+    return k;
+}
+
+// Device scratch of the pair bounds: boxes, then u0, then (with a tail) tmax,
+// then t1.
+struct PairBufs {
+    uint32_t *box = nullptr;
+    float *u0 = nullptr, *tmax = nullptr, *t1 = nullptr;
+    int n_enum = kPairGray, k1 = kPairGray;
+};
+
+// The 16 quadratic genes in descending order of their influence: the mean
+// gradient over the unit box (the device call's elites are not on the host).
+void gene_order(const csx_model &m, const PruneConst &pc, uint8_t (&perm)[16]) {
+    double infl[16];
     for (int k = 0; k < 16; ++k) {
         double g = static_cast<double>(m.w_lin[k]);
         for (int j = 0; j < 16; ++j) g += 0.5 * static_cast<double>(pc.qs[k][j]);
         infl[k] = std::fabs(g);
-        P.perm[k] = static_cast<uint8_t>(k);
+        perm[k] = static_cast<uint8_t>(k);
     }
-    std::stable_sort(P.perm, P.perm + 16, [&](uint8_t a, uint8_t b) { return infl[a] > infl[b]; });
+    std::stable_sort(perm, perm + 16, [&](uint8_t a, uint8_t b) { return infl[a] > infl[b]; });
+}
+
+// The pair table's arguments: the model in gene_order, and the table's own
+// rounding.
+PairArgs make_pair_args(const csx_model &m, const PruneConst &pc, int ne, bool tail,
+                        const float *tab, const PairBufs &b) {
+    PairArgs P{};
+    double qsum = 0.0, lsum = 0.0;
+    gene_order(m, pc, P.perm);
     for (int i = 0; i < 16; ++i) {
         P.lin[i] = m.w_lin[P.perm[i]];
         for (int j = 0; j < 16; ++j) {
@@ -659,12 +756,14 @@ PairArgs make_pair_args(const csx_model &m, const PruneConst &pc, uint64_t lambd
     const double e = 2.0 * gam * (std::fabs(static_cast<double>(P.w16)) + 4.0 * lsum + 4.0 * qsum) + 1e-30;
     P.err = std::nextafter(static_cast<float>(e * (1.0 + std::ldexp(1.0, -20))), INFINITY);
     P.tab = tab;
-    P.box = box;
-    P.u0 = u0;
-    P.tmax = tail ? tmax : nullptr;
+    P.box = b.box;
+    P.u0 = b.u0;
+    P.t1 = b.t1;
+    P.tmax = b.tmax;
+    P.tail = tail ? 1 : 0;
     P.ne = ne;
-    P.n_enum = pair_enum(lambda, ne);
-    P.tpp_log2 = std::min(5, P.n_enum - kPairGray);
+    P.n_enum = b.n_enum;
+    P.k1 = b.k1;
     return P;
 }
 

@@ -368,7 +368,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     const uint64_t min_prune = env_u64("CSX_PRUNE_MIN_CANDS", 400ull * 3 * sms * kThreads);
     pl->prune_ok = pl->prune && lam_range >= min_prune;
     if (pl->prune_ok && grid_override == 0) {
-        // the selection scratch holds one key per CTA: at most 8 CTAs of 256 threads per SM
+        // the selection scratch holds one key per CTA: at most 3 CTAs per SM
         pl->el_smem = prune_el_smem(pl->sort_n, ne, cx.num_sms, cx.max_smem);
         pl->smem = prune_smem(pl->sort_n, ne, cx.num_sms, pl->el_smem);
         pl->prune = pl->smem + 1024 <= cx.max_smem;
@@ -538,48 +538,53 @@ int enqueue_merge(Entry *cur, Entry *nxt, uint32_t nl, uint32_t kpad, cudaStream
     return CSX_OK;
 }
 
-// Device scratch of the pair bounds: boxes, then u0, then (with a tail) tmax.
-struct PairBufs {
-    uint32_t *box = nullptr;
-    float *u0 = nullptr, *tmax = nullptr;
-};
-
-size_t pair_bytes(int ne, bool tail) {
+size_t pair_bytes(uint64_t lambda, int ne, bool tail) {
     const size_t n = static_cast<size_t>(ne);
-    return (n * 16 + n * n * (tail ? 2 : 1)) * sizeof(float);
+    const int k1 = pair_k1(pair_enum(lambda, ne), ne);
+    return (n * 16 + n * n * (tail ? 2 : 1) + ((n * (n + 1) / 2) << k1)) * sizeof(float);
 }
 
-PairBufs pair_bufs(void *base, int ne, bool tail) {
+PairBufs pair_bufs(void *base, uint64_t lambda, int ne, bool tail) {
     const size_t n = static_cast<size_t>(ne);
     PairBufs b;
+    b.n_enum = pair_enum(lambda, ne);
+    b.k1 = pair_k1(b.n_enum, ne);
     b.box = static_cast<uint32_t *>(base);
     b.u0 = reinterpret_cast<float *>(b.box + n * 16);
     b.tmax = tail ? b.u0 + n * n : nullptr;
+    b.t1 = b.u0 + n * n * (tail ? 2 : 1);
     return b;
 }
 
-int enqueue_pairs(const csx_model &m, const PruneConst &pc, uint64_t lambda, int ne, bool tail, const float *tab,
-                  const PairBufs &b, cudaStream_t st, uint32_t *launches) {
+int enqueue_pairs(const csx_model &m, const PruneConst &pc, int ne, bool tail, const float *tab, const PairBufs &b,
+                  cudaStream_t st, uint32_t *launches) {
     prune_box_kernel<<<(ne * 16 + 127) / 128, 128, 0, st>>>(tab, ne, pc.s, b.box);
     CSX_CUDA(cudaGetLastError());
-    const PairArgs P = make_pair_args(m, pc, lambda, ne, tail, tab, b.box, b.u0, b.tmax);
-    const uint64_t threads = (static_cast<uint64_t>(ne) * ne) << P.tpp_log2;
-    pair_bound_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(P);
+    const PairArgs P = make_pair_args(m, pc, ne, tail, tab, b);
+    const uint64_t pairs = static_cast<uint64_t>(ne) * (ne + 1) / 2;
+    const uint64_t per_block = 128u >> (b.k1 - kPairGray + 4);
+    pair_bound_kernel<<<static_cast<unsigned>((pairs + per_block - 1) / per_block), 128, 0, st>>>(P);
     CSX_CUDA(cudaGetLastError());
     *launches += 2;
     return CSX_OK;
 }
 
 // The pruning screen's arguments past the plain screen's.
-PruneArgs prune_args(const ScreenArgs &A, const Plan &pl, const PairBufs &b, uint32_t *pub, int num_sms) {
-    PruneArgs P;
+PruneArgs prune_args(const ScreenArgs &A, const csx_model &m, const Plan &pl, const PairBufs &b, uint32_t *pub,
+                     int num_sms) {
+    PruneArgs P{};
     static_cast<ScreenArgs &>(P) = A;
+    uint8_t perm[16];
+    gene_order(m, pl.pc, perm);
+    for (int k = 0; k < b.k1; ++k) P.goff[k] = (3 + 2ull * perm[k]) * kGolden;
+    P.k1 = static_cast<uint32_t>(b.k1);
+    P.t1 = b.t1;
     P.pc = pl.pc;
     P.box = b.box;
     P.u0 = b.u0;
     P.tmax = b.tmax;
     P.pub = pub;
-    P.sel_cap = 8u * static_cast<uint32_t>(num_sms);
+    P.sel_cap = 3u * static_cast<uint32_t>(num_sms);
     P.el_smem = pl.el_smem ? 1u : 0u;
     P.bm_words = prune_bm_words(static_cast<int>(A.sc.ne));
     // a rebuild reads the whole table once per CTA: every 8 rounds for 64
@@ -610,8 +615,8 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     PairBufs pairs;
     if (pl.prune) {
         CSX_CUDA(cx.pub.ensure(static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t)));
-        CSX_CUDA(cx.pairs.ensure(pair_bytes(ne, pl.tail)));
-        pairs = pair_bufs(cx.pairs.p, ne, pl.tail);
+        CSX_CUDA(cx.pairs.ensure(pair_bytes(pl.lam, ne, pl.tail)));
+        pairs = pair_bufs(cx.pairs.p, pl.lam, ne, pl.tail);
     }
     if (!pl.short_path) {
         CSX_CUDA(cx.recs.ensure(g.n_seg * sizeof(SegRec)));
@@ -643,7 +648,7 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     CSX_CUDA(cudaGetLastError());
     ++launches;
     if (pl.prune) {
-        rc = enqueue_pairs(model, pl.pc, pl.lam, ne, pl.tail, tab, pairs, st, &launches);
+        rc = enqueue_pairs(model, pl.pc, ne, pl.tail, tab, pairs, st, &launches);
         if (rc) return rc;
     }
     CSX_CUDA(mark(1));
@@ -662,7 +667,7 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
 
     const ScreenArgs A = screen_args(cfg, model, sc, pl, tab, items, ctrl, static_cast<Entry *>(cx.lists_a.p));
     if (pl.prune) {
-        const PruneArgs P = prune_args(A, pl, pairs, static_cast<uint32_t *>(cx.pub.p), cx.num_sms);
+        const PruneArgs P = prune_args(A, model, pl, pairs, static_cast<uint32_t *>(cx.pub.p), cx.num_sms);
         screen_p_fn(pl.tail, pl.tc)<<<pl.grid, kThreads, pl.smem, st>>>(P);
     } else if (pl.tc) {
         TcScreenArgs P;
