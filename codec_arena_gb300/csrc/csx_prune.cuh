@@ -46,7 +46,18 @@
 namespace csx {
 
 constexpr int kPruneMs = 3;  // order statistics each CTA publishes: its 1st, 2nd and 4th best
-constexpr uint32_t kPruneMergeRounds = 16;  // rounds between merges of a non-empty buffer
+// Candidates per thread between the CTA's barriers, and outer rounds between
+// merges of a non-empty buffer.
+constexpr int kPruneRounds = 64;
+constexpr uint32_t kPruneMergeRounds = 4;
+// kGolden's inverse modulo 2^64: a draw offset back from its state.
+constexpr uint64_t golden_inverse() {
+    uint64_t x = kGolden;  // correct to 3 bits; each Newton step doubles them
+    for (int i = 0; i < 5; ++i) x *= 2 - kGolden * x;
+    return x;
+}
+constexpr uint64_t kGoldenInv = golden_inverse();
+static_assert(kGolden * kGoldenInv == 1, "inverse modulo 2^64");
 
 struct PruneConst {
     float qs[16][16];  // Qs = Q + Q^T (Qs_kk = 2 Q_kk): grad of the quadratic block is Qs x
@@ -323,9 +334,9 @@ __global__ void __launch_bounds__(128, 3) pair_bound_kernel(const __grid_constan
 // and those whose first k1 crossover bits cannot either (or that jump).
 constexpr uint32_t kWqCap = 64;
 struct WarpQueue {
-    uint64_t st[kWqCap];  // splitmix64 state of the candidate's first draw
-    uint4 q1[kWqCap];     // item, candidate, draw offset, ea | eb << 11 | immigrant << 30 | jump << 31
-    uint4 q2[kWqCap];     // the same
+    uint4 q1[kWqCap];   // splitmix64 state of the candidate's first draw, its index in the item,
+    uint4 q2[kWqCap];   //   ea | eb << 11 | immigrant << 30 | jump << 31
+    uint32_t i1[kWqCap], i2[kWqCap];  // its item
 };
 
 // The bound of one queued candidate from its 16 crossover bits (and its jump):
@@ -424,19 +435,18 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     __syncthreads();
 
     Entry *buf = E + A.kpad;
-    uint32_t item = 0, left = 0, dcand = 0, ddraw = 0;
+    uint32_t item = 0, left = 0, n_it = 0;
     uint64_t st = 0;  // state of the candidate's first draw
     uint32_t screened = 0, exact = 0;  // per thread: far below 2^32
     bool valid = false;
     auto next_item = [&]() {
         item = atomicAdd(&A.ctrl->next_item, 1u);
         valid = item < n_items;
+        n_it = left = 0;  // a thread without work counts down from 2^32 and never passes
         if (valid) {
             const Item it = A.items[item];
             st = stream_seed(A.seed, it.stream) + (it.draw0 + 1) * kGolden;
-            left = it.n;
-            dcand = 0;
-            ddraw = 0;
+            n_it = left = it.n;
             screened += it.n;
             valid = left > 0;
         }
@@ -445,11 +455,16 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     unsigned int gk = 0;
     uint32_t round = 0, n1 = 0, n2 = 0;  // n1, n2: the warp's queue lengths
     const uint32_t lt = (1u << lane) - 1u;
+    const bool pow2 = (A.sc.ne & (A.sc.ne - 1)) == 0;
     // candidates the CTA's full queue could not take (one from either warp
     // queue); the warp pauses until the flush
     uint32_t n_def = 0;
     Pend def[2] = {{0u, 0u, 0u}, {0u, 0u, 0u}};
-    auto push = [&](const Pend &q) {
+    auto push = [&](const uint4 &e, uint32_t itm) {
+        const Item it = A.items[itm];
+        const uint64_t s0 = (static_cast<uint64_t>(e.y) << 32) | e.x;
+        const uint64_t draw = (s0 - stream_seed(A.seed, it.stream)) * kGoldenInv - 1;
+        const Pend q{itm, e.z, static_cast<uint32_t>(draw - it.draw0)};
         const unsigned int ps = atomicAdd(&s_pend_n, 1u);
         if (ps < kPendCap) {
             pend[ps] = q;
@@ -507,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         if (!any) break;
         float ts = s_ts;
         const unsigned long long t1 = s_t1;
-        if ((round & 7u) == 0) gk = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
+        gk = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
         if ((static_cast<unsigned long long>(gk) << 32) > t1) ts = okey_score(gk);
         const float tlo = __fsub_rd(ts, A.pc.err);
         // rebuild the bitmap: early on at rounds 1, 2, 4, ..., then every bm_period
@@ -522,30 +537,32 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         }
         ++round;
 #pragma unroll 1
-        for (int rr = 0; rr < kRounds; ++rr) {
-            bool pass = false;
+        for (int rr = 0; rr < kPruneRounds; ++rr) {
             const uint64_t s0 = st;
-            uint4 e = make_uint4(item, dcand, ddraw, 0u);
-            if (valid) {
-                const uint32_t ea = fastmod_u32(draw_hi(s0), A.sc.ne_magic, A.sc.ne);
-                const uint32_t eb = fastmod_u32(draw_hi(s0 + kGolden), A.sc.ne_magic, A.sc.ne);
-                const bool imm = (draw_vh(s0 + 2 * kGolden) >> 8) < A.sc.imm_thr;
-                const bool jump = (draw_vh(s0 + (imm ? 32ull : 61ull) * kGolden) >> 8) < A.sc.jump_thr;
-                const uint32_t pi = ea * A.sc.ne + eb;
-                const bool on = A.bm_words ? ((bm[pi >> 5] >> (pi & 31u)) & 1u) != 0u : !(A.u0[pi] < tlo);
-                pass = imm || jump || on;
-                e.w = ea | (eb << 11) | (imm ? 1u << 30 : 0u) | (jump && !imm ? 1u << 31 : 0u);
-                const uint32_t len = (imm ? 33u : 62u) + (jump ? 2u : 0u);
-                st += static_cast<uint64_t>(len) * kGolden;
-                ddraw += len;
-                ++dcand;
-                if (--left == 0) next_item();
+            const uint32_t itm = item, dcand = n_it - left;
+            const uint32_t xa = draw_hi(s0), xb = draw_hi(s0 + kGolden);
+            uint32_t ea, eb;
+            if (pow2) {
+                ea = xa & (A.sc.ne - 1);
+                eb = xb & (A.sc.ne - 1);
+            } else {
+                ea = fastmod_u32(xa, A.sc.ne_magic, A.sc.ne);
+                eb = fastmod_u32(xb, A.sc.ne_magic, A.sc.ne);
             }
+            const bool imm = (draw_vh(s0 + 2 * kGolden) >> 8) < A.sc.imm_thr;
+            const uint64_t sj = s0 + (imm ? 32u : 61u) * kGolden;  // the jump test's draw ends a candidate without one
+            const bool jump = (draw_vh(sj) >> 8) < A.sc.jump_thr;
+            st = sj + (jump ? 3u : 1u) * kGolden;
+            const uint32_t pi = ea * A.sc.ne + eb;
+            const bool on = A.bm_words ? ((bm[pi >> 5] >> (pi & 31u)) & 1u) != 0u : !(A.u0[pi] < tlo);
+            const bool pass = valid && (imm || jump || on);
+            if (--left == 0) next_item();
             const uint32_t m = __ballot_sync(0xffffffffu, pass);
             if (pass) {
                 const uint32_t slot = n1 + __popc(m & lt);
-                wq.st[slot] = s0;
-                wq.q1[slot] = e;
+                wq.q1[slot] = make_uint4(static_cast<uint32_t>(s0), static_cast<uint32_t>(s0 >> 32), dcand,
+                                         ea | (eb << 11) | (imm ? 1u << 30 : 0u) | (jump && !imm ? 1u << 31 : 0u));
+                wq.i1[slot] = itm;
             }
             n1 += __popc(m);
             if (n1 < 32 && (n1 + n2 == 0 || __any_sync(0xffffffffu, valid))) continue;
@@ -554,29 +571,35 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
             {
                 const uint32_t nb = min(n1, 32u);
                 n1 -= nb;
-                bool to2 = false, imm = false;
+                bool to2 = false, immq = false;
                 uint4 q = make_uint4(0u, 0u, 0u, 0u);
+                uint32_t iq = 0;
                 if (lane < nb) {
                     q = wq.q1[n1 + lane];
-                    const uint64_t sq = wq.st[n1 + lane];
-                    const uint32_t ea = q.w & 2047u, eb = (q.w >> 11) & 2047u;
-                    imm = (q.w & (1u << 30)) != 0u;
-                    bool jump = (q.w >> 31) != 0u;
-                    if (jump && !kTail) {  // a jump past gene 15 leaves the score as it is
-                        jump = draw_hi(sq + 62 * kGolden) % 29u < 16u;
-                        if (!jump) q.w &= 0x7fffffffu;
+                    iq = wq.i1[n1 + lane];
+                    const uint64_t sq = (static_cast<uint64_t>(q.y) << 32) | q.x;
+                    const uint32_t qa = q.w & 2047u, qb = (q.w >> 11) & 2047u;
+                    immq = (q.w & (1u << 30)) != 0u;
+                    bool jq = (q.w >> 31) != 0u;
+                    if (jq && !kTail) {  // a jump past gene 15 leaves the score as it is
+                        jq = draw_hi(sq + 62 * kGolden) % 29u < 16u;
+                        if (!jq) q.w &= 0x7fffffffu;
                     }
                     uint32_t mask = 0;
 #pragma unroll
                     for (uint32_t k = 0; k < kMaxMaskGenes; ++k)
                         if (k < A.k1) mask |= (draw_bitword(sq + A.goff[k]) >> 31) << k;
-                    if (ea > eb) mask ^= (1u << A.k1) - 1u;
-                    const float b1 = A.t1[(static_cast<size_t>(pair_index(ea, eb)) << A.k1) + mask];
-                    to2 = !imm && (jump || !(b1 < tlo));
+                    if (qa > qb) mask ^= (1u << A.k1) - 1u;
+                    const float b1 = A.t1[(static_cast<size_t>(pair_index(qa, qb)) << A.k1) + mask];
+                    to2 = !immq && (jq || !(b1 < tlo));
                 }
-                if (imm) push(Pend{q.x, q.y, q.z});  // immigrants are always scored
+                if (immq) push(q, iq);  // immigrants are always scored
                 const uint32_t m2 = __ballot_sync(0xffffffffu, to2);
-                if (to2) wq.q2[n2 + __popc(m2 & lt)] = q;
+                if (to2) {
+                    const uint32_t slot = n2 + __popc(m2 & lt);
+                    wq.q2[slot] = q;
+                    wq.i2[slot] = iq;
+                }
                 n2 += __popc(m2);
             }
             // the second queue: each candidate's own bound
@@ -586,9 +609,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                 n2 -= nb;
                 if (lane < nb) {
                     const uint4 q = wq.q2[n2 + lane];
-                    const Item it = A.items[q.x];
-                    const uint64_t sq = stream_seed(A.seed, it.stream) + (it.draw0 + q.z + 1) * kGolden;
-                    if (!(prune_bound<kTail>(A, bx, sq, q.w) < tlo)) push(Pend{q.x, q.y, q.z});  // NaN: scored
+                    const uint64_t sq = (static_cast<uint64_t>(q.y) << 32) | q.x;
+                    if (!(prune_bound<kTail>(A, bx, sq, q.w) < tlo)) push(q, wq.i2[n2 + lane]);  // NaN: scored
                 }
             }
             if (__any_sync(0xffffffffu, n_def > 0)) break;

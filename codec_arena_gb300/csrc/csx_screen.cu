@@ -587,9 +587,9 @@ PruneArgs prune_args(const ScreenArgs &A, const csx_model &m, const Plan &pl, co
     P.sel_cap = 3u * static_cast<uint32_t>(num_sms);
     P.el_smem = pl.el_smem ? 1u : 0u;
     P.bm_words = prune_bm_words(static_cast<int>(A.sc.ne));
-    // a rebuild reads the whole table once per CTA: every 8 rounds for 64
+    // a rebuild reads the whole table once per CTA: every 2 outer rounds for 64
     // elites (128 words), less often in proportion for more
-    P.bm_period = std::max<uint32_t>(8, pow2_at_least(P.bm_words / 16));
+    P.bm_period = std::max<uint32_t>(2, pow2_at_least(P.bm_words / 64));
     return P;
 }
 
