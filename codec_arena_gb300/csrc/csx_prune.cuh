@@ -580,18 +580,16 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                     const uint64_t sq = (static_cast<uint64_t>(q.y) << 32) | q.x;
                     const uint32_t qa = q.w & 2047u, qb = (q.w >> 11) & 2047u;
                     immq = (q.w & (1u << 30)) != 0u;
-                    bool jq = (q.w >> 31) != 0u;
-                    if (jq && !kTail) {  // a jump past gene 15 leaves the score as it is
-                        jq = draw_hi(sq + 62 * kGolden) % 29u < 16u;
-                        if (!jq) q.w &= 0x7fffffffu;
-                    }
+                    // what its jump can add (a jump past gene 15 adds nothing without a tail)
+                    float jc = 0.0f;
+                    if (q.w >> 31) jc = A.jb.c[draw_hi(sq + 62 * kGolden) % 29u];
                     uint32_t mask = 0;
 #pragma unroll
                     for (uint32_t k = 0; k < kMaxMaskGenes; ++k)
                         if (k < A.k1) mask |= (draw_bitword(sq + A.goff[k]) >> 31) << k;
                     if (qa > qb) mask ^= (1u << A.k1) - 1u;
                     const float b1 = A.t1[(static_cast<size_t>(pair_index(qa, qb)) << A.k1) + mask];
-                    to2 = !immq && (jq || !(b1 < tlo));
+                    to2 = !immq && !(__fadd_ru(b1, jc) < tlo);
                 }
                 if (immq) push(q, iq);  // immigrants are always scored
                 const uint32_t m2 = __ballot_sync(0xffffffffu, to2);
