@@ -52,6 +52,7 @@
 #include "csx_device.cuh"
 #include "csx_tc.cuh"
 #include "csx_pipeline.cuh"
+#include "csx_dense.cuh"
 #include "csx_screen_kernels.cuh"
 #include "csx_prune.cuh"
 #include "csx_ties.cuh"
@@ -139,6 +140,8 @@ uint32_t unit_threshold(float prob) {
 struct Plan {
     StreamGeom g;
     bool short_path = false;
+    bool dense = false;     // items from block maps (csx_dense.cuh) instead of the walk
+    DenseGeom dg{};
     uint64_t items_cap = 0;
     uint32_t kpad = 0, sort_n = 0, buf_cap = 0;
     int grid = 0;
@@ -331,6 +334,31 @@ void segment_geometry(const csx_cfg &cfg, uint64_t seg, bool slack, StreamGeom &
     g.ckcap = static_cast<uint32_t>(cover / (1ull << g.d_log2) + 3);
 }
 
+// Generations up to this many candidates build their items from block maps:
+// 0.12 ms per 1e6 candidates, where the walk and its links take 0.50 ms at 2e5,
+// 0.70 at 1e6, 1.13 at 4e6, 1.37 at 1.6e7 and 1.80 at 4e7 (T = 4): the lines
+// cross near 9e6. Blocks of 512 draws (8 candidates an item) up to 5e5, where
+// items of 16 would leave threads of the screen without work; 1024 above
+// (items 0.147 ms against 0.159 at 1e6, 0.51 against 0.56 at 4e6).
+constexpr uint64_t kDenseMaxCands = 8'000'000;
+
+// Block maps for the call's streams: enough groups of 32 blocks that the
+// longest candidates fill them; the geometry's segment count and checkpoint
+// capacity then size the groups' records and scratch.
+void dense_geometry(const csx_cfg &cfg, uint64_t lam, Plan *pl) {
+    StreamGeom &g = pl->g;
+    const uint64_t my_max = std::max(g.per, g.my_last);
+    const uint64_t len = (unit_threshold(cfg.imm_p) == (1u << 24) ? 33 : 62) + (unit_threshold(cfg.jump_p) ? 2 : 0);
+    pl->dg.b_log2 = lam <= 500'000 ? 9 : 10;
+    const uint64_t gdraws = static_cast<uint64_t>(kDenseGroup) << pl->dg.b_log2;
+    const uint64_t gps = (my_max * len + gdraws - 1) / gdraws;
+    if (gps * gdraws > 2 * my_max * len) return;  // short streams: their groups would mostly lie past their ends
+    pl->dg.gps = static_cast<uint32_t>(gps);
+    pl->dense = true;
+    g.n_seg = gps * g.nT;
+    g.ckcap = kDenseWords;
+}
+
 // A share of one generation's work items (csx_screen_items): every share
 // builds the same item list and screens its part of it.
 struct Shard {
@@ -407,6 +435,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     // 2.65e9, 256 candidates beat 512 by 0.5% with three CTAs per SM and by
     // 0.25% with the filter kernel's two)
     uint64_t d = item_cands ? item_cands : env_u64("CSX_ITEM_CANDS", 0);
+    bool sized = d != 0;  // item or segment sizes asked for: the walk's items
     if (d == 0) {
         const uint64_t target = 64ull * 3 * static_cast<uint64_t>(sharded ? kItemRefSms : cx.num_sms) * kThreads;
         d = std::max<uint64_t>(1, lam_range / target);
@@ -428,6 +457,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     // It depends on lambda only, so every share of a sharded call builds the
     // same segments.
     uint64_t seg = seg_cands ? seg_cands : env_u64("CSX_SEG_CANDS", 0);
+    sized = sized || seg != 0;
     if (seg == 0) {
         uint64_t r = static_cast<uint64_t>(std::sqrt(static_cast<double>(lam_range)));
         while (r * r > lam_range) --r;
@@ -436,6 +466,12 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     }
     segment_geometry(cfg, seg, true, g);
     pl->short_path = my_max <= D;
+    pl->dense = false;
+    if (!pl->short_path && lam_range <= kDenseMaxCands && !sized) dense_geometry(cfg, lam_range, pl);
+    if (pl->dense) {  // every block of a group is an item, the last group's up to the stream's end
+        pl->items_cap = g.n_seg * kDenseGroup;
+        return CSX_OK;
+    }
     // a segment's range of cnt candidates splits at the multiples of D inside
     // it: at most 2 + cnt / D items, and the ranges partition the candidates
     pl->items_cap = pl->short_path ? g.nT : 2 * g.n_seg + lam_range / D + 1;
@@ -479,6 +515,24 @@ int enqueue_items(const SynthConst &sc, const Plan &pl, SegRec *recs, uint64_t *
         stream_items_kernel<<<unit_blocks(g.nT, 256), 256, 0, st>>>(g, items, ctrl);
         CSX_CUDA(cudaGetLastError());
         ++*launches;
+        return CSX_OK;
+    }
+    if (pl.dense) {
+        const DenseGeom &d = pl.dg;
+        const uint32_t words = (kDenseGroup << d.b_log2) / 32 + 2;
+        const size_t msm = 2ull * words * 4 + kDenseGroup * 64 * 2;
+        dense_map_kernel<<<static_cast<unsigned>(g.n_seg), 256, msm, st>>>(sc, g, d, ck);
+        CSX_CUDA(cudaGetLastError());
+        const size_t csm = std::max<size_t>(std::min(d.gps, kDenseTile) * 64ull * 4, kDenseGroup * 64 * 2);
+        CSX_CUDA(cudaFuncSetAttribute(dense_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kDenseTile * 64 * 4)));
+        dense_chain_kernel<<<static_cast<unsigned>(g.nT), 1024, csm, st>>>(g, d, ck, so, ctrl);
+        CSX_CUDA(cudaGetLastError());
+        scan_kernel<<<1, 1024, 0, st>>>(so, g.n_seg, off, ctrl, pl.items_cap);
+        CSX_CUDA(cudaGetLastError());
+        dense_emit_kernel<<<unit_blocks(g.n_seg, 4), 128, 0, st>>>(g, d, ck, so, off, items, ctrl);
+        CSX_CUDA(cudaGetLastError());
+        *launches += 4;
         return CSX_OK;
     }
     walk_kernel<<<unit_blocks(g.n_seg, 128), 128, 0, st>>>(sc, g, recs, ck, ctrl);
