@@ -10,14 +10,18 @@
 // 16 genes is 25.6 MB. The normal equations are FP64 multiply-adds
 // (nf(nf+1)/2 per row) and run on the FP64 pipe; everything else is a few
 // hundred FP32 FMAs per row.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 
 #include "csx_screen.h"
 #include "csx_surrogate.h"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -36,7 +40,7 @@ constexpr int kPartBlocksFull = 64;                // the same for the full layo
 constexpr int kGramRows = 32;                      // rows per Φ tile in the normal equations
 constexpr int kGramBlk = 4;                        // each thread owns a 4×4 block of ΦᵀΦ
 constexpr int kGramThreads = 1024;                 // 4×4 blocks per CTA (CTAs along y split the blocks)
-constexpr int kSolveThreads = 1024;
+constexpr int kSolveThreads = 256;
 
 __host__ __device__ constexpr int tri(int i) { return i * (i + 1) / 2; }
 __host__ __device__ constexpr int gram_nb(int nf) { return (nf + kGramBlk - 1) / kGramBlk; }
@@ -76,13 +80,36 @@ __device__ void load_coef(CoefT<QG> &s, const float *coef, int ng) {
 }
 
 // Stage rows [r0, r0 + kRowThreads) of the gene table into shared memory
-// (coalesced), row stride `st` (odd, so a thread-per-row read is conflict free).
+// (coalesced), row stride `st` (odd, so a thread-per-row read is conflict
+// free). Eight loads are in flight per thread: one at a time, the 29 loads of
+// a full tile cost 29 trips to memory, two thirds of the row kernels' time.
 __device__ void stage_rows(float *tile, const float *genes, int64_t n, int ldg, int ng, int st, int64_t r0) {
-    const int64_t rows = (n - r0 < kRowThreads) ? (n - r0) : kRowThreads;
-    const int total = static_cast<int>(rows) * ng;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int r = idx / ng, k = idx - r * ng;
-        tile[r * st + k] = genes[(r0 + r) * static_cast<int64_t>(ldg) + k];
+    const int rows = static_cast<int>((n - r0 < kRowThreads) ? (n - r0) : kRowThreads);
+    const int total = rows * ng, step = static_cast<int>(blockDim.x);
+    const int dr = step / ng, dk = step - dr * ng;
+    const float *src = genes + r0 * static_cast<int64_t>(ldg);
+    int idx = threadIdx.x, r = idx / ng, k = idx - r * ng;
+    while (idx < total) {
+        float v[8];
+        int at[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            at[u] = -1;
+            if (idx < total) {
+                v[u] = src[r * static_cast<int64_t>(ldg) + k];
+                at[u] = r * st + k;
+            }
+            idx += step;
+            r += dr;
+            k += dk;
+            if (k >= ng) {
+                k -= ng;
+                ++r;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (at[u] >= 0) tile[at[u]] = v[u];
     }
 }
 
@@ -255,14 +282,24 @@ __device__ __forceinline__ void feature_pair(int f, int ng, int &a, int &b) {
 }
 
 // Per-block partial sums of Σ_r gout_r Φ_f(g_r), FP64, thread f per feature.
+// The rows of a tile are staged 64 at a time as FP64: x = [g, 1] and, for an
+// FP32 gout, h = gout x (48 bits: exact), so that a feature's term is one
+// FMA(h_a, x_b, sum), the same real product rounded once as FMA(gout, x_a x_b,
+// sum). The FP64 pipe (two lanes per SM) bounds it: converting both genes and
+// multiplying them per feature took four of its operations where one does
+// (100,003 rows of 29 genes: 210 µs). An FP64 gout keeps FMA(gout, x_a x_b):
+// gout x_a would round.
+constexpr int kCoefRows = 64;
+
 template <typename TG>
 __global__ void __launch_bounds__(kRowThreads) sg_grad_coef_kernel(int ng, int nf, const float *__restrict__ genes,
                                                                    int64_t n, int ldg, const TG *__restrict__ gout,
                                                                    double *__restrict__ part) {
     constexpr int kPer = (kFeatCap + kRowThreads - 1) / kRowThreads;  // features per thread (2)
-    extern __shared__ float tile[];
-    __shared__ double go_s[kRowThreads];
-    const int st = stride_for(ng);
+    constexpr bool kF32 = sizeof(TG) == 4;
+    constexpr int kX = kMaxLin + 1;
+    __shared__ double xs[kCoefRows][kX], hs[kF32 ? kCoefRows : 1][kX];
+    __shared__ double go_s[kCoefRows];
     int a[kPer], b[kPer];
 #pragma unroll
     for (int m = 0; m < kPer; ++m) {
@@ -271,23 +308,29 @@ __global__ void __launch_bounds__(kRowThreads) sg_grad_coef_kernel(int ng, int n
         if (f < nf) feature_pair(f, ng, a[m], b[m]);
     }
     double acc[kPer] = {};
-    for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * kRowThreads; r0 < n;
-         r0 += static_cast<int64_t>(gridDim.x) * kRowThreads) {
-        __syncthreads();
-        stage_rows(tile, genes, n, ldg, ng, st, r0);
-        const int64_t rows = (n - r0 < kRowThreads) ? (n - r0) : kRowThreads;
-        if (threadIdx.x < rows) {
-            tile[threadIdx.x * st + ng] = 1.0f;
-            go_s[threadIdx.x] = static_cast<double>(gout[r0 + threadIdx.x]);
-        }
-        __syncthreads();
+    const int nx = ng + 1;
+    for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * kRowThreads; t0 < n;
+         t0 += static_cast<int64_t>(gridDim.x) * kRowThreads) {
+        const int64_t t1 = t0 + kRowThreads < n ? t0 + kRowThreads : n;
+        for (int64_t r0 = t0; r0 < t1; r0 += kCoefRows) {
+            const int rows = static_cast<int>(t1 - r0 < kCoefRows ? t1 - r0 : kCoefRows);
+            __syncthreads();
+#pragma unroll 8
+            for (int idx = threadIdx.x; idx < rows * nx; idx += kRowThreads) {
+                const int r = idx / nx, k = idx - r * nx;
+                const double x = k < ng ? static_cast<double>(genes[(r0 + r) * static_cast<int64_t>(ldg) + k]) : 1.0;
+                xs[r][k] = x;
+                if (kF32) hs[kF32 ? r : 0][k] = static_cast<double>(gout[r0 + r]) * x;
+            }
+            if (!kF32 && threadIdx.x < rows) go_s[threadIdx.x] = static_cast<double>(gout[r0 + threadIdx.x]);
+            __syncthreads();
 #pragma unroll
-        for (int m = 0; m < kPer; ++m) {
-            if (threadIdx.x + m * kRowThreads < nf) {
-                for (int r = 0; r < rows; ++r) {
-                    const double phi =
-                        static_cast<double>(tile[r * st + a[m]]) * static_cast<double>(tile[r * st + b[m]]);
-                    acc[m] = fma(go_s[r], phi, acc[m]);
+            for (int m = 0; m < kPer; ++m) {
+                if (threadIdx.x + m * kRowThreads < nf) {
+#pragma unroll 4
+                    for (int r = 0; r < rows; ++r)
+                        acc[m] = kF32 ? fma(hs[kF32 ? r : 0][a[m]], xs[r][b[m]], acc[m])
+                                      : fma(go_s[r], xs[r][a[m]] * xs[r][b[m]], acc[m]);
                 }
             }
         }
@@ -299,13 +342,32 @@ __global__ void __launch_bounds__(kRowThreads) sg_grad_coef_kernel(int ng, int n
     }
 }
 
-__global__ void sg_sum_parts_kernel(const double *__restrict__ part, int nparts, int stride, int nf,
-                                    double *__restrict__ out) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf) return;
-    double s = 0.0;
-    for (int p = 0; p < nparts; ++p) s += part[static_cast<int64_t>(p) * stride + f];
-    out[f] = s;
+// Sums of `nparts` partial results: eight threads per entry take every eighth
+// part, so that the loads of one entry overlap (one thread per entry waited
+// for 152 loads in turn: 21 µs for 153 entries, 27 for the normal equations').
+constexpr int kSumSplit = 8;
+
+__device__ __forceinline__ double sum_parts(const double *__restrict__ p, int nparts, int64_t stride, bool live,
+                                            double (*s)[32]) {
+    double v = 0.0;
+    if (live) {
+#pragma unroll 4
+        for (int q = threadIdx.y; q < nparts; q += kSumSplit) v += p[q * stride];
+    }
+    s[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y != 0) return 0.0;
+#pragma unroll
+    for (int y = 1; y < kSumSplit; ++y) v += s[y][threadIdx.x];
+    return v;
+}
+
+__global__ void __launch_bounds__(32 * kSumSplit) sg_sum_parts_kernel(const double *__restrict__ part, int nparts,
+                                                                      int stride, int nf, double *__restrict__ out) {
+    __shared__ double s[kSumSplit][32];
+    const int f = blockIdx.x * 32 + threadIdx.x;
+    const double v = sum_parts(part + f, nparts, stride, f < nf, s);
+    if (threadIdx.y == 0 && f < nf) out[f] = v;
 }
 
 // Normal equations: thread t of CTA column y owns the 4×4 block number
@@ -389,10 +451,14 @@ __global__ void __launch_bounds__(kGramThreads) sg_gram_kernel(int ng, int nf, c
     if (rhs_here) part_r[static_cast<int64_t>(blockIdx.x) * kFeatCap + t] = racc;
 }
 
-__global__ void sg_gram_sum_kernel(const double *__restrict__ part_g, int nparts, int nf, double *__restrict__ gram) {
-    const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // (pair, u, v)
+__global__ void __launch_bounds__(32 * kSumSplit) sg_gram_sum_kernel(const double *__restrict__ part_g, int nparts,
+                                                                     int nf, double *__restrict__ gram) {
+    __shared__ double sp[kSumSplit][32];
+    const int64_t e = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;  // (pair, u, v)
     const int npairs = gram_pairs(nf);
-    if (e >= static_cast<int64_t>(npairs) * kGramBlk * kGramBlk) return;
+    const int64_t total = static_cast<int64_t>(npairs) * kGramBlk * kGramBlk;
+    const double s = sum_parts(part_g + e, nparts, total, e < total, sp);
+    if (threadIdx.y != 0 || e >= total) return;
     const int t = static_cast<int>(e / (kGramBlk * kGramBlk)), uv = static_cast<int>(e % (kGramBlk * kGramBlk));
     const int u = uv / kGramBlk, v = uv - u * kGramBlk;
     int bi = 0;
@@ -400,75 +466,204 @@ __global__ void sg_gram_sum_kernel(const double *__restrict__ part_g, int nparts
     const int bj = t - tri(bi);
     const int a = bi * kGramBlk + u, b = bj * kGramBlk + v;
     if (a >= nf || b >= nf) return;
-    double s = 0.0;
-    for (int p = 0; p < nparts; ++p) s += part_g[(static_cast<int64_t>(p) * npairs + t) * (kGramBlk * kGramBlk) + uv];
     gram[static_cast<int64_t>(a) * nf + b] = s;
     gram[static_cast<int64_t>(b) * nf + a] = s;
 }
 
-// (G + αI) w = rhs + α·prior by Cholesky, FP64, packed lower triangle L
-// (tri(n) entries, then y[n]) in shared memory up to 166 coefficients, in a
-// global scratch for the full surface's 465; one CTA of 32×32 threads.
-__device__ void ridge_solve_body(double *L, int n, const double *__restrict__ gram, const double *__restrict__ rhs,
-                                 double alpha, const double *__restrict__ prior, double *__restrict__ w,
-                                 int *status) {
-    double *y = L + tri(n);
-    __shared__ int bad;
-    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    if (tid == 0) bad = 0;
-    for (int i = ty; i < n; i += 32)
-        for (int j = tx; j <= i; j += 32) L[tri(i) + j] = gram[static_cast<int64_t>(i) * n + j] + (i == j ? alpha : 0.0);
-    for (int i = tid; i < n; i += kSolveThreads) y[i] = rhs[i] + (prior ? alpha * prior[i] : 0.0);
+// (G + αI) w = rhs + α·prior, FP64, by a square-root-free Cholesky
+// factorisation (L D Lᵀ) of the matrix with the right side as one more row: at
+// the end that row holds D⁻¹ L⁻¹ (rhs + α·prior), and only Lᵀ w = that is left
+// to solve. A cluster of eight CTAs holds the packed rows in shared memory, row
+// i in CTA i mod 8, and takes four columns per step: every CTA sends its rows'
+// four entries to all (distributed shared memory), all meet at the cluster's
+// barrier, each factors the 4×4 diagonal block and the columns' entries for
+// itself and updates its own rows.
+//
+// What bounds it is the chain of pivots: a reciprocal and a few dependent
+// FP64 operations per column (no square root, no division per row), then the
+// barrier per four columns; the updates run on eight SMs' FP64 pipes (two
+// lanes each).
+constexpr int kSolveCtas = 8;
+constexpr int kSolveNb = 4;
+
+__host__ __device__ constexpr int solve_rows(int n, int r) {  // rows r, r + 8, ... <= n (n is the right side)
+    return r <= n ? (n - r) / kSolveCtas + 1 : 0;
+}
+// Doubles before local row q (global row r + 8 q, r + 8 q + 1 long).
+__host__ __device__ constexpr int solve_off(int r, int q) { return q * (r + 1) + kSolveCtas * (q * (q - 1) / 2); }
+constexpr size_t solve_smem(int n) {  // the largest CTA's rows, two column buffers, L's columns, the copy for n <= 166
+    return (static_cast<size_t>(solve_off(kSolveCtas - 1, solve_rows(n, 0))) + 2ull * (n + 1) * kSolveNb +
+            static_cast<size_t>(n + 1) * kSolveNb + (n <= kMaxFeat ? static_cast<size_t>(tri(n)) : 0u)) *
+           sizeof(double);
+}
+
+// 1 / d for a pivot: a float reciprocal of the significand and two Newton
+// steps x += x (1 - m x), then the exponent: eight dependent operations where
+// the division takes some thirty. Within an ulp or two of 1 / d for the
+// exponents a normal equation's pivot can have; the division otherwise
+// (zero, negative, subnormal, infinite, NaN, or a reciprocal near underflow).
+__device__ __forceinline__ double pivot_rcp(double d) {
+    const int64_t bits = __double_as_longlong(d);
+    const int64_t e = bits >> 52;  // sign and biased exponent
+    if (e < 2 || e > 2040) return 1.0 / d;
+    const double m = __longlong_as_double((bits & 0x000fffffffffffffll) | 0x3ff0000000000000ll);
+    double x = static_cast<double>(__frcp_rn(static_cast<float>(m)));
+    x = fma(x, fma(-m, x, 1.0), x);
+    x = fma(x, fma(-m, x, 1.0), x);
+    return __longlong_as_double(__double_as_longlong(x) - ((e - 1023) << 52));
+}
+
+// Lᵀ w = z by one warp: lane l holds z_l, z_{l+32}, ...; `row(i)` is L's row i.
+template <int kPer, class RowFn>
+__device__ __forceinline__ void back_substitute(int n, const double *zrow, RowFn row, double *__restrict__ w) {
+    const int lane = threadIdx.x & 31;
+    double z[kPer], cur[kPer], nxt[kPer];
+#pragma unroll
+    for (int m = 0; m < kPer; ++m) {
+        const int j = lane + 32 * m;
+        z[m] = j < n ? zrow[j] : 0.0;
+        cur[m] = j < n - 1 ? row(n - 1)[j] : 0.0;
+    }
+    for (int i = n - 1; i >= 0; --i) {
+#pragma unroll
+        for (int m = 0; m < kPer; ++m) {  // the next row's entries while this one is used
+            const int j = lane + 32 * m;
+            nxt[m] = j < i - 1 ? row(i - 1)[j] : 0.0;
+        }
+        double mine = 0.0;
+#pragma unroll
+        for (int m = 0; m < kPer; ++m)
+            if (m == i >> 5) mine = z[m];
+        const double wi = __shfl_sync(0xffffffffu, mine, i & 31);
+        if (lane == 0) w[i] = wi;
+#pragma unroll
+        for (int m = 0; m < kPer; ++m) {
+            z[m] = fma(-cur[m], wi, z[m]);
+            cur[m] = nxt[m];
+        }
+    }
+}
+
+__global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThreads)
+    sg_ridge_solve_kernel(int n, const double *__restrict__ gram, const double *__restrict__ rhs, double alpha,
+                          const double *__restrict__ prior, double *__restrict__ w, int *status) {
+    extern __shared__ double sm[];
+    __shared__ double s_l[kSolveNb][kSolveNb], s_r[kSolveNb];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int r = static_cast<int>(cluster.block_rank());
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nrows = solve_rows(n, r);
+    double *A = sm;                                              // this CTA's packed rows
+    double *P = sm + solve_off(kSolveCtas - 1, solve_rows(n, 0));  // two buffers of (n + 1) x 4 column entries
+    double *Lc = P + 2 * (n + 1) * kSolveNb;                     // the step's columns of L, all rows
+    double *Lfull = Lc + (n + 1) * kSolveNb;                     // n <= 166: L in one CTA for the last solve
+    for (int q = warp; q < nrows; q += kSolveThreads / 32) {
+        const int i = r + kSolveCtas * q;
+        double *row = A + solve_off(r, q);
+        for (int j = lane; j <= i; j += 32) {
+            double v;
+            if (i < n) v = gram[static_cast<int64_t>(i) * n + j] + (i == j ? alpha : 0.0);
+            else v = j < n ? rhs[j] + (prior ? alpha * prior[j] : 0.0) : 0.0;
+            row[j] = v;
+        }
+    }
+    int bad = 0;  // thread 0's count is the one reported
     __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        if (tid == 0) {
-            const double d = L[tri(k) + k];
-            if (!(d > 0.0) && bad == 0) bad = k + 1;
-            L[tri(k) + k] = sqrt(d);
+    for (int k0 = 0, buf = 0; k0 < n; k0 += kSolveNb, buf ^= 1) {
+        const int nb = min(kSolveNb, n - k0);
+        double *Pb = P + buf * (n + 1) * kSolveNb;
+        // own rows' entries of the four columns to every CTA
+        const int q0 = k0 > r ? (k0 - r + kSolveCtas - 1) / kSolveCtas : 0;  // first own row >= k0
+        for (int e = tid; e < (nrows - q0) * kSolveNb * kSolveCtas; e += kSolveThreads) {
+            const int c = e & (kSolveNb - 1), dst = (e >> 2) & (kSolveCtas - 1), q = q0 + (e >> 5);
+            const int i = r + kSolveCtas * q;
+            if (c < nb && k0 + c <= i)
+                cluster.map_shared_rank(Pb, dst)[i * kSolveNb + c] = A[solve_off(r, q) + k0 + c];
+        }
+        cluster.sync();
+        if (warp == 0) {  // the 4x4 diagonal block, every lane alike
+            double d[kSolveNb][kSolveNb], l[kSolveNb][kSolveNb], rc[kSolveNb];
+#pragma unroll
+            for (int a = 0; a < kSolveNb; ++a)
+#pragma unroll
+                for (int b = 0; b <= a; ++b) d[a][b] = a < nb ? Pb[(k0 + a) * kSolveNb + b] : (a == b ? 1.0 : 0.0);
+#pragma unroll
+            for (int k = 0; k < kSolveNb; ++k) {
+                if (!(d[k][k] > 0.0) && bad == 0) bad = k0 + k + 1;
+                rc[k] = pivot_rcp(d[k][k]);
+#pragma unroll
+                for (int a = k + 1; a < kSolveNb; ++a) l[a][k] = d[a][k] * rc[k];
+#pragma unroll
+                for (int a = k + 1; a < kSolveNb; ++a)
+#pragma unroll
+                    for (int b = k + 1; b <= a; ++b) d[a][b] = fma(-d[a][k], l[b][k], d[a][b]);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int k = 0; k < kSolveNb; ++k) {
+                    s_r[k] = rc[k];
+#pragma unroll
+                    for (int a = k + 1; a < kSolveNb; ++a) s_l[a][k] = l[a][k];
+                }
+            }
         }
         __syncthreads();
-        const double p = L[tri(k) + k];
-        for (int i = k + 1 + tid; i < n; i += kSolveThreads) L[tri(i) + k] /= p;
+        // the columns below: u (undivided) back into the buffer, l = u / d beside it
+        for (int i = k0 + tid; i <= n; i += kSolveThreads) {
+            double u[kSolveNb];
+#pragma unroll
+            for (int c = 0; c < kSolveNb; ++c) u[c] = (c < nb && k0 + c <= i) ? Pb[i * kSolveNb + c] : 0.0;
+#pragma unroll
+            for (int c = 1; c < kSolveNb; ++c)
+#pragma unroll
+                for (int m = 0; m < c; ++m) u[c] = fma(-u[m], s_l[c][m], u[c]);
+#pragma unroll
+            for (int c = 0; c < kSolveNb; ++c) {
+                Pb[i * kSolveNb + c] = u[c];
+                Lc[i * kSolveNb + c] = u[c] * s_r[c];
+            }
+        }
         __syncthreads();
-        for (int i = k + 1 + ty; i < n; i += 32) {
-            const double lik = L[tri(i) + k];
-            for (int j = k + 1 + tx; j <= i; j += 32) L[tri(i) + j] = fma(-lik, L[tri(j) + k], L[tri(i) + j]);
+        for (int q = q0 + warp; q < nrows; q += kSolveThreads / 32) {
+            const int i = r + kSolveCtas * q;
+            double *row = A + solve_off(r, q);
+            if (lane < nb && k0 + lane < i) row[k0 + lane] = Lc[i * kSolveNb + lane];  // L's entries stay in the row
+            const double u0 = Pb[i * kSolveNb], u1 = Pb[i * kSolveNb + 1], u2 = Pb[i * kSolveNb + 2],
+                         u3 = Pb[i * kSolveNb + 3];
+            const int jend = i < n ? i : n - 1;
+            for (int j = k0 + kSolveNb + lane; j <= jend; j += 32) {
+                double v = row[j];
+                v = fma(-u0, Lc[j * kSolveNb], v);
+                v = fma(-u1, Lc[j * kSolveNb + 1], v);
+                v = fma(-u2, Lc[j * kSolveNb + 2], v);
+                v = fma(-u3, Lc[j * kSolveNb + 3], v);
+                row[j] = v;
+            }
         }
         __syncthreads();
     }
-    for (int j = 0; j < n; ++j) {  // L z = y
-        if (tid == 0) y[j] /= L[tri(j) + j];
-        __syncthreads();
-        const double yj = y[j];
-        for (int i = j + 1 + tid; i < n; i += kSolveThreads) y[i] = fma(-L[tri(i) + j], yj, y[i]);
-        __syncthreads();
+    cluster.sync();  // every row of L is final
+    if (r == 0) {
+        const double *zrow = cluster.map_shared_rank(A, n % kSolveCtas) + solve_off(n % kSolveCtas, n / kSolveCtas);
+        if (n <= kMaxFeat) {  // L into this CTA, then the solve on local rows
+            for (int i = warp; i < n; i += kSolveThreads / 32) {
+                const double *src = cluster.map_shared_rank(A, i % kSolveCtas) + solve_off(i % kSolveCtas, i / kSolveCtas);
+                for (int j = lane; j < i; j += 32) Lfull[tri(i) + j] = src[j];
+            }
+            __syncthreads();
+            if (warp == 0)
+                back_substitute<(kMaxFeat + 31) / 32>(n, zrow, [&](int i) { return Lfull + tri(i); }, w);
+        } else if (warp == 0) {
+            back_substitute<(kFullFeat + 31) / 32>(
+                n, zrow,
+                [&](int i) {
+                    return cluster.map_shared_rank(A, i % kSolveCtas) + solve_off(i % kSolveCtas, i / kSolveCtas);
+                },
+                w);
+        }
+        if (tid == 0) *status = bad;
     }
-    for (int j = n - 1; j >= 0; --j) {  // Lᵀ w = z
-        if (tid == 0) y[j] /= L[tri(j) + j];
-        __syncthreads();
-        const double yj = y[j];
-        for (int i = tid; i < j; i += kSolveThreads) y[i] = fma(-L[tri(j) + i], yj, y[i]);
-        __syncthreads();
-    }
-    for (int i = tid; i < n; i += kSolveThreads) w[i] = y[i];
-    if (tid == 0) *status = bad;
-}
-
-__global__ void __launch_bounds__(kSolveThreads) sg_ridge_solve_kernel(int n, const double *__restrict__ gram,
-                                                                       const double *__restrict__ rhs, double alpha,
-                                                                       const double *__restrict__ prior,
-                                                                       double *__restrict__ w, int *status) {
-    extern __shared__ double L[];
-    ridge_solve_body(L, n, gram, rhs, alpha, prior, w, status);
-}
-
-__global__ void __launch_bounds__(kSolveThreads) sg_ridge_solve_global_kernel(int n, const double *__restrict__ gram,
-                                                                              const double *__restrict__ rhs,
-                                                                              double alpha,
-                                                                              const double *__restrict__ prior,
-                                                                              double *__restrict__ w, int *status,
-                                                                              double *scratch) {
-    ridge_solve_body(scratch, n, gram, rhs, alpha, prior, w, status);
+    cluster.sync();  // no CTA leaves while its rows are read
 }
 
 template <int QG>
@@ -512,6 +707,59 @@ __global__ void __launch_bounds__(kRowThreads) sg_ascend_kernel(const float *__r
     }
 }
 
+// The same for few rows: sixteen lanes per row, lane k with gene k (its
+// gradient's 16 coefficients in registers) and gene 16 + k, the row's genes
+// exchanged by shuffles. One thread per row leaves most SMs without work below
+// some ten thousand rows (5,120 rows: 20 CTAs). The gradient is accumulated in
+// grad_f32's order, the score by the row's first lane in score_f32's, so the
+// results are the same bits.
+constexpr int kLaneRows = 16;  // rows per CTA
+constexpr int64_t kLaneMaxRows = 30000;
+
+__global__ void __launch_bounds__(kLaneRows * 16) sg_ascend_lanes_kernel(const float *__restrict__ coef, int ng,
+                                                                         float *__restrict__ genes, int64_t n,
+                                                                         int ldg, float eta, int steps,
+                                                                         float *__restrict__ score) {
+    __shared__ CoefT<kQuadGenes> c;
+    __shared__ float fin[kLaneRows][kMaxLin + 3];
+    const int k = threadIdx.x & 15, rr = threadIdx.x >> 4;
+    const int64_t r = static_cast<int64_t>(blockIdx.x) * kLaneRows + rr;
+    float *row = genes + (r < n ? r : 0) * static_cast<int64_t>(ldg);
+    float g0 = row[k], g1 = k + 16 < ng ? row[k + 16] : 0.0f;
+    load_coef<CSX_SG_FP32, kQuadGenes>(c, coef, ng);
+    __syncthreads();
+    float q[16];
+#pragma unroll
+    for (int l = 0; l < 16; ++l) q[l] = l <= k ? c.q[tri(k) + l] : c.q[tri(l) + k];
+    const float w0 = c.lin[k], w1 = k + 16 < kMaxLin ? c.lin[k + 16] : 0.0f;
+    for (int s = 0; s < steps; ++s) {
+        float d = w0;
+#pragma unroll
+        for (int l = 0; l < 16; ++l) {
+            const float x = __shfl_sync(0xffffffffu, g0, l, 16);
+            d = __fmaf_rn(q[l], x, d);
+            if (l == k) d = __fmaf_rn(q[l], x, d);  // the square's derivative: its term twice
+        }
+        g0 = fmaxf(fminf(__fmaf_rn(eta, d, g0), 1.0f), 0.0f);
+        g1 = fmaxf(fminf(__fmaf_rn(eta, w1, g1), 1.0f), 0.0f);
+    }
+    if (r < n) {
+        if (steps > 0) {
+            row[k] = g0;
+            if (k + 16 < ng) row[k + 16] = g1;
+        }
+        fin[rr][k] = g0;
+        if (k + 16 < kMaxLin) fin[rr][k + 16] = k + 16 < ng ? g1 : 0.0f;
+    }
+    __syncwarp();
+    if (score && r < n && k == 0) {
+        float g[kMaxLin];
+#pragma unroll
+        for (int m = 0; m < kMaxLin; ++m) g[m] = fin[rr][m];
+        score[r] = score_f32(c, g);
+    }
+}
+
 #define SG_CUDA(call)                                                                       \
     do {                                                                                    \
         cudaError_t e_ = (call);                                                            \
@@ -551,11 +799,10 @@ size_t part_gram_bytes(int nf) {
 }
 constexpr size_t kPartCoefBytes = static_cast<size_t>(kPartBlocks) * kFeatCap * sizeof(double);
 size_t gram_smem(int nf) { return static_cast<size_t>(kGramRows) * gram_nb(nf) * kGramBlk * sizeof(double); }
-constexpr size_t kSolveSmem = (static_cast<size_t>(tri(kMaxFeat)) + kMaxFeat) * sizeof(double);
 
 int enable_smem() {  // on the current device, every call (cheap)
     SG_CUDA(cudaFuncSetAttribute(sg_ridge_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kSolveSmem)));
+                                 static_cast<int>(std::max(solve_smem(kMaxFeat), solve_smem(kFullFeat)))));
     SG_CUDA(cudaFuncSetAttribute(sg_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(gram_smem(kFullFeat))));
     return CSX_OK;
@@ -571,9 +818,9 @@ int coef_grad(int ng, int nf, const float *genes, int64_t n, int ldg, const TG *
                                                    ? (n + kRowThreads - 1) / kRowThreads
                                                    : kPartBlocks)
                                             : 1);
-    sg_grad_coef_kernel<TG><<<grid, kRowThreads, tile_bytes(ng), s>>>(ng, nf, genes, n, ldg, gout, part);
+    sg_grad_coef_kernel<TG><<<grid, kRowThreads, 0, s>>>(ng, nf, genes, n, ldg, gout, part);
     SG_CUDA(cudaGetLastError());
-    sg_sum_parts_kernel<<<(nf + 255) / 256, 256, 0, s>>>(part, grid, kFeatCap, nf, dcoef);
+    sg_sum_parts_kernel<<<(nf + 31) / 32, dim3(32, kSumSplit), 0, s>>>(part, grid, kFeatCap, nf, dcoef);
     SG_CUDA(cudaGetLastError());
     return CSX_OK;
 }
@@ -687,10 +934,10 @@ int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, co
     sg_gram_kernel<<<dim3(grid, ycols), threads, gram_smem(nf), s>>>(ng, nf, d_genes, n, ldg, d_fit, part_g, part_r);
     SG_CUDA(cudaGetLastError());
     const int64_t ne = static_cast<int64_t>(npairs) * kGramBlk * kGramBlk;
-    sg_gram_sum_kernel<<<static_cast<unsigned>((ne + 255) / 256), 256, 0, s>>>(part_g, grid, nf, d_gram);
+    sg_gram_sum_kernel<<<static_cast<unsigned>((ne + 31) / 32), dim3(32, kSumSplit), 0, s>>>(part_g, grid, nf, d_gram);
     SG_CUDA(cudaGetLastError());
     if (d_fit) {
-        sg_sum_parts_kernel<<<(nf + 255) / 256, 256, 0, s>>>(part_r, grid, kFeatCap, nf, d_rhs);
+        sg_sum_parts_kernel<<<(nf + 31) / 32, dim3(32, kSumSplit), 0, s>>>(part_r, grid, kFeatCap, nf, d_rhs);
         SG_CUDA(cudaGetLastError());
     }
     return CSX_OK;
@@ -702,20 +949,9 @@ int csx_sg_ridge_solve(int nf, const double *d_gram, const double *d_rhs, double
         return CSX_ERR_BAD_ARGS;
     if (int rc = enable_smem()) return rc;
     auto s = static_cast<cudaStream_t>(stream);
-    const size_t bytes = (static_cast<size_t>(tri(nf)) + nf) * sizeof(double);
-    if (nf <= kMaxFeat) {
-        sg_ridge_solve_kernel<<<1, kSolveThreads, bytes, s>>>(nf, d_gram, d_rhs, alpha, d_prior, d_w, d_status);
-        SG_CUDA(cudaGetLastError());
-        return CSX_OK;
-    }
-    // the full surface: the factor does not fit in shared memory
-    void *scratch = nullptr;
-    SG_CUDA(cudaMallocAsync(&scratch, bytes, s));
-    sg_ridge_solve_global_kernel<<<1, kSolveThreads, 0, s>>>(nf, d_gram, d_rhs, alpha, d_prior, d_w, d_status,
-                                                             static_cast<double *>(scratch));
-    const cudaError_t e = cudaGetLastError();
-    SG_CUDA(cudaFreeAsync(scratch, s));
-    SG_CUDA(e);
+    sg_ridge_solve_kernel<<<kSolveCtas, kSolveThreads, solve_smem(nf), s>>>(nf, d_gram, d_rhs, alpha, d_prior, d_w,
+                                                                            d_status);
+    SG_CUDA(cudaGetLastError());
     return CSX_OK;
 }
 
@@ -730,6 +966,9 @@ int csx_sg_ascend(const float *d_coef, int nf, float *d_genes, int64_t n, int ld
     if (is_full(nf))
         sg_ascend_kernel<kMaxLin><<<row_grid(n), kRowThreads, tile_bytes(ng), s>>>(d_coef, ng, d_genes, n, ldg, eta,
                                                                                  steps, d_score);
+    else if (n <= kLaneMaxRows)
+        sg_ascend_lanes_kernel<<<static_cast<unsigned>((n + kLaneRows - 1) / kLaneRows), kLaneRows * 16, 0, s>>>(
+            d_coef, ng, d_genes, n, ldg, eta, steps, d_score);
     else
         sg_ascend_kernel<kQuadGenes><<<row_grid(n), kRowThreads, tile_bytes(ng), s>>>(d_coef, ng, d_genes, n, ldg,
                                                                                     eta, steps, d_score);
