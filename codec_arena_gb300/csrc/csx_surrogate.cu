@@ -18,8 +18,10 @@
 #include <cstdint>
 #include <cstdio>
 
+#include "csx_device.cuh"
 #include "csx_screen.h"
 #include "csx_surrogate.h"
+#include "csx_tc.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -370,7 +372,11 @@ __global__ void __launch_bounds__(32 * kSumSplit) sg_sum_parts_kernel(const doub
     if (threadIdx.y == 0 && f < nf) out[f] = v;
 }
 
-// Normal equations: thread t of CTA column y owns the 4×4 block number
+struct GramRange;
+__device__ __forceinline__ bool gram_finite(const GramRange *r, int ng);
+
+// Normal equations in FP64 (the full surface, and tables with a non-finite
+// entry; csx_gram.cuh otherwise): thread t of CTA column y owns the 4×4 block number
 // y·1024 + t, (bi, bj) with bj <= bi, of ΦᵀΦ; CTA row x accumulates rows of
 // its chunk. Column 0's threads t < nf also accumulate (Φᵀy)_t. Φ for
 // kGramRows rows is staged in shared memory in FP64 (exact: a product of two
@@ -378,7 +384,9 @@ __global__ void __launch_bounds__(32 * kSumSplit) sg_sum_parts_kernel(const doub
 __global__ void __launch_bounds__(kGramThreads) sg_gram_kernel(int ng, int nf, const float *__restrict__ genes,
                                                                int64_t n, int ldg, const double *__restrict__ fit,
                                                                double *__restrict__ part_g,
-                                                               double *__restrict__ part_r) {
+                                                               double *__restrict__ part_r,
+                                                               const GramRange *__restrict__ range) {
+    if (range && gram_finite(range, ng)) return;  // sg_gram_mma_kernel's table
     extern __shared__ double phi[];  // [kGramRows][featpad]
     __shared__ float gs[kGramRows][kMaxLin + 1];
     __shared__ double ys[kGramRows];
@@ -760,6 +768,12 @@ __global__ void __launch_bounds__(kLaneRows * 16) sg_ascend_lanes_kernel(const f
     }
 }
 
+}  // namespace
+
+#include "csx_gram.cuh"
+
+namespace {
+
 #define SG_CUDA(call)                                                                       \
     do {                                                                                    \
         cudaError_t e_ = (call);                                                            \
@@ -803,6 +817,8 @@ size_t gram_smem(int nf) { return static_cast<size_t>(kGramRows) * gram_nb(nf) *
 int enable_smem() {  // on the current device, every call (cheap)
     SG_CUDA(cudaFuncSetAttribute(sg_ridge_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(std::max(solve_smem(kMaxFeat), solve_smem(kFullFeat)))));
+    SG_CUDA(cudaFuncSetAttribute(sg_gram_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kGmSmem)));
     SG_CUDA(cudaFuncSetAttribute(sg_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(gram_smem(kFullFeat))));
     return CSX_OK;
@@ -931,7 +947,31 @@ int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, co
     const int64_t want = (n + kGramRows - 1) / kGramRows;
     const int cap = gram_parts(nf);
     const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
-    sg_gram_kernel<<<dim3(grid, ycols), threads, gram_smem(nf), s>>>(ng, nf, d_genes, n, ldg, d_fit, part_g, part_r);
+    GramRange *range = nullptr;
+    if (!is_full(nf)) {
+        range = reinterpret_cast<GramRange *>(reinterpret_cast<char *>(part_r) + kPartCoefBytes - sizeof(GramRange));
+        auto *part = static_cast<longlong2 *>(d_work);
+        SG_CUDA(cudaMemsetAsync(range, 0, sizeof(GramRange), s));
+        sg_range_kernel<<<static_cast<unsigned>(std::min<int64_t>(n / 64 + 1, 152 * 4)), 256, 0, s>>>(
+            ng, d_genes, n, ldg, d_fit, range);
+        SG_CUDA(cudaGetLastError());
+        const int64_t drain = kGmRows * kGmDrain;
+        const int chunks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(kGmChunks, (n + drain - 1) / drain)));
+        sg_gram_mma_kernel<<<dim3(chunks, kGmBlocks), kGmThreads, kGmSmem, s>>>(ng, nf, d_genes, n, ldg, d_fit, range,
+                                                                                part);
+        SG_CUDA(cudaGetLastError());
+        sg_gram_kernel<<<dim3(grid, ycols), threads, gram_smem(nf), s>>>(ng, nf, d_genes, n, ldg, d_fit, part_g, part_r,
+                                                                        range);
+        SG_CUDA(cudaGetLastError());
+        const int total = tri(nf) + (d_fit ? nf : 0);
+        sg_gram_final_kernel<<<(total + 31) / 32, dim3(32, kSumSplit), 0, s>>>(ng, nf, chunks, range, part, part_g,
+                                                                              part_r, grid, d_gram,
+                                                                              d_fit ? d_rhs : nullptr);
+        SG_CUDA(cudaGetLastError());
+        return CSX_OK;
+    }
+    sg_gram_kernel<<<dim3(grid, ycols), threads, gram_smem(nf), s>>>(ng, nf, d_genes, n, ldg, d_fit, part_g, part_r,
+                                                                    nullptr);
     SG_CUDA(cudaGetLastError());
     const int64_t ne = static_cast<int64_t>(npairs) * kGramBlk * kGramBlk;
     sg_gram_sum_kernel<<<static_cast<unsigned>((ne + 31) / 32), dim3(32, kSumSplit), 0, s>>>(part_g, grid, nf, d_gram);

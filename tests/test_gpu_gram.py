@@ -1,0 +1,80 @@
+"""The refit's normal equations on the tensor cores (fixed point) against
+wider host arithmetic, at the edges of a stage (32 rows), a drain (128) and the
+row chunks, for each layout's gene count, with signed genes, zero columns,
+exact ones, wide exponents and subnormals; and tables with a non-finite entry,
+which the FP64 kernel takes.
+
+Tolerance: a scaled feature is rounded by at most 2^-56, so a row's product by
+2^-55; the digit products past the seventh add at most 6.1 x 2^-56. Per entry
+n x 8.1 x 2^-56 < n x 2^-52 of the columns' scales (each gene's largest value
+rounded up to a power of two), and the final rounding."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu(csx):
+    from conftest import has_gpu
+
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+
+
+def _phi(g, ng):
+    ii, jj = np.tril_indices(16)
+    one = np.ones((len(g), 1), g.dtype)
+    return np.concatenate([one, g[:, :ng], g[:, ii] * g[:, jj]], axis=1)
+
+
+def _run(genes, y, nf):
+    import torch
+
+    from codec_arena_gb300 import surrogate
+
+    gram, rhs = surrogate.normal_equations(torch.from_numpy(genes).cuda(), torch.from_numpy(y).cuda(), nf)
+    return gram.cpu().numpy(), rhs.cpu().numpy()
+
+
+@pytest.mark.parametrize("ng", [16, 17, 29])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 128, 129, 6400, 6401, 9001])
+def test_normal_equations_fixed_point(n, ng):
+    rng = np.random.default_rng(n + ng)
+    g = rng.random((n, ng), dtype=np.float32)
+    g[:, 1] = 2 * g[:, 1] - 1                                     # signed
+    g[:, 2] = np.round(g[:, 2])                                   # exact zeros and ones
+    g[:, 3] = 0.0                                                 # an empty column
+    g[:, 4] *= np.float32(2.0) ** rng.integers(-60, 20, n).astype(np.float32)
+    g[:, 5] = rng.integers(0, 9, n).astype(np.float32) * np.float32(1e-45)  # subnormals
+    g[:, 6] = np.round(g[:, 6], 4)
+    y = rng.normal(0, 30, n)
+    y[:: 7] *= 1e-9
+    gram, rhs = _run(g, y, 1 + ng + 136)
+    wide = g.astype(np.longdouble)
+    phi = _phi(wide, ng)
+    want, wrhs = phi.T @ phi, phi.T @ y.astype(np.longdouble)
+    top = np.abs(g).max(0).astype(np.float64)
+    scale = np.where(top > 0, 2.0 ** np.ceil(np.log2(np.where(top > 0, top, 1.0))), 1.0)
+    fs = _phi(scale[None, :], ng)[0]
+    ys = 2.0 ** np.ceil(np.log2(np.abs(y).max()))
+    assert np.all(np.abs(gram - want) <= n * 2.0 ** -52 * np.outer(fs, fs) + 2.0 ** -52 * np.abs(want))
+    assert np.all(np.abs(rhs - wrhs) <= n * 2.0 ** -52 * fs * ys + 2.0 ** -52 * np.abs(wrhs))
+    np.testing.assert_array_equal(gram, gram.T)
+
+
+@pytest.mark.parametrize("where", ["gene", "y"])
+def test_non_finite_tables_keep_the_fp64_kernel(where):
+    rng = np.random.default_rng(3)
+    g = rng.random((700, 29), dtype=np.float32)
+    y = rng.normal(0, 1, 700)
+    if where == "gene":
+        g[123, 20] = np.inf
+    else:
+        y[5] = np.nan
+    gram, rhs = _run(g, y, 166)
+    with np.errstate(invalid="ignore"):
+        phi = _phi(g.astype(np.float64), 29)
+        want, wrhs = phi.T @ phi, phi.T @ y
+    np.testing.assert_allclose(gram, want, rtol=1e-12)
+    np.testing.assert_allclose(rhs, wrhs, rtol=1e-9, atol=1e-9)
