@@ -37,12 +37,15 @@ namespace {
 
 constexpr int kDigits = 7;
 constexpr int kGmRows = 32;       // table rows per stage
-constexpr int kGmDrain = 4;       // stages between drains: 128 rows keep the FP32 sums exact
+// Stages between drains: 128 rows keep the FP32 sums exact where seven digit
+// products share an accumulator, 256 where four do (stacked digits).
+constexpr int kGmDrain = 4;
 constexpr int kGmN = 64;          // features per column block
 constexpr int kGmBlocks = 3;      // column blocks (166 features at most)
 constexpr int kGmChunks = 50;     // row chunks: 150 CTAs
 constexpr int kGmOutRows = 72;    // pair rows (57) + linear-only genes (13) + y, rounded up
-constexpr int kGmThreads = 544;   // one digit task per thread and stage (136 values x 4 groups of 8 rows)
+constexpr int kGmTasks = 544;     // digit tasks per stage, one per thread: 136 values x 4 groups of 8 rows
+constexpr int kGmThreads = kGmTasks + 32;  // and a warp that issues the MMAs (it waits where their queue is full)
 constexpr int kGmVars = 32;       // variables per row: g_0..g_15, 1, linear-only genes
 constexpr uint32_t kGmA = 128 * kGmRows * 2, kGmB = kGmN * kGmRows * 2;  // bytes of one digit's tiles
 constexpr uint32_t kGmBuf = kDigits * (kGmA + kGmB);
@@ -149,10 +152,21 @@ __device__ __forceinline__ void gm_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         : "memory");
 }
 
+// The integer that v holds, |v| < 2^24, without the conversion unit (16 per SM
+// and clock): its multiple of 4096 and the rest, each read off the significand.
+__device__ __forceinline__ int exact_int(float v) {
+    constexpr float kMagic = 12582912.0f;  // 1.5 x 2^23
+    const float hm = __fmaf_rn(v, 1.0f / 4096.0f, kMagic);
+    const float l = __fmaf_rn(__fsub_rn(hm, kMagic), -4096.0f, v);  // exact, |l| <= 2048
+    const int h = __float_as_int(hm) - 0x4b400000, li = __float_as_int(__fadd_rn(l, kMagic)) - 0x4b400000;
+    return h * 4096 + li;
+}
+
 // One CTA: the table rows of chunk blockIdx.x, the features of column block
 // blockIdx.y. While a stage's MMAs run, the next stage's digits are made in the
 // other buffer. part[(chunk, block)]: kGmOutRows x 64 x {hi, lo}; the chunk's
 // sum is hi 2^-30 + lo 2^-62 of the row's times the feature's scale.
+template <bool kStack>
 __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int nf, const float *__restrict__ genes,
                                                                    int64_t n, int ldg,
                                                                    const double *__restrict__ fit,
@@ -211,7 +225,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
                 x0 = __float_as_uint(src[lk]);
                 if (lk + 16 < ng) x1 = __float_as_uint(src[lk + 16]);
             }
-        } else if (t < stages && fit && r0 + (tid - 512) < hi) {
+        } else if (tid < kGmTasks && t < stages && fit && r0 + (tid - 512) < hi) {
             xy = static_cast<unsigned long long>(__double_as_longlong(fit[r0 + (tid - 512)]));
         }
     };
@@ -234,7 +248,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
             vars[lr * (kGmVars - 1) + lk] = split(x0, lk);
             if (lk + 16 < ng) vars[lr * (kGmVars - 1) + lk + 17] = split(x1, lk + 16);
             if (lk == 15) vars[lr * (kGmVars - 1) + 16] = make_int2(r0 + lr < hi ? 0x800000 * 32 : 0, 0);
-        } else {  // y 2^(55 - E_y), rounded: its 53-bit significand 3 bits up, shifted by its exponent
+        } else if (tid < kGmTasks) {  // y 2^(55 - E_y), rounded: its 53-bit significand 3 bits up, shifted by its exponent
             const int e = static_cast<int>((xy >> 52) & 2047u);
             int64_t m = static_cast<int64_t>((xy & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull)) << 4;
             if (xy >> 63) m = -m;
@@ -242,12 +256,13 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
             yint[tid - 512] = ((m >> sh) + 1) >> 1;
         }
         load(t + 1);
-        __syncthreads();
+        // the digit warps alone: the issuing warp is still waiting on the MMA queue
+        if (tid < kGmTasks) asm volatile("bar.sync 1, %0;" ::"n"(kGmTasks) : "memory");
         unsigned char *buf = bufs + (t & 1) * kGmBuf;
         constexpr int kF = kGmOutRows + kGmN;
-        static_assert(kF * (kGmRows / 8) == kGmThreads, "one task per thread");
+        static_assert(kF * (kGmRows / 8) == kGmTasks, "one task per thread");
         const int kg = tid / kF, f = tid - kg * kF;
-        const uint32_t a = s_va[f], b = s_vb[f];
+        const uint32_t a = tid < kGmTasks ? s_va[f] : 254u, b = tid < kGmTasks ? s_vb[f] : 254u;
         if (a != 254u) {
             uint32_t w[8][2];  // the integers, every digit offset by 128
 #pragma unroll
@@ -267,7 +282,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
             const int row = f < kGmOutRows ? f : f - kGmOutRows;
             unsigned char *dst = buf + (f < kGmOutRows ? 0u : kDigits * kGmA) + (row >> 3) * (kGmRows * 16) +
                                  kg * 128 + (row & 7) * 16;
-            const uint32_t step = f < kGmOutRows ? kGmA : kGmB;
+            const bool is_a = f < kGmOutRows;
 #pragma unroll
             for (int i = 0; i < kDigits; ++i) {  // digit i: byte 6 - i (the first with what lies above it)
                 constexpr int kTop = 0;
@@ -288,7 +303,9 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
                     const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&t2), off);
                     h[e] = *reinterpret_cast<const uint32_t *>(&d);
                 }
-                *reinterpret_cast<uint4 *>(dst + i * step) = make_uint4(h[0], h[1], h[2], h[3]);
+                const uint32_t at = !is_a ? i * kGmB
+                                    : kStack ? (i >> 1) * kGmA + (i & 1) * (64 / 8) * (kGmRows * 16) : i * kGmA;
+                *reinterpret_cast<uint4 *>(dst + at) = make_uint4(h[0], h[1], h[2], h[3]);
             }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -296,6 +313,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
         __syncthreads();
     };
 
+    constexpr int kDrain = kStack ? 2 * kGmDrain : kGmDrain;
     constexpr uint32_t idesc = (1u << 4) | ((kGmN >> 3) << 17) | ((128u >> 4) << 24);  // FP16 x FP16 -> FP32
     int64_t acc_hi[16], acc_lo[16];  // warps 0..15: lane quarter warp % 4, 16 columns
 #pragma unroll
@@ -305,18 +323,21 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
     load(0);
     if (stages > 0) make(0);
     for (int t = 0; t < stages; ++t) {
-        const bool first = t % kGmDrain == 0;
-        if (tid == 0 && s_bad == 0) {
+        const bool first = t % kDrain == 0;
+        if (tid == kGmTasks && s_bad == 0) {
             csx::tc_fence_after();
             const uint32_t a0 = base + (t & 1) * kGmBuf, b0 = a0 + kDigits * kGmA;
-            for (int s = 0; s < kDigits; ++s)
-                for (int i = 0; i <= s; ++i)
-                    for (int ks = 0; ks < kGmRows / 16; ++ks)
-                        gm_mma(tmem + s * kGmN, csx::tc_sdesc(a0 + i * kGmA + ks * 256, 128, kGmRows * 16),
-                               csx::tc_sdesc(b0 + (s - i) * kGmB + ks * 256, 128, kGmRows * 16), idesc,
+            // consecutive MMAs go to different accumulators
+            for (int ks = 0; ks < kGmRows / 16; ++ks)
+                for (int i = 0; i < kDigits; i += kStack ? 2 : 1)
+                    for (int j = 0; i + j < kDigits; ++j)
+                        gm_mma(tmem + (i + j) * kGmN,
+                               csx::tc_sdesc(a0 + (kStack ? i >> 1 : i) * kGmA + ks * 256, 128, kGmRows * 16),
+                               csx::tc_sdesc(b0 + j * kGmB + ks * 256, 128, kGmRows * 16), idesc,
                                !(first && i == 0 && ks == 0));
             csx::tc_commit(csx::smem_u32(&s_mbar[t & 1]));
         }
+        __syncwarp();
         // the other buffer's MMAs (stage t - 1) were waited for below
         if (t + 1 < stages) make(t + 1);
         if (ok && !csx::mbar_wait(csx::smem_u32(&s_mbar[t & 1]), phase[t & 1])) {
@@ -329,7 +350,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
             ok = false;
             break;
         }
-        if (t % kGmDrain == kGmDrain - 1 || t + 1 == stages) {
+        if (t % kDrain == kDrain - 1 || t + 1 == stages) {
             const uint32_t ta = tmem + ((32u * (warp & 3)) << 16) + 16u * (warp >> 2);
             if (warp < 16) {
 #pragma unroll
@@ -338,7 +359,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
                     csx::tc_ld16(ta + s * kGmN, r);
 #pragma unroll
                     for (int c = 0; c < 16; ++c) {
-                        const int v = __float2int_rn(r[c]);
+                        const int v = s & 1 ? exact_int(r[c]) : __float2int_rn(r[c]);
                         if (s < 3) acc_hi[c] += static_cast<int64_t>(v) * (1 << (8 * (2 - s)));
                         else acc_lo[c] += static_cast<int64_t>(v) * (1 << (8 * (6 - s)));
                     }
@@ -355,6 +376,22 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
         }
     }
     const int row = 32 * (warp & 3) + lane;
+    if (kStack) {  // the rows above carry 2^-8 (their last 8 bits lie past 2^-62 and are dropped)
+        longlong2 *up = reinterpret_cast<longlong2 *>(bufs);  // no MMA reads the buffers any more
+        __syncthreads();
+        if (warp < 16 && row >= 64)
+#pragma unroll
+            for (int c = 0; c < 16; ++c) up[(row - 64) * kGmN + 16 * (warp >> 2) + c] = make_longlong2(acc_hi[c], acc_lo[c]);
+        __syncthreads();
+        if (warp < 16 && row < 64) {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                const longlong2 u = up[row * kGmN + 16 * (warp >> 2) + c];
+                acc_hi[c] += u.x >> 8;
+                acc_lo[c] += ((u.x & 255) << 24) + (u.y >> 8);
+            }
+        }
+    }
     if (warp < 16 && row < kGmOutRows) {
         longlong2 *dst = part + ((static_cast<int64_t>(blockIdx.x) * kGmBlocks + blockIdx.y) * kGmOutRows + row) * kGmN +
                          16 * (warp >> 2);

@@ -589,30 +589,28 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
                 cluster.map_shared_rank(Pb, dst)[i * kSolveNb + c] = A[solve_off(r, q) + k0 + c];
         }
         cluster.sync();
-        if (warp == 0) {  // the 4x4 diagonal block, every lane alike
-            double d[kSolveNb][kSolveNb], l[kSolveNb][kSolveNb], rc[kSolveNb];
-#pragma unroll
-            for (int a = 0; a < kSolveNb; ++a)
-#pragma unroll
-                for (int b = 0; b <= a; ++b) d[a][b] = a < nb ? Pb[(k0 + a) * kSolveNb + b] : (a == b ? 1.0 : 0.0);
+        // The 4x4 diagonal block by one warp, lane 4a + b with entry (a, b):
+        // an FP64 instruction takes its 64 cycles whether one lane or all are
+        // active, so the block's updates of one column are one instruction.
+        if (warp == 0) {
+            const int a = (lane >> 2) & 3, b = lane & 3;
+            double v = a >= b && a < nb ? Pb[(k0 + a) * kSolveNb + b] : (a == b ? 1.0 : 0.0);
+            double rc = 0.0, lm = 0.0;  // lane (a, k): l_ak
 #pragma unroll
             for (int k = 0; k < kSolveNb; ++k) {
-                if (!(d[k][k] > 0.0) && bad == 0) bad = k0 + k + 1;
-                rc[k] = pivot_rcp(d[k][k]);
-#pragma unroll
-                for (int a = k + 1; a < kSolveNb; ++a) l[a][k] = d[a][k] * rc[k];
-#pragma unroll
-                for (int a = k + 1; a < kSolveNb; ++a)
-#pragma unroll
-                    for (int b = k + 1; b <= a; ++b) d[a][b] = fma(-d[a][k], l[b][k], d[a][b]);
+                const double d = __shfl_sync(0xffffffffu, v, 5 * k);
+                if (!(d > 0.0) && bad == 0) bad = k0 + k + 1;
+                const double r = pivot_rcp(d);
+                if (b == k) rc = r;
+                const double l = v * r;  // lane (a, k): l_ak
+                if (b == k) lm = l;
+                const double uak = __shfl_sync(0xffffffffu, v, 4 * a + k);   // u_ak
+                const double lbk = __shfl_sync(0xffffffffu, l, 4 * b + k);   // l_bk
+                if (b > k && a >= b) v = fma(-uak, lbk, v);
             }
-            if (lane == 0) {
-#pragma unroll
-                for (int k = 0; k < kSolveNb; ++k) {
-                    s_r[k] = rc[k];
-#pragma unroll
-                    for (int a = k + 1; a < kSolveNb; ++a) s_l[a][k] = l[a][k];
-                }
+            if (lane < 16) {
+                if (a > b) s_l[a][b] = lm;
+                if (a == b) s_r[a] = rc;
             }
         }
         __syncthreads();
@@ -817,7 +815,9 @@ size_t gram_smem(int nf) { return static_cast<size_t>(kGramRows) * gram_nb(nf) *
 int enable_smem() {  // on the current device, every call (cheap)
     SG_CUDA(cudaFuncSetAttribute(sg_ridge_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(std::max(solve_smem(kMaxFeat), solve_smem(kFullFeat)))));
-    SG_CUDA(cudaFuncSetAttribute(sg_gram_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    SG_CUDA(cudaFuncSetAttribute(sg_gram_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kGmSmem)));
+    SG_CUDA(cudaFuncSetAttribute(sg_gram_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(kGmSmem)));
     SG_CUDA(cudaFuncSetAttribute(sg_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(gram_smem(kFullFeat))));
@@ -957,8 +957,9 @@ int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, co
         SG_CUDA(cudaGetLastError());
         const int64_t drain = kGmRows * kGmDrain;
         const int chunks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(kGmChunks, (n + drain - 1) / drain)));
-        sg_gram_mma_kernel<<<dim3(chunks, kGmBlocks), kGmThreads, kGmSmem, s>>>(ng, nf, d_genes, n, ldg, d_fit, range,
-                                                                                part);
+        const bool stack = kPairRows + ng - 16 + 1 <= 64;
+        (stack ? sg_gram_mma_kernel<true> : sg_gram_mma_kernel<false>)<<<dim3(chunks, kGmBlocks), kGmThreads, kGmSmem, s>>>(
+            ng, nf, d_genes, n, ldg, d_fit, range, part);
         SG_CUDA(cudaGetLastError());
         sg_gram_kernel<<<dim3(grid, ycols), threads, gram_smem(nf), s>>>(ng, nf, d_genes, n, ldg, d_fit, part_g, part_r,
                                                                         range);
