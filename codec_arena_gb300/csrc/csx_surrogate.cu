@@ -501,54 +501,66 @@ __host__ __device__ constexpr int solve_rows(int n, int r) {  // rows r, r + 8, 
 __host__ __device__ constexpr int solve_off(int r, int q) { return q * (r + 1) + kSolveCtas * (q * (q - 1) / 2); }
 constexpr size_t solve_smem(int n) {  // the largest CTA's rows, two column buffers, L's columns, the copy for n <= 166
     return (static_cast<size_t>(solve_off(kSolveCtas - 1, solve_rows(n, 0))) + 2ull * (n + 1) * kSolveNb +
-            static_cast<size_t>(n + 1) * kSolveNb + (n <= kMaxFeat ? static_cast<size_t>(tri(n)) : 0u)) *
+            static_cast<size_t>(n + 1) * kSolveNb + 3ull * (kFullFeat + 1) + 2 + (n <= kMaxFeat ? static_cast<size_t>(tri(n)) : 0u)) *
            sizeof(double);
 }
 
-// 1 / d for a pivot: a float reciprocal of the significand and two Newton
-// steps x += x (1 - m x), then the exponent: eight dependent operations where
-// the division takes some thirty. Within an ulp or two of 1 / d for the
-// exponents a normal equation's pivot can have; the division otherwise
-// (zero, negative, subnormal, infinite, NaN, or a reciprocal near underflow).
+// 1 / d for a pivot: a float reciprocal of the significand's leading bits and
+// two Newton steps x += x (1 - m x), then the exponent: four dependent FP64
+// operations of 64 cycles each, where the division takes 565 cycles. Within an
+// ulp or two of 1 / d for the exponents a normal equation's pivot can have; the
+// division otherwise (zero, negative, subnormal, infinite, NaN, or a reciprocal
+// near underflow). The float parts are read off and put back by integer
+// operations: the conversions run on the FP64 pipe too.
 __device__ __forceinline__ double pivot_rcp(double d) {
     const int64_t bits = __double_as_longlong(d);
     const int64_t e = bits >> 52;  // sign and biased exponent
     if (e < 2 || e > 2040) return 1.0 / d;
     const double m = __longlong_as_double((bits & 0x000fffffffffffffll) | 0x3ff0000000000000ll);
-    double x = static_cast<double>(__frcp_rn(static_cast<float>(m)));
+    const float mf = __uint_as_float(0x3f800000u | static_cast<uint32_t>((bits >> 29) & 0x7fffffu));
+    const uint32_t xf = __float_as_uint(__frcp_rn(mf));  // in (1/2, 1]
+    double x = __longlong_as_double((static_cast<int64_t>(xf) << 29) + (static_cast<int64_t>(1023 - 127) << 52));
     x = fma(x, fma(-m, x, 1.0), x);
     x = fma(x, fma(-m, x, 1.0), x);
     return __longlong_as_double(__double_as_longlong(x) - ((e - 1023) << 52));
 }
 
-// Lᵀ w = z by one warp: lane l holds z_l, z_{l+32}, ...; `row(i)` is L's row i.
-template <int kPer, class RowFn>
-__device__ __forceinline__ void back_substitute(int n, const double *zrow, RowFn row, double *__restrict__ w) {
-    const int lane = threadIdx.x & 31;
-    double z[kPer], cur[kPer], nxt[kPer];
-#pragma unroll
-    for (int m = 0; m < kPer; ++m) {
-        const int j = lane + 32 * m;
-        z[m] = j < n ? zrow[j] : 0.0;
-        cur[m] = j < n - 1 ? row(n - 1)[j] : 0.0;
-    }
-    for (int i = n - 1; i >= 0; --i) {
-#pragma unroll
-        for (int m = 0; m < kPer; ++m) {  // the next row's entries while this one is used
-            const int j = lane + 32 * m;
-            nxt[m] = j < i - 1 ? row(i - 1)[j] : 0.0;
+// Lᵀ w = z by one CTA, 32 unknowns at a time from the last: within a block one
+// warp takes an unknown per step, one FMA for all 32 lanes; then every warp
+// takes the block's unknowns off the ones before it, a warp per 32 of them and
+// half of the block. `row(i)` is L's row i; y has n entries in shared memory.
+template <class RowFn>
+__device__ void back_substitute(int n, double *y, double (*half)[kFullFeat + 1], RowFn row, double *__restrict__ w) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i0 = (n - 1) & ~31; i0 >= 0; i0 -= 32) {
+        const int cnt = min(32, n - i0);
+        if (warp == 0) {
+            double z = lane < cnt ? y[i0 + lane] : 0.0;
+            double l = lane < cnt - 1 ? row(i0 + cnt - 1)[i0 + lane] : 0.0;
+            for (int k = cnt - 1; k > 0; --k) {
+                const double nxt = lane < k - 1 ? row(i0 + k - 1)[i0 + lane] : 0.0;  // the next step's entries
+                const double wk = __shfl_sync(0xffffffffu, z, k);
+                if (lane < k) z = fma(-l, wk, z);
+                l = nxt;
+            }
+            if (lane < cnt) {
+                y[i0 + lane] = z;
+                w[i0 + lane] = z;
+            }
         }
-        double mine = 0.0;
-#pragma unroll
-        for (int m = 0; m < kPer; ++m)
-            if (m == i >> 5) mine = z[m];
-        const double wi = __shfl_sync(0xffffffffu, mine, i & 31);
-        if (lane == 0) w[i] = wi;
-#pragma unroll
-        for (int m = 0; m < kPer; ++m) {
-            z[m] = fma(-cur[m], wi, z[m]);
-            cur[m] = nxt[m];
+        __syncthreads();
+        const int groups = i0 >> 5;  // of 32 unknowns before the block
+        for (int t = warp; t < 2 * groups; t += kSolveThreads / 32) {
+            const int j = (t >> 1) * 32 + lane, h = t & 1;
+            const int k1 = min(cnt, 16 * h + 16);
+            double s = 0.0;
+#pragma unroll 8
+            for (int k = 16 * h; k < k1; ++k) s = fma(row(i0 + k)[j], y[i0 + k], s);
+            half[h][j] = s;
         }
+        __syncthreads();
+        for (int j = tid; j < i0; j += kSolveThreads) y[j] -= half[0][j] + half[1][j];
+        __syncthreads();
     }
 }
 
@@ -562,9 +574,11 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nrows = solve_rows(n, r);
     double *A = sm;                                              // this CTA's packed rows
-    double *P = sm + solve_off(kSolveCtas - 1, solve_rows(n, 0));  // two buffers of (n + 1) x 4 column entries
+    double *P = sm + ((solve_off(kSolveCtas - 1, solve_rows(n, 0)) + 1) & ~1);  // two buffers of (n + 1) x 4 column entries
     double *Lc = P + 2 * (n + 1) * kSolveNb;                     // the step's columns of L, all rows
-    double *Lfull = Lc + (n + 1) * kSolveNb;                     // n <= 166: L in one CTA for the last solve
+    double *zs = Lc + (n + 1) * kSolveNb;                        // the last solve's unknowns
+    auto *half = reinterpret_cast<double(*)[kFullFeat + 1]>(zs + kFullFeat + 1);
+    double *Lfull = zs + 3 * (kFullFeat + 1);                    // n <= 166: L in one CTA for the last solve
     for (int q = warp; q < nrows; q += kSolveThreads / 32) {
         const int i = r + kSolveCtas * q;
         double *row = A + solve_off(r, q);
@@ -582,11 +596,14 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
         double *Pb = P + buf * (n + 1) * kSolveNb;
         // own rows' entries of the four columns to every CTA
         const int q0 = k0 > r ? (k0 - r + kSolveCtas - 1) / kSolveCtas : 0;  // first own row >= k0
-        for (int e = tid; e < (nrows - q0) * kSolveNb * kSolveCtas; e += kSolveThreads) {
-            const int c = e & (kSolveNb - 1), dst = (e >> 2) & (kSolveCtas - 1), q = q0 + (e >> 5);
+        for (int e = tid; e < (nrows - q0) * 2 * kSolveCtas; e += kSolveThreads) {  // two columns each
+            const int c = 2 * (e & 1), dst = (e >> 1) & (kSolveCtas - 1), q = q0 + (e >> 4);
             const int i = r + kSolveCtas * q;
-            if (c < nb && k0 + c <= i)
-                cluster.map_shared_rank(Pb, dst)[i * kSolveNb + c] = A[solve_off(r, q) + k0 + c];
+            const double *src = A + solve_off(r, q) + k0 + c;
+            double2 v = make_double2(0.0, 0.0);
+            if (c < nb && k0 + c <= i) v.x = src[0];
+            if (c + 1 < nb && k0 + c + 1 <= i) v.y = src[1];
+            *reinterpret_cast<double2 *>(cluster.map_shared_rank(Pb, dst) + i * kSolveNb + c) = v;
         }
         cluster.sync();
         // The 4x4 diagonal block by one warp, lane 4a + b with entry (a, b):
@@ -595,21 +612,20 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
         if (warp == 0) {
             const int a = (lane >> 2) & 3, b = lane & 3;
             double v = a >= b && a < nb ? Pb[(k0 + a) * kSolveNb + b] : (a == b ? 1.0 : 0.0);
-            double rc = 0.0, lm = 0.0;  // lane (a, k): l_ak
+            double rc = 0.0;  // lane (a, k): 1 / d_k
 #pragma unroll
             for (int k = 0; k < kSolveNb; ++k) {
                 const double d = __shfl_sync(0xffffffffu, v, 5 * k);
+                // u_ak u_bk while the reciprocal is on its way
+                const double uu = __shfl_sync(0xffffffffu, v, 4 * a + k) * __shfl_sync(0xffffffffu, v, 4 * b + k);
                 if (!(d > 0.0) && bad == 0) bad = k0 + k + 1;
                 const double r = pivot_rcp(d);
                 if (b == k) rc = r;
-                const double l = v * r;  // lane (a, k): l_ak
-                if (b == k) lm = l;
-                const double uak = __shfl_sync(0xffffffffu, v, 4 * a + k);   // u_ak
-                const double lbk = __shfl_sync(0xffffffffu, l, 4 * b + k);   // l_bk
-                if (b > k && a >= b) v = fma(-uak, lbk, v);
+                if (b > k && a >= b) v = fma(-uu, r, v);
             }
+            const double l = v * rc;  // a > b: l_ab = u_ab / d_b
             if (lane < 16) {
-                if (a > b) s_l[a][b] = lm;
+                if (a > b) s_l[a][b] = l;
                 if (a == b) s_r[a] = rc;
             }
         }
@@ -651,17 +667,18 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
     cluster.sync();  // every row of L is final
     if (r == 0) {
         const double *zrow = cluster.map_shared_rank(A, n % kSolveCtas) + solve_off(n % kSolveCtas, n / kSolveCtas);
+        for (int j = tid; j < n; j += kSolveThreads) zs[j] = zrow[j];
         if (n <= kMaxFeat) {  // L into this CTA, then the solve on local rows
             for (int i = warp; i < n; i += kSolveThreads / 32) {
                 const double *src = cluster.map_shared_rank(A, i % kSolveCtas) + solve_off(i % kSolveCtas, i / kSolveCtas);
                 for (int j = lane; j < i; j += 32) Lfull[tri(i) + j] = src[j];
             }
             __syncthreads();
-            if (warp == 0)
-                back_substitute<(kMaxFeat + 31) / 32>(n, zrow, [&](int i) { return Lfull + tri(i); }, w);
-        } else if (warp == 0) {
-            back_substitute<(kFullFeat + 31) / 32>(
-                n, zrow,
+            back_substitute(n, zs, half, [&](int i) { return Lfull + tri(i); }, w);
+        } else {
+            __syncthreads();
+            back_substitute(
+                n, zs, half,
                 [&](int i) {
                     return cluster.map_shared_rank(A, i % kSolveCtas) + solve_off(i % kSolveCtas, i / kSolveCtas);
                 },
