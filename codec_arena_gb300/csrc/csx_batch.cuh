@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_batch_kernel(const __grid_
 
     // merge the buffer into the CTA's sorted list; publishes the island's threshold
     auto merge = [&]() {
-        cta_sort_desc(E, B.sort_n);
-        for (uint32_t i = s_kpad + tid; i < B.sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
+        cta_merge_top(E, s_kpad, B.sort_n, min(s_buf_n, B.sort_n - s_kpad));
         if (tid == 0) {
             s_buf_n = 0;
             const Entry kth = E[s_keep - 1];

@@ -122,8 +122,7 @@ __device__ __forceinline__ uint32_t warp_kth_largest(const uint32_t *v, uint32_t
 __device__ __noinline__ void prune_merge(const PruneArgs *A, Entry *E, uint32_t *sel, unsigned int *s_buf_n,
                                          unsigned long long *s_t1, unsigned long long *s_t2, float *s_ts) {
     const uint32_t tid = threadIdx.x;
-    cta_sort_desc(E, A->sort_n);
-    for (uint32_t i = A->kpad + tid; i < A->sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
+    cta_merge_top(E, A->kpad, A->sort_n, *s_buf_n);
     if (tid == 0) {
         *s_buf_n = 0;
         const Entry kth = E[A->keep - 1];
@@ -439,8 +438,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     uint64_t st = 0;  // state of the candidate's first draw
     uint32_t screened = 0, exact = 0;  // per thread: far below 2^32
     bool valid = false;
-    auto next_item = [&]() {
-        item = atomicAdd(&A.ctrl->next_item, 1u);
+    auto start_item = [&]() {
         valid = item < n_items;
         n_it = left = 0;  // a thread without work counts down from 2^32 and never passes
         if (valid) {
@@ -451,7 +449,12 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
             valid = left > 0;
         }
     };
-    next_item();
+    auto next_item = [&]() {
+        item = gridDim.x * kThreads + atomicAdd(&A.ctrl->next_item, 1u);
+        start_item();
+    };
+    item = A.ctrl->item_begin + tid * gridDim.x + blockIdx.x;  // the first: its place in the grid
+    start_item();
     unsigned int gk = 0;
     uint32_t round = 0, n1 = 0, n2 = 0;  // n1, n2: the warp's queue lengths
     const uint32_t lt = (1u << lane) - 1u;

@@ -72,6 +72,46 @@ __device__ void cta_sort_desc(Entry *E, uint32_t n) {
     }
 }
 
+// The CTA's merge: E[0..kpad) is its sorted list, bn entries (zeros after
+// them) lie in the buffer E[kpad..sort_n); afterwards the list holds the best
+// kpad of both, sorted, and the buffer is zero. Only the buffer's power of two
+// is sorted, then the larger of list entry i and buffer entry kpad - 1 - i
+// leaves the best kpad in bitonic order, and one bitonic merge sorts them.
+// Sorting list and buffer together (2048 entries at keep <= 1023: 66 steps of
+// 1024 exchanges) was most of a small screen's instructions: 162 us at 1e6
+// candidates, of which the merges took 90. bn is the same in every thread,
+// read after a barrier.
+__device__ __noinline__ void cta_merge_top(Entry *E, uint32_t kpad, uint32_t sort_n, uint32_t bn) {
+    uint32_t n = 32;
+    while (n < bn) n <<= 1;
+    if (kpad + n > sort_n) {  // a buffer past the last power of two it holds
+        cta_sort_desc(E, sort_n);
+        for (uint32_t i = kpad + threadIdx.x; i < sort_n; i += blockDim.x) E[i] = Entry{0ull, 0ull};
+        __syncthreads();
+        return;
+    }
+    Entry *buf = E + kpad;
+    cta_sort_desc(buf, n);
+    for (uint32_t i = threadIdx.x; i < kpad; i += blockDim.x) {
+        const Entry a = E[i], b = buf[kpad - 1 - i];  // sort_n >= 2 kpad
+        if (better(b, a)) E[i] = b;
+    }
+    __syncthreads();
+    for (uint32_t stride = kpad >> 1; stride > 0; stride >>= 1) {
+        for (uint32_t i = threadIdx.x; i < (kpad >> 1); i += blockDim.x) {
+            const uint32_t lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+            const Entry a = E[lo], b = E[hi];
+            if (better(b, a)) {
+                E[lo] = b;
+                E[hi] = a;
+            }
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) buf[i] = Entry{0ull, 0ull};
+    __syncthreads();
+}
+
 // The reference-order score of one candidate, out of line: it runs only for
 // candidates the filter cannot rule out, and keeping it out of the caller
 // stops the compiler from holding both evaluations' values live at once.
@@ -87,6 +127,7 @@ __device__ __noinline__ float exact_score_at(const ScreenArgs *__restrict__ A, c
 // FullScreenArgs, every candidate scored on the full surface.
 template <bool kFastDelta, class Args = ScreenArgs>
 __global__ void __launch_bounds__(kThreads, 3) screen_kernel(const __grid_constant__ Args A) {
+    constexpr bool kFull = sizeof(Args) == sizeof(FullScreenArgs);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Entry *E = reinterpret_cast<Entry *>(smem_raw);
     float *el = reinterpret_cast<float *>(E + A.sort_n);
@@ -107,7 +148,11 @@ __global__ void __launch_bounds__(kThreads, 3) screen_kernel(const __grid_consta
     __syncthreads();
 
     Entry *buf = E + A.kpad;
-    uint32_t item = atomicAdd(&A.ctrl->next_item, 1u);
+    // every thread's first item is its place in the grid, spread over the CTAs
+    // (the counter hands out the ones after): the threads' first requests to
+    // one counter took 60 us, more than a small screen's own work
+    const uint32_t n_threads = gridDim.x * kThreads;
+    uint32_t item = A.ctrl->item_begin + tid * gridDim.x + blockIdx.x;
     bool valid = item < n_items;
     uint64_t seed_t = 0, p = 0;
     uint32_t left = 0, dcand = 0, ddraw = 0;
@@ -132,8 +177,12 @@ __global__ void __launch_bounds__(kThreads, 3) screen_kernel(const __grid_consta
         const unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
         const int any = __syncthreads_or(valid || has_def);
         if (bn >= A.buf_cap / 2 || (!any && bn > 0)) {
-            cta_sort_desc(E, A.sort_n);
-            for (uint32_t i = A.kpad + tid; i < A.sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
+            if (kFull) {  // the full surface's loop spills 356 bytes next to cta_merge_top, 48 next to the sort
+                cta_sort_desc(E, A.sort_n);
+                for (uint32_t i = A.kpad + tid; i < A.sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
+            } else {
+                cta_merge_top(E, A.kpad, A.sort_n, min(bn, A.buf_cap));
+            }
             if (tid == 0) {
                 s_buf_n = 0;
                 const Entry kth = E[A.keep - 1];
@@ -186,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_kernel(const __grid_consta
             ++dcand;
             ++screened;
             if (--left == 0) {
-                item = atomicAdd(&A.ctrl->next_item, 1u);
+                item = n_threads + atomicAdd(&A.ctrl->next_item, 1u);
                 valid = item < n_items;
                 if (valid) {
                     const Item it = A.items[item];
@@ -241,7 +290,11 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
     __syncthreads();
 
     Entry *buf = E + A.kpad;
-    uint32_t item = atomicAdd(&A.ctrl->next_item, 1u);
+    // every thread's first item is its place in the grid, spread over the CTAs
+    // (the counter hands out the ones after): the threads' first requests to
+    // one counter took 60 us, more than a small screen's own work
+    const uint32_t n_threads = gridDim.x * kThreads;
+    uint32_t item = A.ctrl->item_begin + tid * gridDim.x + blockIdx.x;
     bool valid = item < n_items;
     uint64_t seed_t = 0, p = 0;
     uint32_t left = 0, dcand = 0, ddraw = 0;
@@ -272,8 +325,7 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
 
     // merge the buffer into the CTA's sorted list; publishes the threshold
     auto merge = [&]() {
-        cta_sort_desc(E, A.sort_n);
-        for (uint32_t i = A.kpad + tid; i < A.sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
+        cta_merge_top(E, A.kpad, A.sort_n, s_buf_n);
         if (tid == 0) {
             s_buf_n = 0;
             const Entry kth = E[A.keep - 1];
@@ -340,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
             ++dcand;
             ++screened;
             if (--left == 0) {
-                item = atomicAdd(&A.ctrl->next_item, 1u);
+                item = n_threads + atomicAdd(&A.ctrl->next_item, 1u);
                 valid = item < n_items;
                 if (valid) {
                     const Item it = A.items[item];
@@ -576,7 +628,11 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
     bool tc_ok = true;
 
     Entry *buf = E + A.kpad;
-    uint32_t item = atomicAdd(&A.ctrl->next_item, 1u);
+    // every thread's first item is its place in the grid, spread over the CTAs
+    // (the counter hands out the ones after): the threads' first requests to
+    // one counter took 60 us, more than a small screen's own work
+    const uint32_t n_threads = gridDim.x * kThreads;
+    uint32_t item = A.ctrl->item_begin + tid * gridDim.x + blockIdx.x;
     bool valid = item < n_items;
     uint64_t seed_t = 0, p = 0;
     uint32_t left = 0, dcand = 0, ddraw = 0;
@@ -609,8 +665,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
 
     // merge the buffer into the CTA's sorted list; publishes the threshold
     auto merge = [&]() {
-        cta_sort_desc(E, A.sort_n);
-        for (uint32_t i = A.kpad + tid; i < A.sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
+        cta_merge_top(E, A.kpad, A.sort_n, s_buf_n);
         if (tid == 0) {
             s_buf_n = 0;
             const Entry kth = E[A.keep - 1];
@@ -702,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
                 ++dcand;
                 ++screened;
                 if (--left == 0) {
-                    item = atomicAdd(&A.ctrl->next_item, 1u);
+                    item = n_threads + atomicAdd(&A.ctrl->next_item, 1u);
                     valid = item < n_items;
                     if (valid) {
                         const Item it = A.items[item];
