@@ -324,11 +324,12 @@ __global__ void __launch_bounds__(kThreads, 3) screen_batch_kernel(const __grid_
     }
 }
 
-__global__ void merge_batch_kernel(const IslandDev *__restrict__ isl, uint32_t nl, int b_to_a) {
+__global__ void __launch_bounds__(512) merge_batch_kernel(const IslandDev *__restrict__ isl, uint32_t nl,
+                                                          uint32_t fan, int b_to_a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const IslandDev &I = isl[blockIdx.y];
-    merge_pair(b_to_a ? I.lists_b : I.lists_a, nl, b_to_a ? I.lists_a : I.lists_b, I.kpad, blockIdx.x,
-               reinterpret_cast<Entry *>(smem_raw));
+    merge_lists(b_to_a ? I.lists_b : I.lists_a, nl, b_to_a ? I.lists_a : I.lists_b, I.kpad, fan, blockIdx.x,
+                reinterpret_cast<Entry *>(smem_raw));
 }
 
 template <bool kFastDelta>
@@ -492,9 +493,7 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
     L->grid = per_sm * cx.num_sms;
     if (!L->prune)
         for (int i = 0; i < n; ++i) L->pl[i].grid = L->grid;
-    const size_t msmem = 2ull * L->kpad_max * sizeof(Entry);
-    CSX_CUDA(cudaFuncSetAttribute(merge_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(msmem)));
+    CSX_CUDA(cudaFuncSetAttribute(merge_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 << 10));
 
     // carve: a sizing pass, then the real one
     const uint32_t nl = static_cast<uint32_t>(L->grid);
@@ -603,7 +602,6 @@ int batch_enqueue(Context &cx, const BatchLayout &L, cudaStream_t st, bool captu
         cudaStream_t a = cx.aux[i];
         const IslandBufs &b = L.b[i];
         const Plan &pl = L.pl[i];
-        const StreamGeom &g = pl.g;
         const int ne = L.ne[i];
         CSX_CUDA(cudaStreamWaitEvent(a, cx.ev_fork, 0));
         prep_elites_kernel<<<unit_blocks(static_cast<uint64_t>(ne + 1) * kNtot, 256), 256, 0, a>>>(
@@ -648,12 +646,13 @@ int batch_enqueue(Context &cx, const BatchLayout &L, cudaStream_t st, bool captu
         CSX_CUDA(cudaGetLastError());
         nk += 2;
     }
-    const size_t msmem = 2ull * L.kpad_max * sizeof(Entry);
+    const size_t msmem = merge_smem(L.kpad_max);
+    const uint32_t fan = merge_fan(L.kpad_max);
     uint32_t nl = static_cast<uint32_t>(L.grid);
     int in_b = 0;
     while (nl > 1) {
-        const uint32_t m = (nl + 1) / 2;
-        merge_batch_kernel<<<dim3(m, n), 256, msmem, st>>>(L.d_isl, nl, in_b);
+        const uint32_t m = (nl + fan - 1) / fan;
+        merge_batch_kernel<<<dim3(m, n), 512, msmem, st>>>(L.d_isl, nl, fan, in_b);
         CSX_CUDA(cudaGetLastError());
         ++nk;
         in_b ^= 1;
@@ -807,7 +806,8 @@ int csx_screen_batch(int n_islands, const csx_cfg *cfgs, const csx_model *models
     // the merge tree leaves each island's final list in lists_b after an odd
     // number of levels
     bool in_b = false;
-    for (uint32_t nl = static_cast<uint32_t>(L.grid); nl > 1; nl = (nl + 1) / 2) in_b = !in_b;
+    const uint32_t fan = merge_fan(L.kpad_max);
+    for (uint32_t nl = static_cast<uint32_t>(L.grid); nl > 1; nl = (nl + fan - 1) / fan) in_b = !in_b;
     off = 0;
     for (int i = 0; i < n_islands && !bad; ++i) {
         const uint64_t cnt = std::min<uint64_t>(res[4 * i], std::min<uint64_t>(cfgs[i].keep, cfgs[i].lambda));

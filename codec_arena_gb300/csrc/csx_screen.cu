@@ -29,7 +29,7 @@
 //             candidates in registers; those that beat the CTA's threshold go
 //             to a shared-memory buffer that is merged into the CTA's sorted
 //             top-K list (bitonic sort). HBM sees only items and survivors.
-//  6. merge   a tree of pairwise bitonic merges reduces the CTA lists.
+//  6. merge   a tree of bitonic merges reduces the CTA lists.
 //  7. regen   the K survivors are re-synthesised from (stream, draw) to
 //             recover genes and lineage; the score is re-checked bit for bit.
 //
@@ -97,6 +97,8 @@ struct Context {
     cudaStream_t pst = nullptr;     // private stream of the host batch call
     cudaGraphExec_t gexec = nullptr;
     csx_batch_info binfo{};
+    cudaStream_t hst = nullptr;     // private stream of the host calls
+    unsigned char *hpin = nullptr;  // their page-locked staging: result words, an Entry, survivors, elites
     const Entry *fin = nullptr;  // final list of the last single screen (kpad entries)
     uint32_t fin_kpad = 0;
 };
@@ -576,13 +578,13 @@ ScreenArgs screen_args(const csx_cfg &cfg, const csx_model &model, const SynthCo
 // *fin receives the buffer holding the final list.
 int enqueue_merge(Entry *cur, Entry *nxt, uint32_t nl, uint32_t kpad, cudaStream_t st, Entry **fin,
                   uint32_t *launches) {
-    const size_t msmem = 2ull * kpad * sizeof(Entry);
-    CSX_CUDA(cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(msmem)));
+    const size_t msmem = merge_smem(kpad);
+    CSX_CUDA(cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 << 10));
+    const uint32_t fan = merge_fan(kpad);
     uint32_t n = nl;
     while (n > 1) {
-        const uint32_t m = (n + 1) / 2;
-        merge_kernel<<<m, 256, msmem, st>>>(cur, n, nxt, kpad);
+        const uint32_t m = (n + fan - 1) / fan;
+        merge_kernel<<<m, 512, msmem, st>>>(cur, n, nxt, kpad);
         CSX_CUDA(cudaGetLastError());
         ++*launches;
         std::swap(cur, nxt);
@@ -955,6 +957,7 @@ struct ScreenBufs {
     const unsigned int *tribes;
     const Entry *fin;  // the final top-kpad list (its entry past the survivors shows a tie at the K-th score)
     uint32_t kpad;
+    const Entry *next = nullptr;  // that entry on the host, where the caller has read it already
 };
 
 int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_model_full *full, int ne,
@@ -969,8 +972,12 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
     bool boundary = false;
     if (cnt < bufs.kpad && bufs.fin) {
         Entry next{};
-        CSX_CUDA(cudaMemcpyAsync(&next, bufs.fin + cnt, sizeof(Entry), cudaMemcpyDeviceToHost, st));
-        CSX_CUDA(cudaStreamSynchronize(st));
+        if (bufs.next) {
+            next = *bufs.next;
+        } else {
+            CSX_CUDA(cudaMemcpyAsync(&next, bufs.fin + cnt, sizeof(Entry), cudaMemcpyDeviceToHost, st));
+            CSX_CUDA(cudaStreamSynchronize(st));
+        }
         boundary = next.k1 != 0ull && static_cast<uint32_t>(next.k1 >> 32) == tau;
     }
     std::set<uint64_t> S;
@@ -1101,6 +1108,8 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
     return CSX_OK;
 }
 
+constexpr size_t kHostSurv = 64;  // offset of the survivors in the host staging
+
 // csx_screen / csx_screen_range: host buffers, a private stream, synchronous.
 int screen_host(const csx_cfg *cfg, const csx_model *model, const csx_genome *elites, int n_elites,
                 uint64_t t_begin, uint64_t t_end, csx_survivor *out, uint64_t out_cap, uint64_t *n_out,
@@ -1124,37 +1133,52 @@ int screen_host(const csx_cfg *cfg, const csx_model *model, const csx_genome *el
     CSX_CUDA(cx->genomes.ensure(static_cast<size_t>(n_elites) * sizeof(csx_genome)));
     CSX_CUDA(cx->surv.ensure(static_cast<size_t>(cfg->keep) * sizeof(csx_survivor)));
     CSX_CUDA(cx->result.ensure(4 * sizeof(uint64_t)));
-    cudaStream_t st = nullptr;
-    CSX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    // The stream and the staging are kept for the life of the context (about 1
+    // MB, the largest keep and elite count); the lock above is held until the
+    // stream has run dry, so a call finds both idle.
+    if (!cx->hst) CSX_CUDA(cudaStreamCreateWithFlags(&cx->hst, cudaStreamNonBlocking));
+    if (!cx->hpin)
+        CSX_CUDA(cudaMallocHost(&cx->hpin, kHostSurv + kMaxKeep * sizeof(csx_survivor) + kMaxElites * sizeof(csx_genome)));
+    cudaStream_t st = cx->hst;
     auto *dg = static_cast<csx_genome *>(cx->genomes.p);
     auto *ds = static_cast<csx_survivor *>(cx->surv.p);
     auto *dr = static_cast<unsigned long long *>(cx->result.p);
-    unsigned long long res[4] = {0, 0, 0, 0};
-    cudaError_t e = cudaMemcpyAsync(dg, elites, static_cast<size_t>(n_elites) * sizeof(csx_genome),
+    const auto *res = reinterpret_cast<const unsigned long long *>(cx->hpin);
+    auto *next = reinterpret_cast<Entry *>(cx->hpin + 4 * sizeof(uint64_t));
+    auto *hsurv = reinterpret_cast<csx_survivor *>(cx->hpin + kHostSurv);
+    auto *hgen = reinterpret_cast<csx_genome *>(hsurv + kMaxKeep);
+    const bool give = !(cfg->flags & CSX_FLAG_AS_SHIPPED);
+    std::memcpy(hgen, elites, static_cast<size_t>(n_elites) * sizeof(csx_genome));
+    cudaError_t e = cudaMemcpyAsync(dg, hgen, static_cast<size_t>(n_elites) * sizeof(csx_genome),
                                     cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
         rc = enqueue_screen(*cx, *cfg, *model, dg, n_elites, ds, dr, st, t_begin, t_end, full, shard);
+        // everything the host reads in one trip: the result words, the final
+        // list's entry past the survivors (exact ties) and the survivors
+        const bool has_next = rc == CSX_OK && keep_n < cx->fin_kpad;
         if (rc == CSX_OK) {
-            e = cudaMemcpyAsync(res, dr, sizeof(res), cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            e = cudaMemcpyAsync(cx->hpin, dr, 4 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess && give && has_next)
+                e = cudaMemcpyAsync(next, cx->fin + keep_n, sizeof(Entry), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess && give)
+                e = cudaMemcpyAsync(hsurv, ds, keep_n * sizeof(csx_survivor), cudaMemcpyDeviceToHost, st);
+        }
+        const cudaError_t es = cudaStreamSynchronize(st);  // also where something failed: the staging is idle again
+        if (e == cudaSuccess) e = es;
+        if (rc == CSX_OK && e == cudaSuccess && res[2] == 0 && give) {
             const uint64_t cnt = std::min<uint64_t>(res[0], keep_n);
-            if (e == cudaSuccess && res[2] == 0 && cnt > 0 && !(cfg->flags & CSX_FLAG_AS_SHIPPED)) {
-                e = cudaMemcpyAsync(out, ds, cnt * sizeof(csx_survivor), cudaMemcpyDeviceToHost, st);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-                // whole streams only: an item share does not hold a stream's heap
-                if (e == cudaSuccess && shard.count == 1 &&
-                    !(cfg->flags & (CSX_FLAG_TC_BF16 | CSX_FLAG_TC_FP16)))
-                    rc = fix_ties(*cx, *cfg, *model, full, n_elites, t_begin, t_end, out, cnt,
-                                  ScreenBufs{static_cast<const float *>(cx->tab.p),
-                                             static_cast<const Item *>(cx->items.p), res[3],
-                                             static_cast<const unsigned long long *>(cx->ids.p),
-                                             static_cast<const unsigned int *>(cx->tribes.p), cx->fin,
-                                             cx->fin_kpad},
-                                  st);
-            }
+            std::memcpy(out, hsurv, cnt * sizeof(csx_survivor));
+            // whole streams only: an item share does not hold a stream's heap
+            if (cnt > 0 && shard.count == 1 && !(cfg->flags & (CSX_FLAG_TC_BF16 | CSX_FLAG_TC_FP16)))
+                rc = fix_ties(*cx, *cfg, *model, full, n_elites, t_begin, t_end, out, cnt,
+                              ScreenBufs{static_cast<const float *>(cx->tab.p),
+                                         static_cast<const Item *>(cx->items.p), res[3],
+                                         static_cast<const unsigned long long *>(cx->ids.p),
+                                         static_cast<const unsigned int *>(cx->tribes.p), cx->fin, cx->fin_kpad,
+                                         cnt == keep_n && has_next ? next : nullptr},
+                              st);
         }
     }
-    cudaStreamDestroy(st);
     if (e != cudaSuccess) {
         std::fprintf(stderr, "csx: %s\n", cudaGetErrorString(e));
         return CSX_ERR_CUDA;

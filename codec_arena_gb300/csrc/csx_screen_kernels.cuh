@@ -420,42 +420,59 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
 
 // ---- 5. merge tree ------------------------------------------------------------------
 
-// Merge lists 2j and 2j+1 of `in` (nl lists of kpad entries, best first) into
-// list j of `out`; S holds 2 * kpad entries of shared memory.
-__device__ void merge_pair(const Entry *__restrict__ in, uint32_t nl, Entry *__restrict__ out, uint32_t kpad,
-                           uint32_t j, Entry *S) {
-    const uint32_t a = 2 * j, b = 2 * j + 1;
-    const Entry *la = in + static_cast<size_t>(a) * kpad;
-    Entry *o = out + static_cast<size_t>(j) * kpad;
-    if (b >= nl) {
-        for (uint32_t i = threadIdx.x; i < kpad; i += blockDim.x) o[i] = la[i];
-        return;
-    }
-    const Entry *lb = in + static_cast<size_t>(b) * kpad;
-    for (uint32_t i = threadIdx.x; i < kpad; i += blockDim.x) {
-        S[i] = la[i];
-        S[2 * kpad - 1 - i] = lb[i];  // descending ++ ascending: bitonic
-    }
+// Lists per CTA of a merge level: what 128 KB of shared memory hold, two to
+// eight. Three levels of up to eight lists reduce a screen's 304 to 456 lists
+// where pairs took nine launches (39 us of a 2e5-candidate screen's 180).
+__host__ __device__ constexpr uint32_t merge_fan(uint32_t kpad) {
+    uint32_t f = 8;
+    while (f > 2 && f * kpad * sizeof(Entry) > (128u << 10)) f >>= 1;
+    return f;
+}
+__host__ __device__ constexpr size_t merge_smem(uint32_t kpad) { return merge_fan(kpad) * static_cast<size_t>(kpad) * sizeof(Entry); }
+
+// Merge lists [j fan, (j + 1) fan) of `in` (nl lists of kpad entries, best
+// first; past the last, nothing) into list j of `out`, in shared memory S: a
+// tree of pairs, each the larger of entry i and the other list's entry kpad -
+// 1 - i (the best kpad, bitonic) and a bitonic merge.
+__device__ void merge_lists(const Entry *__restrict__ in, uint32_t nl, Entry *__restrict__ out, uint32_t kpad,
+                            uint32_t fan, uint32_t j, Entry *S) {
+    const uint32_t first = j * fan;
+    const uint32_t n = min(fan, nl - first);
+    const Entry *src = in + static_cast<size_t>(first) * kpad;
+    for (uint32_t i = threadIdx.x; i < fan * kpad; i += blockDim.x) S[i] = i < n * kpad ? src[i] : Entry{0ull, 0ull};
     __syncthreads();
-    for (uint32_t stride = kpad; stride > 0; stride >>= 1) {
-        for (uint32_t i = threadIdx.x; i < kpad; i += blockDim.x) {
-            const uint32_t lo = 2 * i - (i & (stride - 1));
-            const uint32_t hi = lo + stride;
-            const Entry x = S[lo], y = S[hi];
-            if (better(y, x)) {
-                S[lo] = y;
-                S[hi] = x;
-            }
+    const uint32_t half = kpad >> 1;
+    for (uint32_t d = 1; d < n; d <<= 1) {  // list g of every 2 d takes list g + d
+        const uint32_t pairs = fan / (2 * d);
+        for (uint32_t i = threadIdx.x; i < pairs * kpad; i += blockDim.x) {
+            Entry *a = S + static_cast<size_t>(i / kpad) * 2 * d * kpad;
+            const uint32_t q = i & (kpad - 1);
+            const Entry x = a[q], y = a[d * kpad + kpad - 1 - q];
+            if (better(y, x)) a[q] = y;
         }
         __syncthreads();
+        for (uint32_t stride = half; stride > 0; stride >>= 1) {
+            for (uint32_t i = threadIdx.x; i < pairs * half; i += blockDim.x) {
+                Entry *a = S + static_cast<size_t>(i / half) * 2 * d * kpad;
+                const uint32_t q = i & (half - 1);
+                const uint32_t lo = 2 * q - (q & (stride - 1)), hi = lo + stride;
+                const Entry x = a[lo], y = a[hi];
+                if (better(y, x)) {
+                    a[lo] = y;
+                    a[hi] = x;
+                }
+            }
+            __syncthreads();
+        }
     }
+    Entry *o = out + static_cast<size_t>(j) * kpad;
     for (uint32_t i = threadIdx.x; i < kpad; i += blockDim.x) o[i] = S[i];
 }
 
-__global__ void merge_kernel(const Entry *__restrict__ in, uint32_t nl, Entry *__restrict__ out,
-                             uint32_t kpad) {
+__global__ void __launch_bounds__(512) merge_kernel(const Entry *__restrict__ in, uint32_t nl,
+                                                    Entry *__restrict__ out, uint32_t kpad) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    merge_pair(in, nl, out, kpad, blockIdx.x, reinterpret_cast<Entry *>(smem_raw));
+    merge_lists(in, nl, out, kpad, merge_fan(kpad), blockIdx.x, reinterpret_cast<Entry *>(smem_raw));
 }
 
 // ---- 6. regenerate survivors ------------------------------------------------------
