@@ -159,12 +159,24 @@ __global__ void walk_kernel(SynthConst sc, StreamGeom g, SegRec *__restrict__ re
         const uint64_t m = k >> g.d_log2;  // k is a multiple of D here
         if (m < g.ckcap) ckp[m] = e - static_cast<uint64_t>(rem);
         const uint32_t n = static_cast<uint32_t>(min(static_cast<uint64_t>(D), limit - k));
+        // Two candidates per step: the second's tests are hashed beside the
+        // first's as if that were the common 62 draws (97% are), and taken
+        // only if it was. A step is a chain of one hash and a few operations,
+        // so the second candidate costs little but its own instructions.
         uint32_t j = 0;
         do {
-            const uint32_t len = cand_len(sc, st);
+            const uint64_t st1 = st + 62 * kGolden;
+            const bool i0 = (draw_vh(st + 2 * kGolden) >> 8) < sc.imm_thr;
+            const bool j0 = (draw_vh(st + 61 * kGolden) >> 8) < sc.jump_thr;
+            const bool i1 = (draw_vh(st1 + 2 * kGolden) >> 8) < sc.imm_thr;
+            const bool j1 = (draw_vh(st1 + 61 * kGolden) >> 8) < sc.jump_thr;
+            const bool two = !i0 && !j0 && j + 1 < n && rem > 62;
+            bool imm = two ? i1 : i0, jump = two ? j1 : j0;
+            if (imm) jump = (draw_vh((two ? st1 : st) + 32 * kGolden) >> 8) < sc.jump_thr;
+            const uint32_t len = (two ? 62u : 0u) + (imm ? 33u : 62u) + (jump ? 2u : 0u);
             rem -= static_cast<int32_t>(len);
             st += static_cast<uint64_t>(len) * kGolden;
-            ++j;
+            j += two ? 2u : 1u;
         } while (j < n && rem > 0);
         k += j;
     }
@@ -177,74 +189,37 @@ __global__ void walk_kernel(SynthConst sc, StreamGeom g, SegRec *__restrict__ re
     recs[s] = r;
 }
 
-// Speculative run of one chain by a half-warp: lane j tests the start x + 62 j
-// assuming every earlier step of the run is the common 62-draw one (no
-// immigrant, no jump). f = first lane whose tests say otherwise (16 if none);
-// the run's starts are x + 62 i for i <= min(f, 15) and the next start after
-// it is x + 62 f + len (or x + 62*16).
+// Speculative run of one chain by a warp: lane j tests the start 62 j draws
+// past the one with state st, assuming every earlier step of the run is the
+// common 62-draw one (no immigrant, no jump). The run's starts end at the first
+// lane whose tests say otherwise, whose own length ends the run. Two hashes
+// side by side, a third for an immigrant's jump test while the ballot is on its
+// way.
 struct Run {
-    uint32_t n;     // starts in the run
-    uint64_t next;  // the chain's next start after the run
+    uint32_t n;    // starts in the run: 62 apart
+    uint32_t adv;  // draws from its first start to the chain's next start after it
 };
 
-__device__ __forceinline__ Run half_run(const SynthConst &C, uint64_t seed_t, uint64_t x, int j, int half) {
-    const uint64_t pj = x + 62ull * static_cast<uint64_t>(j);
-    const uint64_t s0 = seed_t + (pj + 1) * kGolden;               // state of draw pj
-    const bool imm = (draw_vh(s0 + 2 * kGolden) >> 8) < C.imm_thr;  // draw pj + 2
-    const bool jb = (draw_vh(s0 + 61 * kGolden) >> 8) < C.jump_thr; // draw pj + 61
-    const uint32_t bn = (__ballot_sync(0xffffffffu, imm || jb) >> (16 * half)) & 0xffffu;
-    const uint32_t bi = (__ballot_sync(0xffffffffu, imm) >> (16 * half)) & 0xffffu;
-    Run r;
-    if (bn == 0) {
-        r.n = 16;
-        r.next = x + 62ull * 16;
-        return r;
-    }
-    const uint32_t f = static_cast<uint32_t>(__ffs(bn) - 1);
-    const uint64_t pf = x + 62ull * f;
-    uint32_t len = 64;            // a jump after a crossover candidate
-    if ((bi >> f) & 1u) {         // an immigrant: its jump test is at draw + 32
-        const bool ja = (draw_vh(seed_t + (pf + 33) * kGolden) >> 8) < C.jump_thr;
-        len = ja ? 35 : 33;
-    }
-    r.n = f + 1;
-    r.next = pf + len;
-    return r;
-}
-
-// The same speculative run by the whole warp: lane j tests x + 62 j, the run
-// has up to 32 starts.
-__device__ __forceinline__ Run warp_run(const SynthConst &C, uint64_t seed_t, uint64_t x, int lane) {
-    const uint64_t pj = x + 62ull * static_cast<uint64_t>(lane);
-    const uint64_t s0 = seed_t + (pj + 1) * kGolden;
+__device__ __forceinline__ Run warp_run(const SynthConst &C, uint64_t st, uint64_t lane_off, int lane) {
+    const uint64_t s0 = st + lane_off;
     const bool imm = (draw_vh(s0 + 2 * kGolden) >> 8) < C.imm_thr;
-    const bool jb = (draw_vh(s0 + 61 * kGolden) >> 8) < C.jump_thr;
-    const uint32_t bn = __ballot_sync(0xffffffffu, imm || jb);
-    const uint32_t bi = __ballot_sync(0xffffffffu, imm);
+    bool jump = (draw_vh(s0 + 61 * kGolden) >> 8) < C.jump_thr;
+    const uint32_t bn = __ballot_sync(0xffffffffu, imm || jump);
+    if (imm) jump = (draw_vh(s0 + 32 * kGolden) >> 8) < C.jump_thr;
+    const uint32_t f = bn ? static_cast<uint32_t>(__ffs(bn) - 1) : 31u;
     Run r;
-    if (bn == 0) {
-        r.n = 32;
-        r.next = x + 62ull * 32;
-        return r;
-    }
-    const uint32_t f = static_cast<uint32_t>(__ffs(bn) - 1);
-    const uint64_t pf = x + 62ull * f;
-    uint32_t len = 64;
-    if ((bi >> f) & 1u) {
-        const bool ja = (draw_vh(seed_t + (pf + 33) * kGolden) >> 8) < C.jump_thr;
-        len = ja ? 35 : 33;
-    }
     r.n = f + 1;
-    r.next = pf + len;
+    r.adv = __shfl_sync(0xffffffffu, 62u * static_cast<uint32_t>(lane) + (imm ? 33u : 62u) + (jump ? 2u : 0u),
+                        static_cast<int>(f));
     return r;
 }
 
-// Checkpoint (start of every D-th candidate) among the starts [k, k + cnt),
-// which lie at x + 62 (idx - k); D >= 64 > cnt, so at most one.
-__device__ __forceinline__ void record_ckpt(uint64_t *ckp, uint32_t ckcap, uint32_t dl, uint64_t k,
-                                            uint64_t cnt, uint64_t x) {
-    const uint64_t mk = ((k + (1ull << dl) - 1) >> dl) << dl;
-    if (mk < k + cnt && (mk >> dl) < ckcap) ckp[mk >> dl] = x + 62ull * (mk - k);
+// Checkpoints (every D-th start) among the starts [k, k + cnt) of a run from x.
+__device__ __forceinline__ void record_run(uint64_t *ckp, uint32_t ckcap, uint32_t dl, uint64_t k, uint32_t cnt,
+                                           uint64_t x, int lane) {
+    const uint64_t kl = k + static_cast<uint32_t>(lane);
+    if (static_cast<uint32_t>(lane) < cnt && (kl & ((1ull << dl) - 1)) == 0 && (kl >> dl) < ckcap)
+        ckp[kl >> dl] = x + 62ull * static_cast<uint32_t>(lane);
 }
 
 // One warp per link of segment s and s+1 (same stream). Segment s's chain is
@@ -255,15 +230,14 @@ __device__ __forceinline__ void record_ckpt(uint64_t *ckp, uint32_t ckcap, uint3
 // one s's chain lands on, and only s's chain is walked. (Walking both chains
 // to their first shared start costs about four times the instructions.) If
 // s's chain passes the last of those checkpoints first, the meeting lies past
-// s+1's exit: the two chains then advance together, 16 lanes each, from s's
-// position and that checkpoint. Below M = the nearer of the two next starts
-// both chains' starts are known, and within a run they are 62 apart, so the
-// first shared start below M is y if (y - x) is a multiple of 62 inside x's
-// run (or symmetrically). Otherwise both move to their first start at or past
-// M and the search goes on.
+// s+1's exit: the two chains then advance in turn, a run of the one that is
+// behind at a time, from s's position and that checkpoint. Below the nearer of
+// the two next starts both chains' starts are in their current runs, 62 apart,
+// so the runs share a start exactly if the later run's first start lies a
+// multiple of 62 into the other run.
 __global__ void link_kernel(SynthConst sc, StreamGeom g, SegRec *__restrict__ recs,
                             uint64_t *__restrict__ ck, Ctrl *__restrict__ ctrl) {
-    const int lane = threadIdx.x & 31, half = lane >> 4, j = lane & 15;
+    const int lane = threadIdx.x & 31;
     const uint64_t s = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (s >= g.n_seg) return;  // whole warps leave together
     SegRec r = recs[s];
@@ -280,82 +254,82 @@ __global__ void link_kernel(SynthConst sc, StreamGeom g, SegRec *__restrict__ re
     const uint64_t *cky = ck + (s + 1) * g.ckcap;
     const uint32_t D = 1u << g.d_log2;
     const uint32_t mcap = min(g.ckcap, (n_next + D - 1) >> g.d_log2);  // >= 1: a chain has a start
-    uint32_t cm = 0;
-    uint64_t cy = cky[0];
-    while (cm + 1 < mcap && cy < x) cy = cky[++cm];
-    uint64_t y = cy, kb = static_cast<uint64_t>(cm) << g.d_log2;  // guess chain of s + 1
     uint64_t steps = 0;
     bool fail = false;
-    if (cy >= x) {
+    // Each lane holds one of the next 32 checkpoints, so that a run's starts are
+    // compared with all of them at once.
+    const uint64_t lane_off = 62ull * static_cast<uint64_t>(lane) * kGolden;
+    const uint64_t last = cky[mcap - 1];
+    uint64_t y = last, kb = static_cast<uint64_t>(mcap - 1) << g.d_log2;  // guess chain of s + 1
+    bool met = false;
+    if (x <= last) {
+        uint32_t cm = 0;  // first checkpoint of the window
+        uint64_t ckw = cky[min(static_cast<uint32_t>(lane), mcap - 1)];
+        uint64_t st = seed_t + (x + 1) * kGolden;
         for (;;) {
-            const Run run = warp_run(sc, seed_t, x, lane);
-            const uint64_t d = cy - x;  // < one checkpoint gap + a run: fits 32 bits
-            const uint32_t dq = static_cast<uint32_t>(d) / 62u;
-            if (static_cast<uint32_t>(d) == dq * 62u && dq < run.n) {  // lands on it
-                if (lane == 0) record_ckpt(ckp, g.ckcap, g.d_log2, k, dq, x);
-                k += dq;
-                x = cy;
+            const Run run = warp_run(sc, st, lane_off, lane);
+            // the first start that is a checkpoint (the window's lanes ascend)
+            const uint64_t d64 = ckw - x;
+            const uint32_t d = static_cast<uint32_t>(d64), dq = d / 62u;
+            const uint32_t bh = __ballot_sync(0xffffffffu, d64 < 62u * 32u && dq * 62u == d && dq < run.n);
+            const int h = bh ? __ffs(bh) - 1 : 0;
+            const uint32_t take = bh ? __shfl_sync(0xffffffffu, dq, h) : run.n;
+            record_run(ckp, g.ckcap, g.d_log2, k, take, x, lane);
+            k += take;
+            if (bh) {
+                x += 62ull * take;
+                kb = static_cast<uint64_t>(min(cm + static_cast<uint32_t>(h), mcap - 1)) << g.d_log2;
+                met = true;
                 break;
             }
-            if (lane == 0) record_ckpt(ckp, g.ckcap, g.d_log2, k, run.n, x);
-            k += run.n;
-            x = run.next;
+            x += run.adv;
+            st += static_cast<uint64_t>(run.adv) * kGolden;
             steps += run.n;
-            while (cy < x && cm + 1 < mcap) cy = cky[++cm];
-            if (cy < x) {  // past the last checkpoint: meet beyond it (below)
-                y = cy;
-                kb = static_cast<uint64_t>(cm) << g.d_log2;
+            if (steps > g.link_cap) {
+                fail = true;
                 break;
+            }
+            if (x > last) break;  // past the last checkpoint: meet beyond it (below)
+            while (__shfl_sync(0xffffffffu, ckw, 31) < x) {  // the window is behind: the next one
+                cm += 32;
+                ckw = cky[min(cm + static_cast<uint32_t>(lane), mcap - 1)];
+            }
+        }
+    }
+    if (!met && !fail) {
+        uint64_t sx = seed_t + (x + 1) * kGolden, sy = seed_t + (y + 1) * kGolden;
+        Run rx = warp_run(sc, sx, lane_off, lane), ry = warp_run(sc, sy, lane_off, lane);
+        for (;;) {
+            const uint64_t d64 = x <= y ? y - x : x - y;
+            const uint32_t d = static_cast<uint32_t>(d64), dq = d / 62u;
+            if (d64 < 62u * 32u && dq * 62u == d && dq < (x <= y ? rx.n : ry.n)) {
+                if (x <= y) {
+                    record_run(ckp, g.ckcap, g.d_log2, k, dq, x, lane);
+                    k += dq;
+                    x = y;
+                } else {
+                    kb += dq;
+                }
+                break;
+            }
+            if (x + rx.adv <= y + ry.adv) {
+                record_run(ckp, g.ckcap, g.d_log2, k, rx.n, x, lane);
+                k += rx.n;
+                steps += rx.n;
+                x += rx.adv;
+                sx += static_cast<uint64_t>(rx.adv) * kGolden;
+                rx = warp_run(sc, sx, lane_off, lane);
+            } else {
+                kb += ry.n;
+                steps += ry.n;
+                y += ry.adv;
+                sy += static_cast<uint64_t>(ry.adv) * kGolden;
+                ry = warp_run(sc, sy, lane_off, lane);
             }
             if (steps > g.link_cap) {
                 fail = true;
                 break;
             }
-        }
-        if (x == cy) {
-            y = cy;
-            kb = static_cast<uint64_t>(cm) << g.d_log2;
-        }
-    }
-    while (x != y && !fail) {
-        const Run mine = half_run(sc, seed_t, half ? y : x, j, half);
-        Run rx, ry;
-        rx.n = __shfl_sync(0xffffffffu, mine.n, 0);
-        rx.next = __shfl_sync(0xffffffffu, mine.next, 0);
-        ry.n = __shfl_sync(0xffffffffu, mine.n, 16);
-        ry.next = __shfl_sync(0xffffffffu, mine.next, 16);
-        const uint64_t m = rx.next < ry.next ? rx.next : ry.next;
-        // starts below m: x + 62 i for i < ix, y + 62 i for i < iy. Both chains
-        // lie within a run (< 17 * 64 draws) of each other and of m, so the
-        // differences fit 32 bits.
-        const uint32_t ix = m > x ? min(rx.n, (static_cast<uint32_t>(m - x) + 61u) / 62u) : 0u;
-        const uint32_t iy = m > y ? min(ry.n, (static_cast<uint32_t>(m - y) + 61u) / 62u) : 0u;
-        bool met = false;
-        uint32_t adv_x = ix, adv_y = iy;
-        const uint32_t d = static_cast<uint32_t>(x < y ? y - x : x - y);
-        const uint32_t dq = d / 62u;
-        if (dq * 62u == d) {  // the leading start is on the lagging chain's run?
-            if (x < y && dq < ix) {
-                met = true;
-                adv_x = dq;
-                adv_y = 0;
-            } else if (x > y && dq < iy) {
-                met = true;
-                adv_x = 0;
-                adv_y = dq;
-            }
-        }
-        if (lane == 0) record_ckpt(ckp, g.ckcap, g.d_log2, k, adv_x, x);
-        const uint64_t nx = met ? x + 62ull * adv_x : (ix == rx.n ? rx.next : x + 62ull * ix);
-        const uint64_t ny = met ? y + 62ull * adv_y : (iy == ry.n ? ry.next : y + 62ull * iy);
-        k += adv_x;
-        kb += adv_y;
-        x = nx;
-        y = ny;
-        steps += adv_x + adv_y;
-        if (steps > g.link_cap) {
-            fail = true;
-            break;
         }
     }
     if (lane == 0) {
