@@ -25,8 +25,11 @@
 //   f(g) = 16 w0 + sum_k w_k g_k + sum_{j<=i<16} Q_ij g_i g_j,
 // so with u = g - c over the first 16 genes:
 //   f(g) = f(c) + grad f(c) . u + sum_{j<=i<16} Q_ij u_i u_j + tail
-//        <= f(c) + sum_k |grad_k f(c)| r_k + q(r) + tail,
-//   q(r) = sum_i max(Q_ii, 0) r_i^2 + sum_{j<i} |Q_ij| r_i r_j,
+//        <= f(c) + sum_k |grad_k f(c)| r_k + sum_k d_k r_k^2 + tail
+// for any d >= 0 with diag(d) - Q positive semidefinite (quad_diag: about half
+// of sum_i max(Q_ii, 0) r_i^2 + sum_{j<i} |Q_ij| r_i r_j, which d_k = Q_kk +
+// sum_{j != k} |Q_kj| / 2 gives, and the pairs the table leaves fall from 12 to
+// 9% on the committed surface, from 30 to 23% on a seeded 153-term one).
 // grad f(c) = w + Qs c (Qs = Q + Q^T); the tail sum_{k>=16} w_k g_k is taken at
 // its largest over both parents' boxes. A jump to value v at gene j < 16 is a
 // box of centre v and radius 0; past gene 15 it raises f by at most
@@ -61,8 +64,8 @@ static_assert(kGolden * kGoldenInv == 1, "inverse modulo 2^64");
 
 struct PruneConst {
     float qs[16][16];  // Qs = Q + Q^T (Qs_kk = 2 Q_kk): grad of the quadratic block is Qs x
+    float d[16];       // diag(d) - Q is positive semidefinite (quad_diag)
     float s;           // half-width of a gene's mutation box around its clamped parent gene
-    float c0;          // the bound's constant part (above) at that half-width, rounded up
     float err;         // bound rounding + reference-order rounding, rounded up
 };
 
@@ -176,7 +179,7 @@ __global__ void prune_box_kernel(const float *__restrict__ tab, int ne, float s,
 // first k1 genes, u0 over all masks. The genes are taken in the order `perm`
 // (the ones that matter most first); the masks of the first n_enum are
 // enumerated and the others take the hull of both parents' boxes:
-//   max over masks of [f(c) + sum |grad_k f(c)| r_k] + q(r) + tail.
+//   max over masks of [f(c) + sum |grad_k f(c)| r_k] + sum d_k r_k^2 + tail.
 // A pair and its mirror have the same masks (complemented), so a <= b is
 // evaluated once. A group of 2^(k1 - 5) x 16 threads takes a pair: each thread
 // fixes genes 5..k1-1, takes every 16th value of the enumerated genes from k1
@@ -190,6 +193,7 @@ constexpr int kMaxMaskGenes = 8;
 struct PairArgs {
     float qs[16][16];  // Qs in `perm` order
     float lin[16];     // linear weights in that order
+    float d[16];       // PruneConst::d in that order
     float tl[kNtot - 16];
     float w16, s, err;
     const float *tab;
@@ -295,12 +299,7 @@ __global__ void __launch_bounds__(128, 3) pair_bound_kernel(const __grid_constan
     if (!mine) return;
     float q2 = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        float t = fmaxf(0.5f * A.qs[i][i], 0.0f) * r[i];
-#pragma unroll
-        for (int j = 0; j < i; ++j) t = __fmaf_rn(fabsf(A.qs[i][j]), r[j], t);
-        q2 = __fmaf_rn(t, r[i], q2);
-    }
+    for (int i = 0; i < 16; ++i) q2 = __fmaf_ru(A.d[i], __fmul_ru(r[i], r[i]), q2);
     float tl = 0.0f;
     if (A.tail) {
 #pragma unroll
@@ -339,7 +338,7 @@ struct WarpQueue {
 };
 
 // The bound of one queued candidate from its 16 crossover bits (and its jump):
-// f(c) + sum |grad_k f(c)| r_k + c0 (+ the pair's tail).
+// f(c) + sum (|grad_k f(c)| + d_k r_k) r_k (+ the pair's tail).
 template <bool kTail>
 __device__ __forceinline__ float prune_bound(const PruneArgs &A, const uint32_t *__restrict__ bx, uint64_t s0,
                                              uint32_t meta) {
@@ -372,9 +371,9 @@ __device__ __forceinline__ float prune_bound(const PruneArgs &A, const uint32_t 
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
         f2 = __fmaf_rn(c[k], __fadd_rn(g[k], A.m.wlin[k]), f2);
-        l1 = __fmaf_rn(fabsf(g[k]), r[k], l1);
+        l1 = __fmaf_rn(__fmaf_rn(A.pc.d[k], r[k], fabsf(g[k])), r[k], l1);
     }
-    float b = __fadd_rn(__fadd_rn(__fmaf_rn(0.5f, f2, A.m.w16), l1), A.pc.c0);
+    float b = __fadd_rn(__fmaf_rn(0.5f, f2, A.m.w16), l1);
     if (kTail) b = __fadd_rn(b, __fadd_rn(A.tmax[ea * A.sc.ne + eb], jidx >= 16u ? A.jb.c[jidx] : 0.0f));
     return b;
 }
@@ -657,20 +656,107 @@ size_t prune_smem(uint32_t sort_n, int ne, int num_sms, bool el_smem) {
            (el_smem ? static_cast<size_t>(ne + 1) * kNtot * sizeof(float) : 0);
 }
 
+// PruneConst::d: d >= 0 with diag(d) - Qsym positive semidefinite (Qsym = Qs /
+// 2, the symmetric form of Q) and a small sum, so that u' Q u <= sum d_k u_k^2.
+// Row sums of |Qsym| dominate; scaled by the largest eigenvalue of
+// diag(d)^-1/2 Qsym diag(d)^-1/2 they still do, and a few rounds move d towards
+// the genes on which the eigenvector shows it binding. The eigenvalues come
+// from power iteration and certify nothing: the d taken is the one whose
+// diag(d) - Qsym passes a Cholesky factorisation with every pivot above 1e-6 of
+// the matrix's largest entry (a double factorisation's error is below 1e-12 of
+// it), raised by a hundredth until it does. About 25,000 multiply-adds.
+inline void quad_diag(const float (&qs)[16][16], float (&out)[16]) {
+    double S[16][16], dom[16], d[16], v[16], best[16], top = 0.0, best_sum = 0.0;
+    for (int i = 0; i < 16; ++i)
+        for (int j = 0; j < 16; ++j) {
+            S[i][j] = 0.5 * static_cast<double>(qs[i][j]);
+            top = std::max(top, std::fabs(S[i][j]));
+        }
+    if (top == 0.0) {
+        for (int i = 0; i < 16; ++i) out[i] = 0.0f;
+        return;
+    }
+    for (int i = 0; i < 16; ++i) {
+        dom[i] = S[i][i];
+        for (int j = 0; j < 16; ++j)
+            if (j != i) dom[i] += std::fabs(S[i][j]);
+        dom[i] = std::max(dom[i], 1e-6 * top);
+        best[i] = d[i] = dom[i];
+        best_sum += dom[i];
+        v[i] = 0.25;
+    }
+    for (int round = 0; round < 4; ++round) {
+        double M[16][16], h[16], shift = 0.0, lam = 0.0;
+        for (int i = 0; i < 16; ++i) h[i] = 1.0 / std::sqrt(d[i]);
+        for (int i = 0; i < 16; ++i) {
+            double row = 0.0;
+            for (int j = 0; j < 16; ++j) {
+                M[i][j] = S[i][j] * h[i] * h[j];
+                row += std::fabs(M[i][j]);
+            }
+            shift = std::max(shift, row);
+        }
+        for (int it = 0; it < 24; ++it) {  // power iteration, shifted so that the largest eigenvalue leads
+            double w[16], n2 = 0.0;
+            lam = 0.0;
+            for (int i = 0; i < 16; ++i) {
+                double s = 0.0;
+                for (int j = 0; j < 16; ++j) s += M[i][j] * v[j];
+                lam += s * v[i];
+                w[i] = s + 0.5 * shift * v[i];
+                n2 += w[i] * w[i];
+            }
+            if (!(n2 > 0.0)) break;
+            const double inv = 1.0 / std::sqrt(n2);
+            for (int i = 0; i < 16; ++i) v[i] = w[i] * inv;
+        }
+        lam = std::max(lam, 1e-6);
+        double sum = 0.0;
+        for (int i = 0; i < 16; ++i) sum += d[i] * lam;
+        if (sum < best_sum) {
+            best_sum = sum;
+            for (int i = 0; i < 16; ++i) best[i] = d[i] * lam;
+        }
+        const double eta = 0.5 / (1.0 + 0.3 * round);
+        for (int i = 0; i < 16; ++i)
+            d[i] = std::max(d[i] * lam * std::pow((v[i] * v[i] + 0.01) / (d[i] * lam / sum + 0.01), eta), 1e-6 * top);
+    }
+    for (int tries = 0;; ++tries) {  // dom itself passes: rows dominated with room
+        const bool last = tries == 64;
+        const double up = std::pow(1.01, tries) * (1.0 + 1e-4);
+        for (int i = 0; i < 16; ++i) d[i] = (last ? dom[i] * 1.001 : best[i] * up) + 2e-6 * top;
+        if (last) break;
+        double L[16][16];
+        bool ok = true;
+        for (int k = 0; k < 16 && ok; ++k)
+            for (int i = k; i < 16; ++i) {
+                double s = (i == k ? d[i] : 0.0) - S[i][k];
+                for (int m = 0; m < k; ++m) s -= L[i][m] * L[k][m];
+                if (i == k) {
+                    if (!(s > 1e-6 * top)) {
+                        ok = false;
+                        break;
+                    }
+                    L[k][k] = std::sqrt(s);
+                } else {
+                    L[i][k] = s / L[k][k];
+                }
+            }
+        if (ok) break;
+    }
+    for (int i = 0; i < 16; ++i) out[i] = std::nextafter(static_cast<float>(d[i]), INFINITY);
+}
+
 // The bound's constants for a model whose filter bound is finite and a
-// mutation width the fast delta form handles. *tail: some linear weight past
-// gene 15 is nonzero. Returns false when the bound cannot be certified
-// (non-finite sums).
+// mutation width the fast delta form handles (PruneConst::d is set by the plan
+// that prunes). *tail: some linear weight past gene 15 is nonzero. Returns
+// false when the bound cannot be certified (non-finite sums).
 bool make_prune(const csx_model &m, float sigma, PruneConst *pc, bool *tail) {
     const double s = std::min(std::fabs(static_cast<double>(sigma)) + std::ldexp(1.0, -24), 1.0);
-    double qsum = 0.0, qpos = 0.0, lsum = 0.0;
+    double qsum = 0.0, lsum = 0.0;
     bool tail_nz = false;
     for (int i = 0; i < 16; ++i)
-        for (int j = 0; j <= i; ++j) {
-            const double q = static_cast<double>(m.w_quad[i * 16 + j]);
-            qsum += std::fabs(q);
-            qpos += (i == j) ? std::max(q, 0.0) : std::fabs(q);
-        }
+        for (int j = 0; j <= i; ++j) qsum += std::fabs(static_cast<double>(m.w_quad[i * 16 + j]));
     for (int k = 0; k < kNtot; ++k) {
         const double w = static_cast<double>(m.w_lin[k]);
         lsum += std::fabs(w);
@@ -682,19 +768,15 @@ bool make_prune(const csx_model &m, float sigma, PruneConst *pc, bool *tail) {
             pc->qs[j][k] = (j == k) ? 2.0f * q : q;  // exact: the weights are finite and below 1e30
         }
     const double up = 1.0 + std::ldexp(1.0, -20);
-    // a box's FP16 radius: at most half the unit interval, and at most s plus
-    // its rounding and its centre's (2^-11 + 2^-12)
-    const double rmax = std::min(s, 0.5) + std::ldexp(1.0, -10);
-    const double c0 = rmax * rmax * qpos * up;
     const double u = std::ldexp(1.0, -24);
     auto gamma = [u](double n) { return n * u / (1.0 - n * u); };
     const double w16 = 16.0 * std::fabs(static_cast<double>(m.w0));
-    const double a_bound = w16 + 3.0 * lsum + 4.0 * qsum + c0;  // magnitudes the bound's f32 sums reach
-    const double a_ref = w16 + lsum + qsum;                      // the reference order's (genes in [0, 1])
+    // magnitudes the bound's f32 sums reach: sum d_k r_k^2 <= 2 qsum (r <= 1/2 + 2^-10, sum d <= 2.002 qsum)
+    const double a_bound = w16 + 3.0 * lsum + 6.0 * qsum;
+    const double a_ref = w16 + lsum + qsum;  // the reference order's (genes in [0, 1])
     const double err = (2.0 * gamma(64) * a_bound + gamma(35) * a_ref) * up + 1e-30;
-    if (!std::isfinite(c0) || !std::isfinite(err) || err > 1e30) return false;
+    if (!std::isfinite(err) || err > 1e30) return false;
     pc->s = std::nextafter(static_cast<float>(s), INFINITY);
-    pc->c0 = c0 > 0.0 ? std::nextafter(static_cast<float>(c0), INFINITY) : 0.0f;
     pc->err = std::nextafter(static_cast<float>(err), INFINITY);
     *tail = tail_nz;
     return true;
@@ -763,6 +845,7 @@ PairArgs make_pair_args(const csx_model &m, const PruneConst &pc, int ne, bool t
     gene_order(m, pc, P.perm);
     for (int i = 0; i < 16; ++i) {
         P.lin[i] = m.w_lin[P.perm[i]];
+        P.d[i] = pc.d[P.perm[i]];
         for (int j = 0; j < 16; ++j) {
             P.qs[i][j] = pc.qs[P.perm[i]][P.perm[j]];
             qsum += std::fabs(static_cast<double>(P.qs[i][j]));

@@ -397,6 +397,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     const uint64_t sms = sharded ? kItemRefSms : static_cast<uint64_t>(cx.num_sms);
     const uint64_t min_prune = env_u64("CSX_PRUNE_MIN_CANDS", 400ull * 3 * sms * kThreads);
     pl->prune_ok = pl->prune && lam_range >= min_prune;
+    if (pl->prune_ok) quad_diag(pl->pc.qs, pl->pc.d);
     if (pl->prune_ok && grid_override == 0) {
         // the selection scratch holds one key per CTA: at most 3 CTAs per SM
         pl->el_smem = prune_el_smem(pl->sort_n, ne, cx.num_sms, cx.max_smem);
