@@ -815,7 +815,7 @@ int csx_screen_batch(int n_islands, const csx_cfg *cfgs, const csx_model *models
             const IslandBufs &b = L.b[i];
             rc = fix_ties(*cx, cfgs[i], models[i], nullptr, n_elites[i], 0, 0, out + off, cnt,
                           ScreenBufs{b.tab, b.items, res[4 * i + 3], b.ids, b.tribes, in_b ? b.lb : b.la,
-                                     L.pl[i].kpad},
+                                     L.pl[i].kpad, b.pairs},
                           st);
             if (rc) return rc;
         }

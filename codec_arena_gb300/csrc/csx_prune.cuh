@@ -337,6 +337,52 @@ struct WarpQueue {
     uint32_t i1[kWqCap], i2[kWqCap];  // its item
 };
 
+// A candidate by its header draws: parents, immigrant, jump, and the state of
+// the next candidate's first draw (the jump test's draw ends a candidate without
+// one).
+struct PairHead {
+    uint32_t ea, eb;
+    bool imm, jump;
+    uint64_t next;
+};
+
+__device__ __forceinline__ PairHead pair_head(const SynthConst &C, bool pow2, uint64_t s0) {
+    PairHead h;
+    const uint32_t xa = draw_hi(s0), xb = draw_hi(s0 + kGolden);
+    if (pow2) {
+        h.ea = xa & (C.ne - 1);
+        h.eb = xb & (C.ne - 1);
+    } else {
+        h.ea = fastmod_u32(xa, C.ne_magic, C.ne);
+        h.eb = fastmod_u32(xb, C.ne_magic, C.ne);
+    }
+    h.imm = (draw_vh(s0 + 2 * kGolden) >> 8) < C.imm_thr;
+    const uint64_t sj = s0 + (h.imm ? 32u : 61u) * kGolden;
+    h.jump = (draw_vh(sj) >> 8) < C.jump_thr;
+    h.next = sj + (h.jump ? 3u : 1u) * kGolden;
+    return h;
+}
+
+__device__ __forceinline__ uint32_t pair_meta(const PairHead &h) {
+    return h.ea | (h.eb << 11) | (h.imm ? 1u << 30 : 0u) | (h.jump && !h.imm ? 1u << 31 : 0u);
+}
+
+// Whether the bound of the masks that agree with the candidate's first k1
+// crossover bits, plus what its jump can add (a jump past gene 15 adds nothing
+// without a tail), leaves it a chance at tlo.
+__device__ __forceinline__ bool mask_passes(const PruneArgs &A, uint64_t s0, uint32_t meta, float tlo) {
+    const uint32_t ea = meta & 2047u, eb = (meta >> 11) & 2047u;
+    float jc = 0.0f;
+    if (meta >> 31) jc = A.jb.c[draw_hi(s0 + 62 * kGolden) % 29u];
+    uint32_t mask = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kMaxMaskGenes; ++k)
+        if (k < A.k1) mask |= (draw_bitword(s0 + A.goff[k]) >> 31) << k;
+    if (ea > eb) mask ^= (1u << A.k1) - 1u;
+    const float b1 = A.t1[(static_cast<size_t>(pair_index(ea, eb)) << A.k1) + mask];
+    return !(__fadd_ru(b1, jc) < tlo);
+}
+
 // The bound of one queued candidate from its 16 crossover bits (and its jump):
 // f(c) + sum (|grad_k f(c)| + d_k r_k) r_k (+ the pair's tail).
 template <bool kTail>
@@ -542,28 +588,16 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         for (int rr = 0; rr < kPruneRounds; ++rr) {
             const uint64_t s0 = st;
             const uint32_t itm = item, dcand = n_it - left;
-            const uint32_t xa = draw_hi(s0), xb = draw_hi(s0 + kGolden);
-            uint32_t ea, eb;
-            if (pow2) {
-                ea = xa & (A.sc.ne - 1);
-                eb = xb & (A.sc.ne - 1);
-            } else {
-                ea = fastmod_u32(xa, A.sc.ne_magic, A.sc.ne);
-                eb = fastmod_u32(xb, A.sc.ne_magic, A.sc.ne);
-            }
-            const bool imm = (draw_vh(s0 + 2 * kGolden) >> 8) < A.sc.imm_thr;
-            const uint64_t sj = s0 + (imm ? 32u : 61u) * kGolden;  // the jump test's draw ends a candidate without one
-            const bool jump = (draw_vh(sj) >> 8) < A.sc.jump_thr;
-            st = sj + (jump ? 3u : 1u) * kGolden;
-            const uint32_t pi = ea * A.sc.ne + eb;
+            const PairHead h = pair_head(A.sc, pow2, s0);
+            st = h.next;
+            const uint32_t pi = h.ea * A.sc.ne + h.eb;
             const bool on = A.bm_words ? ((bm[pi >> 5] >> (pi & 31u)) & 1u) != 0u : !(A.u0[pi] < tlo);
-            const bool pass = valid && (imm || jump || on);
+            const bool pass = valid && (h.imm || h.jump || on);
             if (--left == 0) next_item();
             const uint32_t m = __ballot_sync(0xffffffffu, pass);
             if (pass) {
                 const uint32_t slot = n1 + __popc(m & lt);
-                wq.q1[slot] = make_uint4(static_cast<uint32_t>(s0), static_cast<uint32_t>(s0 >> 32), dcand,
-                                         ea | (eb << 11) | (imm ? 1u << 30 : 0u) | (jump && !imm ? 1u << 31 : 0u));
+                wq.q1[slot] = make_uint4(static_cast<uint32_t>(s0), static_cast<uint32_t>(s0 >> 32), dcand, pair_meta(h));
                 wq.i1[slot] = itm;
             }
             n1 += __popc(m);
@@ -580,18 +614,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                     q = wq.q1[n1 + lane];
                     iq = wq.i1[n1 + lane];
                     const uint64_t sq = (static_cast<uint64_t>(q.y) << 32) | q.x;
-                    const uint32_t qa = q.w & 2047u, qb = (q.w >> 11) & 2047u;
                     immq = (q.w & (1u << 30)) != 0u;
-                    // what its jump can add (a jump past gene 15 adds nothing without a tail)
-                    float jc = 0.0f;
-                    if (q.w >> 31) jc = A.jb.c[draw_hi(sq + 62 * kGolden) % 29u];
-                    uint32_t mask = 0;
-#pragma unroll
-                    for (uint32_t k = 0; k < kMaxMaskGenes; ++k)
-                        if (k < A.k1) mask |= (draw_bitword(sq + A.goff[k]) >> 31) << k;
-                    if (qa > qb) mask ^= (1u << A.k1) - 1u;
-                    const float b1 = A.t1[(static_cast<size_t>(pair_index(qa, qb)) << A.k1) + mask];
-                    to2 = !immq && !(__fadd_ru(b1, jc) < tlo);
+                    to2 = !immq && mask_passes(A, sq, q.w, tlo);
                 }
                 if (immq) push(q, iq);  // immigrants are always scored
                 const uint32_t m2 = __ballot_sync(0xffffffffu, to2);

@@ -101,6 +101,7 @@ struct Context {
     unsigned char *hpin = nullptr;  // their page-locked staging: result words, an Entry, survivors, elites
     const Entry *fin = nullptr;  // final list of the last single screen (kpad entries)
     uint32_t fin_kpad = 0;
+    PairBufs fin_pairs;  // its pair tables, where it pruned
 };
 
 Context g_ctx[64];
@@ -753,6 +754,7 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     if (rc) return rc;
     cx.fin = cur;
     cx.fin_kpad = pl.kpad;
+    cx.fin_pairs = pairs;
     CSX_CUDA(mark(4));
     if (full) {
         FullScreenArgs F;
@@ -958,6 +960,7 @@ struct ScreenBufs {
     const unsigned int *tribes;
     const Entry *fin;  // the final top-kpad list (its entry past the survivors shows a tie at the K-th score)
     uint32_t kpad;
+    PairBufs pairs{};             // the pruning screen's tables (box null: it did not run)
     const Entry *next = nullptr;  // that entry on the host, where the caller has read it already
 };
 
@@ -1017,7 +1020,10 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
             const uint64_t hi = std::min(n_t, lo + size);
             CSX_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));
             const uint32_t ts = static_cast<uint32_t>(t);
-            if (full) {
+            if (!all && bufs.pairs.box && pl.prune_ok) {
+                tie_collect_pruned_kernel<<<blocks, 256, 0, st>>>(prune_args(A, model, pl, bufs.pairs, nullptr, cx.num_sms),
+                                                                  n_items, ts, lo, hi, thr, d_hits, d_count, cap);
+            } else if (full) {
                 if (pl.fast_delta)
                     tie_collect_kernel<true><<<blocks, 256, 0, st>>>(F, n_items, ts, lo, hi, thr, all, d_hits, d_count, cap);
                 else
@@ -1176,7 +1182,7 @@ int screen_host(const csx_cfg *cfg, const csx_model *model, const csx_genome *el
                                          static_cast<const Item *>(cx->items.p), res[3],
                                          static_cast<const unsigned long long *>(cx->ids.p),
                                          static_cast<const unsigned int *>(cx->tribes.p), cx->fin, cx->fin_kpad,
-                                         cnt == keep_n && has_next ? next : nullptr},
+                                         cx->fin_pairs, cnt == keep_n && has_next ? next : nullptr},
                               st);
         }
     }

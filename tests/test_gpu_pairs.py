@@ -19,9 +19,10 @@ def _need_gpu(csx):
 
 @pytest.mark.parametrize("tail", [False, True])
 @pytest.mark.parametrize("ne", [2, 3, 33, 362, 363, 1536])
-def test_pair_table_sizes(ne, tail):
+def test_pair_table_sizes(monkeypatch, ne, tail):
     from codec_arena_gb300 import _lib, screen, workloads as wl
 
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
     rng = np.random.default_rng(ne + 7 * tail)
     w = rng.normal(0, 1, 166 if tail else 153).astype(np.float32)
     if tail:
@@ -36,3 +37,27 @@ def test_pair_table_sizes(ne, tail):
                                               flags=form | _lib.FLAG_NO_PRUNE), m, el)
             assert n == k == 700_001
             assert got.tobytes() == ref.tobytes(), (form, sigma)
+
+
+@pytest.mark.parametrize("sigma,tail", [(0.0, False), (0.0, True), (0.05, False)])
+def test_tied_survivors_with_pair_tables(monkeypatch, sigma, tail):
+    """Streams replayed for exact ties through the pair tables: integer weights
+    on genes of a coarse grid tie by the hundred (sigma 0), in the pruned single
+    screen and in a batch; the unpruned screen replays them without tables."""
+    from codec_arena_gb300 import _lib, islands, screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    rng = np.random.default_rng(5)
+    w = rng.integers(-3, 4, 166 if tail else 153).astype(np.float32)
+    m = screen.Model.from_compact(w)
+    el = wl.seeded_elites(40, seed=2)
+    el["g"] = np.round(el["g"] * 4) / 4
+    cfg = screen.Cfg(2_000_003, 100, 9, threads=3, sigma=sigma)
+    got, n = screen.screen(cfg, m, el)
+    ref, _ = screen.screen(screen.Cfg(2_000_003, 100, 9, threads=3, sigma=sigma, flags=_lib.FLAG_NO_PRUNE), m, el)
+    assert n == 2_000_003
+    if sigma == 0.0:
+        assert len(set(zip(ref["score"].tolist(), ref["stream"].tolist()))) < len(ref)  # ties inside a stream
+    assert got.tobytes() == ref.tobytes()
+    for surv, k in islands.screen_batch([cfg, cfg], [m, m], [el, el]):
+        assert k == n and surv.tobytes() == ref.tobytes()
