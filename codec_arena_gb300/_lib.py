@@ -133,6 +133,7 @@ SURROGATE_SIGNATURES = {
     "csx_sg_normal_equations": (_int, [_int, _vp, _i64, _int, _vp, _vp, _vp, _vp, _vp]),
     "csx_sg_ridge_solve": (_int, [_int, _vp, _vp, ctypes.c_double, _vp, _vp, _vp, _vp]),
     "csx_sg_ascend": (_int, [_vp, _int, _vp, _i64, _int, _f32, _int, _vp, _vp]),
+    "csx_sg_ascend_to": (_int, [_vp, _int, _vp, _i64, _int, _int, _f32, _int, _vp, _int, _vp, _vp]),
 }
 SIGNATURES.update(SURROGATE_SIGNATURES)
 

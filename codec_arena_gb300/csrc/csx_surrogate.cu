@@ -689,10 +689,18 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
     cluster.sync();  // no CTA leaves while its rows are read
 }
 
+// The rows an ascent reads and writes (the same ones in place); columns ng..cols
+// are copied where they differ.
+struct AscendRows {
+    const float *in;
+    float *out;
+    int ldi, ldo, cols;
+};
+
 template <int QG>
-__global__ void __launch_bounds__(kRowThreads) sg_ascend_kernel(const float *__restrict__ coef, int ng,
-                                                                float *__restrict__ genes, int64_t n, int ldg,
-                                                                float eta, int steps, float *__restrict__ score) {
+__global__ void __launch_bounds__(kRowThreads) sg_ascend_kernel(const float *__restrict__ coef, int ng, AscendRows R,
+                                                                int64_t n, float eta, int steps,
+                                                                float *__restrict__ score) {
     __shared__ CoefT<QG> c;
     extern __shared__ float tile[];
     const int st = stride_for(ng);
@@ -700,7 +708,7 @@ __global__ void __launch_bounds__(kRowThreads) sg_ascend_kernel(const float *__r
     for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * kRowThreads; r0 < n;
          r0 += static_cast<int64_t>(gridDim.x) * kRowThreads) {
         __syncthreads();
-        stage_rows(tile, genes, n, ldg, ng, st, r0);
+        stage_rows(tile, R.in, n, R.ldi, ng, st, r0);
         __syncthreads();
         const int64_t r = r0 + threadIdx.x;
         if (r < n) {
@@ -725,7 +733,14 @@ __global__ void __launch_bounds__(kRowThreads) sg_ascend_kernel(const float *__r
         const int total = static_cast<int>(rows) * ng;
         for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
             const int rr = idx / ng, k = idx - rr * ng;
-            genes[(r0 + rr) * static_cast<int64_t>(ldg) + k] = tile[rr * st + k];
+            R.out[(r0 + rr) * static_cast<int64_t>(R.ldo) + k] = tile[rr * st + k];
+        }
+        if (R.in != R.out && R.cols > ng) {
+            const int more = R.cols - ng;
+            for (int idx = threadIdx.x; idx < static_cast<int>(rows) * more; idx += blockDim.x) {
+                const int rr = idx / more, k = ng + idx - rr * more;
+                R.out[(r0 + rr) * static_cast<int64_t>(R.ldo) + k] = R.in[(r0 + rr) * static_cast<int64_t>(R.ldi) + k];
+            }
         }
     }
 }
@@ -740,15 +755,14 @@ constexpr int kLaneRows = 16;  // rows per CTA
 constexpr int64_t kLaneMaxRows = 30000;
 
 __global__ void __launch_bounds__(kLaneRows * 16) sg_ascend_lanes_kernel(const float *__restrict__ coef, int ng,
-                                                                         float *__restrict__ genes, int64_t n,
-                                                                         int ldg, float eta, int steps,
-                                                                         float *__restrict__ score) {
+                                                                         AscendRows R, int64_t n, float eta,
+                                                                         int steps, float *__restrict__ score) {
     __shared__ CoefT<kQuadGenes> c;
     __shared__ float fin[kLaneRows][kMaxLin + 3];
     const int k = threadIdx.x & 15, rr = threadIdx.x >> 4;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * kLaneRows + rr;
-    float *row = genes + (r < n ? r : 0) * static_cast<int64_t>(ldg);
-    float g0 = row[k], g1 = k + 16 < ng ? row[k + 16] : 0.0f;
+    const float *src = R.in + (r < n ? r : 0) * static_cast<int64_t>(R.ldi);
+    float g0 = src[k], g1 = k + 16 < ng ? src[k + 16] : 0.0f;
     load_coef<CSX_SG_FP32, kQuadGenes>(c, coef, ng);
     __syncthreads();
     float q[16];
@@ -767,10 +781,11 @@ __global__ void __launch_bounds__(kLaneRows * 16) sg_ascend_lanes_kernel(const f
         g1 = fmaxf(fminf(__fmaf_rn(eta, w1, g1), 1.0f), 0.0f);
     }
     if (r < n) {
-        if (steps > 0) {
-            row[k] = g0;
-            if (k + 16 < ng) row[k + 16] = g1;
-        }
+        float *row = R.out + r * static_cast<int64_t>(R.ldo);
+        row[k] = g0;
+        if (k + 16 < ng) row[k + 16] = g1;
+        if (R.in != R.out)
+            for (int m = ng + k; m < R.cols; m += 16) row[m] = src[m];
         fin[rr][k] = g0;
         if (k + 16 < kMaxLin) fin[rr][k + 16] = k + 16 < ng ? g1 : 0.0f;
     }
@@ -1013,25 +1028,34 @@ int csx_sg_ridge_solve(int nf, const double *d_gram, const double *d_rhs, double
     return CSX_OK;
 }
 
-int csx_sg_ascend(const float *d_coef, int nf, float *d_genes, int64_t n, int ldg, float eta, int steps,
-                  float *d_score, void *stream) {
+static int sg_ascend(const float *d_coef, int nf, const AscendRows &R, int64_t n, float eta, int steps,
+                     float *d_score, void *stream) {
     int ng = 0;
-    if (int rc = check_layout(nf, ldg, n, ng)) return rc;
-    if (steps < 0) return CSX_ERR_BAD_ARGS;
+    if (int rc = check_layout(nf, R.ldi < R.ldo ? R.ldi : R.ldo, n, ng)) return rc;
+    if (steps < 0 || R.cols < ng || R.cols > R.ldi || R.cols > R.ldo) return CSX_ERR_BAD_ARGS;
     if (n == 0) return CSX_OK;
-    if (!d_coef || !d_genes) return CSX_ERR_BAD_ARGS;
+    if (!d_coef || !R.in || !R.out) return CSX_ERR_BAD_ARGS;
     auto s = static_cast<cudaStream_t>(stream);
     if (is_full(nf))
-        sg_ascend_kernel<kMaxLin><<<row_grid(n), kRowThreads, tile_bytes(ng), s>>>(d_coef, ng, d_genes, n, ldg, eta,
-                                                                                 steps, d_score);
+        sg_ascend_kernel<kMaxLin><<<row_grid(n), kRowThreads, tile_bytes(ng), s>>>(d_coef, ng, R, n, eta, steps, d_score);
     else if (n <= kLaneMaxRows)
         sg_ascend_lanes_kernel<<<static_cast<unsigned>((n + kLaneRows - 1) / kLaneRows), kLaneRows * 16, 0, s>>>(
-            d_coef, ng, d_genes, n, ldg, eta, steps, d_score);
+            d_coef, ng, R, n, eta, steps, d_score);
     else
-        sg_ascend_kernel<kQuadGenes><<<row_grid(n), kRowThreads, tile_bytes(ng), s>>>(d_coef, ng, d_genes, n, ldg,
-                                                                                    eta, steps, d_score);
+        sg_ascend_kernel<kQuadGenes><<<row_grid(n), kRowThreads, tile_bytes(ng), s>>>(d_coef, ng, R, n, eta, steps,
+                                                                                     d_score);
     SG_CUDA(cudaGetLastError());
     return CSX_OK;
+}
+
+int csx_sg_ascend(const float *d_coef, int nf, float *d_genes, int64_t n, int ldg, float eta, int steps,
+                  float *d_score, void *stream) {
+    return sg_ascend(d_coef, nf, AscendRows{d_genes, d_genes, ldg, ldg, ldg}, n, eta, steps, d_score, stream);
+}
+
+int csx_sg_ascend_to(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int cols, float eta,
+                     int steps, float *d_out, int ldo, float *d_score, void *stream) {
+    return sg_ascend(d_coef, nf, AscendRows{d_genes, d_out, ldg, ldo, cols}, n, eta, steps, d_score, stream);
 }
 
 }  // extern "C"

@@ -21,6 +21,7 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
+import torch.autograd.forward_ad as _fwd
 
 from . import _lib
 from ._lib import SG_BF16, SG_FP32, SG_FP64, check, lib
@@ -173,11 +174,21 @@ def ascend(genes: torch.Tensor, coef: torch.Tensor, eta: float, steps: int):
     """Gradient-guided mutation: `steps` projected ascent steps
     g <- clamp01(g + eta·∇score(g)) on a copy of `genes`.
     Returns (new genes, FP32 scores)."""
-    out = _genes(genes).clone()
-    coef = coef.detach().to(device=out.device, dtype=torch.float32).contiguous()
+    src = _genes(genes)
+    coef = coef.detach().to(device=src.device, dtype=torch.float32).contiguous()
     nf = coef.numel()
     _ng(nf)
-    sc = torch.empty(out.shape[0], dtype=torch.float32, device=out.device)
+    sc = torch.empty(src.shape[0], dtype=torch.float32, device=src.device)
+    # the kernel reads src and writes the copy, unless the clone has a place of
+    # its own (in a graph, a dual number's) or src's rows overlap
+    if (type(src) is torch.Tensor and not src.requires_grad and _fwd._current_level < 0
+            and src.stride(0) >= src.shape[1]):
+        out = torch.empty_like(src)
+        check(lib().csx_sg_ascend_to(coef.data_ptr(), nf, src.data_ptr(), src.shape[0], src.stride(0), src.shape[1],
+                                     float(eta), int(steps), out.data_ptr(), out.stride(0), sc.data_ptr(),
+                                     _stream(out.device)), "sg_ascend_to")
+        return out, sc
+    out = src.clone()
     check(lib().csx_sg_ascend(coef.data_ptr(), nf, out.data_ptr(), out.shape[0], out.stride(0), float(eta),
                               int(steps), sc.data_ptr(), _stream(out.device)), "sg_ascend")
     return out, sc

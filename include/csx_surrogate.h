@@ -83,6 +83,10 @@ int csx_sg_ridge_solve(int nf, const double *d_gram, const double *d_rhs, double
    in place; d_score (may be NULL) receives the final FP32 scores. */
 int csx_sg_ascend(const float *d_coef, int nf, float *d_genes, int64_t n, int ldg, float eta, int steps,
                   float *d_score, void *stream);
+/* The same from d_genes (left as they are) into d_out (row stride ldo): the
+ * first `cols` columns of every row, the ones past the layout's genes copied. */
+int csx_sg_ascend_to(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int cols, float eta,
+                     int steps, float *d_out, int ldo, float *d_score, void *stream);
 
 #ifdef __cplusplus
 }
