@@ -122,7 +122,8 @@ __device__ __forceinline__ uint32_t warp_kth_largest(const uint32_t *v, uint32_t
     return prefix;
 }
 
-__device__ __noinline__ void prune_merge(const PruneArgs *A, Entry *E, uint32_t *sel, unsigned int *s_buf_n,
+template <class Args>
+__device__ __noinline__ void prune_merge(const Args *A, Entry *E, uint32_t *sel, unsigned int *s_buf_n,
                                          unsigned long long *s_t1, unsigned long long *s_t2, float *s_ts) {
     const uint32_t tid = threadIdx.x;
     cta_merge_top(E, A->kpad, A->sort_n, *s_buf_n);
@@ -688,72 +689,73 @@ size_t prune_smem(uint32_t sort_n, int ne, int num_sms, bool el_smem) {
 // from power iteration and certify nothing: the d taken is the one whose
 // diag(d) - Qsym passes a Cholesky factorisation with every pivot above 1e-6 of
 // the matrix's largest entry (a double factorisation's error is below 1e-12 of
-// it), raised by a hundredth until it does. About 25,000 multiply-adds.
-inline void quad_diag(const float (&qs)[16][16], float (&out)[16]) {
-    double S[16][16], dom[16], d[16], v[16], best[16], top = 0.0, best_sum = 0.0;
-    for (int i = 0; i < 16; ++i)
-        for (int j = 0; j < 16; ++j) {
+// it), raised by a hundredth until it does. About 100 N^2 multiply-adds.
+template <int N>
+void quad_diag(const float (&qs)[N][N], float (&out)[N]) {
+    double S[N][N], dom[N], d[N], v[N], best[N], top = 0.0, best_sum = 0.0;
+    for (int i = 0; i < N; ++i)
+        for (int j = 0; j < N; ++j) {
             S[i][j] = 0.5 * static_cast<double>(qs[i][j]);
             top = std::max(top, std::fabs(S[i][j]));
         }
     if (top == 0.0) {
-        for (int i = 0; i < 16; ++i) out[i] = 0.0f;
+        for (int i = 0; i < N; ++i) out[i] = 0.0f;
         return;
     }
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < N; ++i) {
         dom[i] = S[i][i];
-        for (int j = 0; j < 16; ++j)
+        for (int j = 0; j < N; ++j)
             if (j != i) dom[i] += std::fabs(S[i][j]);
         dom[i] = std::max(dom[i], 1e-6 * top);
         best[i] = d[i] = dom[i];
         best_sum += dom[i];
-        v[i] = 0.25;
+        v[i] = 1.0 / std::sqrt(static_cast<double>(N));
     }
     for (int round = 0; round < 4; ++round) {
-        double M[16][16], h[16], shift = 0.0, lam = 0.0;
-        for (int i = 0; i < 16; ++i) h[i] = 1.0 / std::sqrt(d[i]);
-        for (int i = 0; i < 16; ++i) {
+        double M[N][N], h[N], shift = 0.0, lam = 0.0;
+        for (int i = 0; i < N; ++i) h[i] = 1.0 / std::sqrt(d[i]);
+        for (int i = 0; i < N; ++i) {
             double row = 0.0;
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < N; ++j) {
                 M[i][j] = S[i][j] * h[i] * h[j];
                 row += std::fabs(M[i][j]);
             }
             shift = std::max(shift, row);
         }
         for (int it = 0; it < 24; ++it) {  // power iteration, shifted so that the largest eigenvalue leads
-            double w[16], n2 = 0.0;
+            double w[N], n2 = 0.0;
             lam = 0.0;
-            for (int i = 0; i < 16; ++i) {
+            for (int i = 0; i < N; ++i) {
                 double s = 0.0;
-                for (int j = 0; j < 16; ++j) s += M[i][j] * v[j];
+                for (int j = 0; j < N; ++j) s += M[i][j] * v[j];
                 lam += s * v[i];
                 w[i] = s + 0.5 * shift * v[i];
                 n2 += w[i] * w[i];
             }
             if (!(n2 > 0.0)) break;
             const double inv = 1.0 / std::sqrt(n2);
-            for (int i = 0; i < 16; ++i) v[i] = w[i] * inv;
+            for (int i = 0; i < N; ++i) v[i] = w[i] * inv;
         }
         lam = std::max(lam, 1e-6);
         double sum = 0.0;
-        for (int i = 0; i < 16; ++i) sum += d[i] * lam;
+        for (int i = 0; i < N; ++i) sum += d[i] * lam;
         if (sum < best_sum) {
             best_sum = sum;
-            for (int i = 0; i < 16; ++i) best[i] = d[i] * lam;
+            for (int i = 0; i < N; ++i) best[i] = d[i] * lam;
         }
         const double eta = 0.5 / (1.0 + 0.3 * round);
-        for (int i = 0; i < 16; ++i)
+        for (int i = 0; i < N; ++i)
             d[i] = std::max(d[i] * lam * std::pow((v[i] * v[i] + 0.01) / (d[i] * lam / sum + 0.01), eta), 1e-6 * top);
     }
     for (int tries = 0;; ++tries) {  // dom itself passes: rows dominated with room
         const bool last = tries == 64;
         const double up = std::pow(1.01, tries) * (1.0 + 1e-4);
-        for (int i = 0; i < 16; ++i) d[i] = (last ? dom[i] * 1.001 : best[i] * up) + 2e-6 * top;
+        for (int i = 0; i < N; ++i) d[i] = (last ? dom[i] * 1.001 : best[i] * up) + 2e-6 * top;
         if (last) break;
-        double L[16][16];
+        double L[N][N];
         bool ok = true;
-        for (int k = 0; k < 16 && ok; ++k)
-            for (int i = k; i < 16; ++i) {
+        for (int k = 0; k < N && ok; ++k)
+            for (int i = k; i < N; ++i) {
                 double s = (i == k ? d[i] : 0.0) - S[i][k];
                 for (int m = 0; m < k; ++m) s -= L[i][m] * L[k][m];
                 if (i == k) {
@@ -768,7 +770,7 @@ inline void quad_diag(const float (&qs)[16][16], float (&out)[16]) {
             }
         if (ok) break;
     }
-    for (int i = 0; i < 16; ++i) out[i] = std::nextafter(static_cast<float>(d[i]), INFINITY);
+    for (int i = 0; i < N; ++i) out[i] = std::nextafter(static_cast<float>(d[i]), INFINITY);
 }
 
 // The bound's constants for a model whose filter bound is finite and a

@@ -55,6 +55,7 @@
 #include "csx_dense.cuh"
 #include "csx_screen_kernels.cuh"
 #include "csx_prune.cuh"
+#include "csx_prune_full.cuh"
 #include "csx_ties.cuh"
 
 namespace csx {
@@ -160,6 +161,8 @@ struct Plan {
     bool el_smem = false;   // its elite table in shared memory (prune_el_smem)
     uint64_t lam = 0;       // candidates of the streams this call screens
     PruneConst pc{};
+    bool prune_full = false;  // the full surface's pruning screen (csx_prune_full.cuh)
+    FullPrune fp{};
 };
 
 int context_init(Context &cx, int dev) {
@@ -407,7 +410,17 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     } else {
         pl->prune = false;
     }
-    if (!pl->prune)
+    pl->prune_full = full && grid_override == 0 && pl->fast_delta &&
+                     !(cfg.flags & (CSX_FLAG_NO_PRUNE | CSX_FLAG_EXACT_ALL)) && lam_range >= min_prune &&
+                     make_full_prune(*full, cfg.sigma, &pl->fp);
+    if (pl->prune_full) {
+        const size_t without = full_prune_smem(pl->sort_n, ne, cx.num_sms, false);
+        const size_t with = full_prune_smem(pl->sort_n, ne, cx.num_sms, true);
+        pl->el_smem = with + 1024 <= cx.max_smem && prune_fit(with) >= prune_fit(without);
+        pl->smem = pl->el_smem ? with : without;
+        pl->prune_full = pl->smem + 1024 <= cx.max_smem;
+    }
+    if (!pl->prune && !pl->prune_full)
         pl->smem = pl->tc ? static_cast<size_t>(pl->sort_n) * sizeof(Entry) +
                                 static_cast<size_t>(ne + 1) * kNtot * sizeof(float) + kTcSmemExtra
                           : screen_smem(pl->sort_n, ne, pl->filter);
@@ -425,6 +438,12 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
         int rc = screen_occupancy(screen_tc_fn(pl->fast_delta, pl->fp16), cx.num_sms, pl->smem, &pl->grid);
         if (rc) return rc;
         pl->grid = kTcCtasPerSm * cx.num_sms;
+    } else if (pl->prune_full) {
+        int rc = screen_occupancy(screen_ft_kernel, cx.num_sms, pl->smem, &pl->grid);
+        if (rc) return rc;
+        // the occupancy query reports one CTA per SM for a kernel that allocates
+        // tensor memory; registers, shared memory and 64 columns each hold three
+        pl->grid = std::max(1, prune_fit(pl->smem)) * cx.num_sms;
     } else if (full) {
         int rc = screen_occupancy(screen_full_fn(pl->fast_delta), cx.num_sms, pl->smem, &pl->grid);
         if (rc) return rc;
@@ -671,8 +690,8 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     CSX_CUDA(cx.lists_a.ensure(static_cast<size_t>(nl) * pl.kpad * sizeof(Entry)));
     CSX_CUDA(cx.lists_b.ensure(static_cast<size_t>((nl + 1) / 2) * pl.kpad * sizeof(Entry)));
     PairBufs pairs;
+    if (pl.prune || pl.prune_full) CSX_CUDA(cx.pub.ensure(static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t)));
     if (pl.prune) {
-        CSX_CUDA(cx.pub.ensure(static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t)));
         CSX_CUDA(cx.pairs.ensure(pair_bytes(pl.lam, ne, pl.tail)));
         pairs = pair_bufs(cx.pairs.p, pl.lam, ne, pl.tail);
     }
@@ -694,7 +713,8 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     auto mark = [&](int i) -> cudaError_t { return cx.timed ? cudaEventRecord(cx.ev[i], st) : cudaSuccess; };
     CSX_CUDA(mark(0));
     CSX_CUDA(cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), st));
-    if (pl.prune) CSX_CUDA(cudaMemsetAsync(cx.pub.p, 0, static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t), st));
+    if (pl.prune || pl.prune_full)
+        CSX_CUDA(cudaMemsetAsync(cx.pub.p, 0, static_cast<size_t>(kPruneMs) * nl * sizeof(uint32_t), st));
 
     const SynthConst sc = make_synth(cfg, ne);
 
@@ -736,6 +756,15 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
         rc = tc_error_bound(model, pl.fp16, &P.err_abs);
         if (rc) return rc;
         screen_tc_fn(fast, pl.fp16)<<<pl.grid, kThreads, pl.smem, st>>>(P);
+    } else if (pl.prune_full) {
+        FullPruneArgs F{};
+        static_cast<ScreenArgs &>(F) = A;
+        F.fm = make_full_model(*full);
+        F.fp = pl.fp;
+        F.pub = static_cast<uint32_t *>(cx.pub.p);
+        F.sel_cap = 3u * static_cast<uint32_t>(cx.num_sms);
+        F.el_smem = pl.el_smem ? 1u : 0u;
+        screen_ft_kernel<<<pl.grid, kThreads, pl.smem, st>>>(F);
     } else if (full) {
         FullScreenArgs F;
         static_cast<ScreenArgs &>(F) = A;
