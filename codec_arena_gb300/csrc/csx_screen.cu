@@ -83,6 +83,8 @@ struct Context {
     int num_sms = 0;
     size_t max_smem = 0;
     cudaEvent_t done = nullptr;
+    cudaStream_t side = nullptr;  // the pair tables, beside the item building
+    cudaEvent_t side_go = nullptr, side_done = nullptr;
     cudaEvent_t ev[6] = {};
     bool timed = false;
     csx_run_info info{};
@@ -173,6 +175,9 @@ int context_init(Context &cx, int dev) {
     CSX_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cx.max_smem = static_cast<size_t>(v);
     CSX_CUDA(cudaEventCreateWithFlags(&cx.done, cudaEventDisableTiming));
+    CSX_CUDA(cudaStreamCreateWithFlags(&cx.side, cudaStreamNonBlocking));
+    CSX_CUDA(cudaEventCreateWithFlags(&cx.side_go, cudaEventDisableTiming));
+    CSX_CUDA(cudaEventCreateWithFlags(&cx.side_done, cudaEventDisableTiming));
     for (auto &e : cx.ev) CSX_CUDA(cudaEventCreate(&e));
     cx.init = true;
     return CSX_OK;
@@ -531,8 +536,9 @@ DevModel make_dev_model(const csx_model &model) {
 // The item-building stages on `st` (walk, link, assembly, scan, emit), or one
 // item per stream when every stream fits in one item. recs / ck / so / off
 // are unused on the short path.
+// `walked` (if not null) is recorded once the walk is through.
 int enqueue_items(const SynthConst &sc, const Plan &pl, SegRec *recs, uint64_t *ck, SegOut *so, uint32_t *off,
-                  Item *items, Ctrl *ctrl, cudaStream_t st, uint32_t *launches) {
+                  Item *items, Ctrl *ctrl, cudaStream_t st, uint32_t *launches, cudaEvent_t walked = nullptr) {
     const StreamGeom &g = pl.g;
     if (pl.short_path) {
         stream_items_kernel<<<unit_blocks(g.nT, 256), 256, 0, st>>>(g, items, ctrl);
@@ -560,6 +566,7 @@ int enqueue_items(const SynthConst &sc, const Plan &pl, SegRec *recs, uint64_t *
     }
     walk_kernel<<<unit_blocks(g.n_seg, 128), 128, 0, st>>>(sc, g, recs, ck, ctrl);
     CSX_CUDA(cudaGetLastError());
+    if (walked) CSX_CUDA(cudaEventRecord(walked, st));
     link_kernel<<<unit_blocks(g.n_seg * 32, 128), 128, 0, st>>>(sc, g, recs, ck, ctrl);
     CSX_CUDA(cudaGetLastError());
     if (g.C >= 64)
@@ -569,7 +576,7 @@ int enqueue_items(const SynthConst &sc, const Plan &pl, SegRec *recs, uint64_t *
     CSX_CUDA(cudaGetLastError());
     scan_kernel<<<1, 1024, 0, st>>>(so, g.n_seg, off, ctrl, pl.items_cap);
     CSX_CUDA(cudaGetLastError());
-    emit_kernel<<<unit_blocks(g.n_seg, 128), 128, 0, st>>>(g, so, off, ck, items, ctrl);
+    emit_kernel<<<unit_blocks(g.n_seg * 32, 128), 128, 0, st>>>(g, so, off, ck, items, ctrl);
     CSX_CUDA(cudaGetLastError());
     *launches += 5;
     return CSX_OK;
@@ -725,17 +732,30 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
         d_genomes, ne, tab, ids, tribes);
     CSX_CUDA(cudaGetLastError());
     ++launches;
-    if (pl.prune) {
-        rc = enqueue_pairs(model, pl.pc, ne, pl.tail, tab, pairs, st, &launches);
-        if (rc) return rc;
-    }
     CSX_CUDA(mark(1));
 
     Item *items = static_cast<Item *>(cx.items.p);
+    // The pair tables on a stream of their own beside the link, which leaves most
+    // of the GPU idle: after the walk, not beside it (its few long CTAs are dealt
+    // out at once, and around a running kernel they pile up on some SMs: items
+    // of 2.65e9 candidates took 22 ms instead of 9). The screen waits for both,
+    // and so does whatever follows this call (cx.done).
+    const bool beside = pl.prune && !pl.short_path && !pl.dense;
+    if (pl.prune && !beside) {
+        rc = enqueue_pairs(model, pl.pc, ne, pl.tail, tab, pairs, st, &launches);
+        if (rc) return rc;
+    }
     rc = enqueue_items(sc, pl, static_cast<SegRec *>(cx.recs.p), static_cast<uint64_t *>(cx.ck.p),
                        static_cast<SegOut *>(cx.segout.p), static_cast<uint32_t *>(cx.off.p), items, ctrl, st,
-                       &launches);
+                       &launches, beside ? cx.side_go : nullptr);
     if (rc) return rc;
+    if (beside) {
+        CSX_CUDA(cudaStreamWaitEvent(cx.side, cx.side_go, 0));
+        rc = enqueue_pairs(model, pl.pc, ne, pl.tail, tab, pairs, cx.side, &launches);
+        CSX_CUDA(cudaEventRecord(cx.side_done, cx.side));  // also where it failed: st waits for what was enqueued
+        CSX_CUDA(cudaStreamWaitEvent(st, cx.side_done, 0));
+        if (rc) return rc;
+    }
     if (shard.count > 1) {
         shard_items_kernel<<<1, 32, 0, st>>>(ctrl, shard.index, shard.count);
         CSX_CUDA(cudaGetLastError());
