@@ -129,6 +129,7 @@ SURROGATE_SIGNATURES = {
     "csx_sg_forward": (_int, [_vp, _int, _vp, _i64, _int, _int, _vp, _vp]),
     "csx_sg_forward_f64": (_int, [_vp, _int, _vp, _i64, _int, _vp, _vp]),
     "csx_sg_backward": (_int, [_vp, _int, _vp, _i64, _int, _int, _vp, _vp, _vp, _vp, _vp]),
+    "csx_sg_backward_f32": (_int, [_vp, _int, _vp, _i64, _int, _int, _vp, _vp, _vp, _vp, _vp]),
     "csx_sg_backward_coef_f64": (_int, [_int, _vp, _i64, _int, _vp, _vp, _vp, _vp]),
     "csx_sg_normal_equations": (_int, [_int, _vp, _i64, _int, _vp, _vp, _vp, _vp, _vp]),
     "csx_sg_ridge_solve": (_int, [_int, _vp, _vp, ctypes.c_double, _vp, _vp, _vp, _vp]),

@@ -364,12 +364,13 @@ __device__ __forceinline__ double sum_parts(const double *__restrict__ p, int np
     return v;
 }
 
+template <typename T>
 __global__ void __launch_bounds__(32 * kSumSplit) sg_sum_parts_kernel(const double *__restrict__ part, int nparts,
-                                                                      int stride, int nf, double *__restrict__ out) {
+                                                                      int stride, int nf, T *__restrict__ out) {
     __shared__ double s[kSumSplit][32];
     const int f = blockIdx.x * 32 + threadIdx.x;
     const double v = sum_parts(part + f, nparts, stride, f < nf, s);
-    if (threadIdx.y == 0 && f < nf) out[f] = v;
+    if (threadIdx.y == 0 && f < nf) out[f] = static_cast<T>(v);
 }
 
 struct GramRange;
@@ -856,8 +857,8 @@ int enable_smem() {  // on the current device, every call (cheap)
     return CSX_OK;
 }
 
-template <typename TG>
-int coef_grad(int ng, int nf, const float *genes, int64_t n, int ldg, const TG *gout, double *dcoef, void *work,
+template <typename TG, typename TD>
+int coef_grad(int ng, int nf, const float *genes, int64_t n, int ldg, const TG *gout, TD *dcoef, void *work,
               cudaStream_t s) {
     if (!dcoef) return CSX_OK;
     if (!work) return CSX_ERR_BAD_ARGS;
@@ -927,8 +928,13 @@ int csx_sg_forward_f64(const double *d_coef, int nf, const float *d_genes, int64
     return CSX_OK;
 }
 
-int csx_sg_backward(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int precision,
-                    const float *d_gout, float *d_dgenes, double *d_dcoef, void *d_work, void *stream) {
+}  // extern "C"
+
+namespace {
+
+template <typename TD>
+int sg_backward(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int precision,
+                const float *d_gout, float *d_dgenes, TD *d_dcoef, void *d_work, void *stream) {
     int ng = 0;
     if (int rc = check_layout(nf, ldg, n, ng)) return rc;
     if (precision != CSX_SG_FP32 && precision != CSX_SG_BF16) return CSX_ERR_BAD_ARGS;
@@ -952,7 +958,21 @@ int csx_sg_backward(const float *d_coef, int nf, const float *d_genes, int64_t n
                                                                                        d_gout, d_dgenes);
         SG_CUDA(cudaGetLastError());
     }
-    return coef_grad<float>(ng, nf, d_genes, n, ldg, d_gout, d_dcoef, d_work, s);
+    return coef_grad(ng, nf, d_genes, n, ldg, d_gout, d_dcoef, d_work, s);
+}
+
+}  // namespace
+
+extern "C" {
+
+int csx_sg_backward(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int precision,
+                    const float *d_gout, float *d_dgenes, double *d_dcoef, void *d_work, void *stream) {
+    return sg_backward(d_coef, nf, d_genes, n, ldg, precision, d_gout, d_dgenes, d_dcoef, d_work, stream);
+}
+
+int csx_sg_backward_f32(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int precision,
+                        const float *d_gout, float *d_dgenes, float *d_dcoef, void *d_work, void *stream) {
+    return sg_backward(d_coef, nf, d_genes, n, ldg, precision, d_gout, d_dgenes, d_dcoef, d_work, stream);
 }
 
 int csx_sg_backward_coef_f64(int nf, const float *d_genes, int64_t n, int ldg, const double *d_gout, double *d_dcoef,
@@ -960,7 +980,7 @@ int csx_sg_backward_coef_f64(int nf, const float *d_genes, int64_t n, int ldg, c
     int ng = 0;
     if (int rc = check_layout(nf, ldg, n, ng)) return rc;
     if (n > 0 && (!d_genes || !d_gout)) return CSX_ERR_BAD_ARGS;
-    return coef_grad<double>(ng, nf, d_genes, n, ldg, d_gout, d_dcoef, d_work, static_cast<cudaStream_t>(stream));
+    return coef_grad(ng, nf, d_genes, n, ldg, d_gout, d_dcoef, d_work, static_cast<cudaStream_t>(stream));
 }
 
 int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, const double *d_fit, double *d_gram,

@@ -61,6 +61,9 @@ int csx_sg_forward_f64(const double *d_coef, int nf, const float *d_genes, int64
    csx_sg_workspace_bytes(nf). */
 int csx_sg_backward(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int precision,
                     const float *d_gout, float *d_dgenes, double *d_dcoef, void *d_work, void *stream);
+/* The same with d_dcoef rounded to float (accumulated in FP64 all the same). */
+int csx_sg_backward_f32(const float *d_coef, int nf, const float *d_genes, int64_t n, int ldg, int precision,
+                        const float *d_gout, float *d_dgenes, float *d_dcoef, void *d_work, void *stream);
 
 /* Same with an FP64 upstream gradient (the ridge residual). */
 int csx_sg_backward_coef_f64(int nf, const float *d_genes, int64_t n, int ldg, const double *d_gout,
