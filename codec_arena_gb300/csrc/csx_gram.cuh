@@ -81,17 +81,25 @@ __device__ __forceinline__ int range_exp64(unsigned long long bits) {
 
 __global__ void __launch_bounds__(256) sg_range_kernel(int ng, const float *__restrict__ genes, int64_t n, int ldg,
                                                        const double *__restrict__ fit, GramRange *__restrict__ out) {
+    // eight rows in flight per warp; up to 16 genes two rows per load (the lane's
+    // upper half takes the second)
     const int lane = threadIdx.x & 31;
     const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    const int two = ng <= 16 ? 1 : 0, col = two ? lane & 15 : lane, sub = two ? lane >> 4 : 0;
+    const int64_t step = nw << two;
     uint32_t m = 0;
     unsigned long long my = 0;
+#pragma unroll 8
+    for (int64_t r = (w0 << two) + sub; r < n; r += step)
+        if (col < ng) m = max(m, __float_as_uint(genes[r * ldg + col]) & 0x7fffffffu);
+    if (fit) {
 #pragma unroll 4
-    for (int64_t r = w0; r < n; r += nw) {
-        if (lane < ng) m = max(m, __float_as_uint(genes[r * ldg + lane]) & 0x7fffffffu);
-        if (lane == 31 && fit)
+        for (int64_t r = w0 * 32 + lane; r < n; r += nw * 32)
             my = max(my, static_cast<unsigned long long>(__double_as_longlong(fit[r])) & 0x7fffffffffffffffull);
+        for (int o = 16; o > 0; o >>= 1) my = max(my, __shfl_xor_sync(0xffffffffu, my, o));
     }
+    if (two) m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
     // one update per CTA and column: an update per warp spent 65 us on the 30
     // addresses at 400,000 rows
     __shared__ uint32_t sm[8][32];
