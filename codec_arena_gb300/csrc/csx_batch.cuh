@@ -464,14 +464,18 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
     const int cap = tune && tune->ctas_per_sm > 0 ? static_cast<int>(tune->ctas_per_sm) : 3;
     if (L->prune) {
         // every island's pruning screen, one after another, each with its own shared memory and up to three CTAs per SM
+    for (int i = 0; i < n && L->prune; ++i) {  // one island's lists and elites too large for the pruning kernel
+        if (cfgs[i].lambda == 0) continue;
+        Plan &pl = L->pl[i];
+        pl.el_smem = prune_el_smem(pl.sort_n, n_elites[i], cx.num_sms, cx.max_smem);
+        pl.smem = prune_smem(pl.sort_n, n_elites[i], cx.num_sms, pl.el_smem);
+        L->prune = pl.smem + 1024 <= cx.max_smem;
+    }
         // (as the single screen); the lists are laid out for the widest grid
         L->smem = 0;
         for (int i = 0; i < n; ++i) {
             if (cfgs[i].lambda == 0) continue;
             Plan &pl = L->pl[i];
-            pl.el_smem = prune_el_smem(pl.sort_n, n_elites[i], cx.num_sms, cx.max_smem);
-            pl.smem = prune_smem(pl.sort_n, n_elites[i], cx.num_sms, pl.el_smem);
-            if (pl.smem + 1024 > cx.max_smem) return CSX_ERR_LIMIT;
             const int fit = std::min(cap, std::max(1, static_cast<int>((228u << 10) / (pl.smem + 1024))));
             pl.grid = fit * cx.num_sms;
             L->smem = std::max(L->smem, pl.smem);
@@ -479,8 +483,10 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
         }
         per_sm = std::max(per_sm, 1);
         for (bool tail : {false, true})
-            CSX_CUDA(cudaFuncSetAttribute(screen_p_fn(tail, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(L->smem)));
+            for (bool bx_smem : {false, true})
+                CSX_CUDA(cudaFuncSetAttribute(screen_p_fn(tail, false, bx_smem),
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              static_cast<int>(L->smem)));
     } else {
         L->smem = screen_smem(L->sort_n, ne_max, L->filter);
         if (L->smem + 2048 > cx.max_smem) return CSX_ERR_LIMIT;
@@ -628,7 +634,7 @@ int batch_enqueue(Context &cx, const BatchLayout &L, cudaStream_t st, bool captu
             if (L.cfg[i].lambda == 0) continue;
             const Plan &pl = L.pl[i];
             CSX_CUDA(cudaMemsetAsync(L.pub, 0, static_cast<size_t>(kPruneMs) * pl.grid * sizeof(uint32_t), st));
-            screen_p_fn(pl.tail, false)<<<pl.grid, kThreads, pl.smem, st>>>(L.pargs[i]);
+            screen_p_fn(pl.tail, false, prune_bx_smem(pl.sort_n, L.ne[i]))<<<pl.grid, kThreads, pl.smem, st>>>(L.pargs[i]);
             CSX_CUDA(cudaGetLastError());
             ++nk;
         }

@@ -386,11 +386,12 @@ __device__ __forceinline__ bool mask_passes(const PruneArgs &A, uint64_t s0, uin
 
 // The bound of one queued candidate from its 16 crossover bits (and its jump):
 // f(c) + sum (|grad_k f(c)| + d_k r_k) r_k (+ the pair's tail).
-template <bool kTail>
+// Elite e's boxes are bx[kStride e ..].
+template <bool kTail, int kStride>
 __device__ __forceinline__ float prune_bound(const PruneArgs &A, const uint32_t *__restrict__ bx, uint64_t s0,
                                              uint32_t meta) {
     const uint32_t ea = meta & 2047u, eb = (meta >> 11) & 2047u;
-    const uint32_t *pa = bx + ea * 17, *pb = bx + eb * 17;
+    const uint32_t *pa = bx + ea * kStride, *pb = bx + eb * kStride;
     uint32_t jidx = kNoJump;
     float jval = 0.0f;
     if (meta >> 31) {
@@ -445,7 +446,8 @@ __device__ __forceinline__ float prune_bound(const PruneArgs &A, const uint32_t 
 // and rank by that score rounded to f32 (the FP64 top-K; PruneConst::err
 // covers the rounding of those scores too) -- instead of the reference's f32
 // order.
-template <bool kTail, bool kFp64>
+// kFar: the box table stays in global memory (prune_bx_smem).
+template <bool kTail, bool kFp64, bool kFar>
 __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_constant__ PruneArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Entry *E = reinterpret_cast<Entry *>(smem_raw);
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     const float *el = A.el_smem ? el_copy : A.el;
     Pend *pend = reinterpret_cast<Pend *>(el_copy + (A.el_smem ? (A.sc.ne + 1) * kNtot : 0u));
     uint32_t *bx = reinterpret_cast<uint32_t *>(pend + kPendCap);
-    uint32_t *bm = bx + A.sc.ne * 17;
+    uint32_t *bm = bx + (kFar ? 0u : A.sc.ne * 17);
     uint32_t *sel = bm + A.bm_words;
     __shared__ unsigned int s_buf_n, s_pend_n;
     __shared__ unsigned long long s_t1, s_t2;
@@ -467,7 +469,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     for (uint32_t i = tid; i < A.sort_n; i += kThreads) E[i] = Entry{0ull, 0ull};
     if (A.el_smem)
         for (uint32_t i = tid; i < (A.sc.ne + 1) * kNtot; i += kThreads) el_copy[i] = A.el[i];
-    for (uint32_t i = tid; i < A.sc.ne * 16; i += kThreads) bx[(i >> 4) * 17 + (i & 15u)] = A.box[i];
+    if (!kFar)
+        for (uint32_t i = tid; i < A.sc.ne * 16; i += kThreads) bx[(i >> 4) * 17 + (i & 15u)] = A.box[i];
     for (uint32_t i = tid; i < A.bm_words; i += kThreads) bm[i] = 0xffffffffu;
     if (tid == 0) {
         s_buf_n = 0;
@@ -635,7 +638,9 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                 if (lane < nb) {
                     const uint4 q = wq.q2[n2 + lane];
                     const uint64_t sq = (static_cast<uint64_t>(q.y) << 32) | q.x;
-                    if (!(prune_bound<kTail>(A, bx, sq, q.w) < tlo)) push(q, wq.i2[n2 + lane]);  // NaN: scored
+                    const float f = kFar ? prune_bound<kTail, 16>(A, A.box, sq, q.w)
+                                         : prune_bound<kTail, 17>(A, bx, sq, q.w);
+                    if (!(f < tlo)) push(q, wq.i2[n2 + lane]);  // NaN: scored
                 }
             }
             if (__any_sync(0xffffffffu, n_def > 0)) break;
@@ -657,10 +662,15 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
 using PruneScreenFn = void (*)(PruneArgs);
 
 // The pruning kernel of a plan: with a linear tail or not, ranking in the
-// reference's f32 order or (the precision form) in FP64.
-PruneScreenFn screen_p_fn(bool tail, bool fp64) {
-    if (tail) return fp64 ? screen_p_kernel<true, true> : screen_p_kernel<true, false>;
-    return fp64 ? screen_p_kernel<false, true> : screen_p_kernel<false, false>;
+// reference's f32 order or (the precision form) in FP64, the box table in
+// shared memory or not.
+template <bool kFar>
+PruneScreenFn screen_p_pick(bool tail, bool fp64) {
+    if (tail) return fp64 ? screen_p_kernel<true, true, kFar> : screen_p_kernel<true, false, kFar>;
+    return fp64 ? screen_p_kernel<false, true, kFar> : screen_p_kernel<false, false, kFar>;
+}
+PruneScreenFn screen_p_fn(bool tail, bool fp64, bool bx_smem) {
+    return bx_smem ? screen_p_pick<false>(tail, fp64) : screen_p_pick<true>(tail, fp64);
 }
 
 // Words of the pair bitmap for ne elites: one bit per pair up to 16 KB of
@@ -670,13 +680,17 @@ inline uint32_t prune_bm_words(int ne) {
     return w <= 4096 ? static_cast<uint32_t>(w) : 0u;
 }
 
+// Whether the box table goes to shared memory: not beside lists of 4096 entries
+// where the elites are more than the queues leave room for (1057 of them).
+inline bool prune_bx_smem(uint32_t sort_n, int ne) { return sort_n < 8192 || ne <= 1024; }
+
 // Shared memory of the pruning screen: the sort buffer, the warps' queues, the
-// CTA's queue, the box table, the pair bitmap and the selection scratch of the
+// CTA's queue, the box table (prune_bx_smem), the pair bitmap and the selection scratch of the
 // published keys (one per CTA, at most 3 CTAs per SM), with el_smem the elite
 // table.
 size_t prune_smem(uint32_t sort_n, int ne, int num_sms, bool el_smem) {
     return static_cast<size_t>(sort_n) * sizeof(Entry) + (kThreads / 32) * sizeof(WarpQueue) +
-           kPendCap * sizeof(Pend) + static_cast<size_t>(ne) * 17 * sizeof(uint32_t) +
+           kPendCap * sizeof(Pend) + (prune_bx_smem(sort_n, ne) ? static_cast<size_t>(ne) * 17 * sizeof(uint32_t) : 0) +
            prune_bm_words(ne) * sizeof(uint32_t) + 3ull * num_sms * sizeof(uint32_t) +
            (el_smem ? static_cast<size_t>(ne + 1) * kNtot * sizeof(float) : 0);
 }

@@ -433,7 +433,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     if (grid_override > 0) {
         pl->grid = grid_override;
     } else if (pl->prune) {
-        int rc = screen_occupancy(screen_p_fn(pl->tail, pl->tc), cx.num_sms, pl->smem, &pl->grid);
+        int rc = screen_occupancy(screen_p_fn(pl->tail, pl->tc, prune_bx_smem(pl->sort_n, ne)), cx.num_sms, pl->smem, &pl->grid);
         if (rc) return rc;
     } else if (pl->tc) {
         // The occupancy query reports one CTA per SM for this kernel, yet three
@@ -766,7 +766,7 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     const ScreenArgs A = screen_args(cfg, model, sc, pl, tab, items, ctrl, static_cast<Entry *>(cx.lists_a.p));
     if (pl.prune) {
         const PruneArgs P = prune_args(A, model, pl, pairs, static_cast<uint32_t *>(cx.pub.p), cx.num_sms);
-        screen_p_fn(pl.tail, pl.tc)<<<pl.grid, kThreads, pl.smem, st>>>(P);
+        screen_p_fn(pl.tail, pl.tc, prune_bx_smem(pl.sort_n, ne))<<<pl.grid, kThreads, pl.smem, st>>>(P);
     } else if (pl.tc) {
         TcScreenArgs P;
         P.A = A;

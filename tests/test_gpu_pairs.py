@@ -61,3 +61,58 @@ def test_tied_survivors_with_pair_tables(monkeypatch, sigma, tail):
     assert got.tobytes() == ref.tobytes()
     for surv, k in islands.screen_batch([cfg, cfg], [m, m], [el, el]):
         assert k == n and surv.tobytes() == ref.tobytes()
+
+
+@pytest.mark.parametrize("keep,ne,tail", [(2048, 1024, False), (2048, 1025, True), (4096, 1100, False)])
+def test_long_lists_beside_many_elites(monkeypatch, orc, keep, ne, tail):
+    """Lists of 4096 entries leave no room for the box table of more than 1024
+    elites: the kernel reads it where it is, with the oracle's survivors."""
+    import os
+
+    from codec_arena_gb300 import screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    rng = np.random.default_rng(keep + ne)
+    w = rng.normal(0, 1, 166 if tail else 153).astype(np.float32)
+    el = wl.seeded_elites(ne, seed=3)
+    got, n = screen.screen(screen.Cfg(300_001, keep, 5, threads=3), screen.Model.from_compact(w), el)
+    assert screen.last_run_info()["screen_ctas"] > 0
+    want, wn = orc.screen(orc.cfg(300_001, keep, 5, threads=3), orc.model_from_compact(w), el,
+                          cpu_threads=os.cpu_count() or 4)
+    assert n == wn == 300_001 and got.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("lam,nf,flag", [(22_800_000, 153, 0), (23_000_000, 153, 0), (2_300_000, 161, 0x20),
+                                         (2_400_000, 161, 0x20), (20_000_000, 465, 0), (22_000_000, 465, 0)])
+def test_both_sides_of_the_pruning_floor(monkeypatch, lam, nf, flag):
+    """The automatic choice at 64 elites, either side of the floor (128 + 68
+    candidates per thread; 20 with FP64 ranking; 180 on the full surface),
+    against the screen without pruning."""
+    from codec_arena_gb300 import _lib, screen, workloads as wl
+
+    monkeypatch.delenv("CSX_PRUNE_MIN_CANDS", raising=False)
+    w = np.random.default_rng(nf).normal(0, 0.3, nf).astype(np.float32)
+    m = screen.ModelFull.from_compact(w) if nf == 465 else screen.Model.from_compact(w)
+    el = wl.seeded_elites(64, seed=3)
+    got, n = screen.screen(screen.Cfg(lam, 192, 5, threads=4, flags=flag), m, el)
+    ref, k = screen.screen(screen.Cfg(lam, 192, 5, threads=4, flags=flag | _lib.FLAG_NO_PRUNE), m, el)
+    assert n == k == lam and got.tobytes() == ref.tobytes()
+
+
+@pytest.mark.parametrize("floor", ["79999", "80001"])
+def test_batch_prunes_by_its_mean_island(monkeypatch, floor):
+    """Islands of 40,000, 40,000 and 160,000 candidates (a mean of 80,000) and an
+    empty one, either side of the floor; each equals its single screen."""
+    from codec_arena_gb300 import islands, screen, workloads as wl
+
+    rng = np.random.default_rng(2)
+    models = [screen.Model.from_compact(rng.normal(0, 1, 153).astype(np.float32)) for _ in range(4)]
+    el = [wl.seeded_elites(20 + j, seed=j) for j in range(4)]
+    cfgs = [screen.Cfg(lam, 30, 5 + j, threads=2) for j, lam in enumerate((40_000, 40_000, 0, 160_000))]
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", floor)
+    res = islands.screen_batch(cfgs, models, el)
+    for c, m, e, (surv, n) in zip(cfgs, models, el, res):
+        assert n == c.lambda_
+        if c.lambda_:
+            want, _ = screen.screen(c, m, e)
+            assert surv.tobytes() == want.tobytes()
