@@ -10,8 +10,8 @@
 // small islands are short of parallel work, so islands overlap). Then either
 // form screens them:
 //
-// * pruned (every island admits the pruning bound and clears the
-//   pruning floor): each island's pruning screen (csx_prune.cuh) runs over the
+// * pruned (every island admits the pruning bound and their mean budget clears
+//   the pruning floor): each island's pruning screen (csx_prune.cuh) runs over the
 //   whole GPU in turn, with its own shared memory and grid, waiting only for
 //   its own island's items, and writes its CTA lists into the island's area;
 // * otherwise one persistent launch screens every island's items (below): a
@@ -448,22 +448,22 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
     L->ne_max = static_cast<uint32_t>(ne_max);
 
     // plans (the grid is set below; item and segment sizes do not depend on it)
-    uint64_t items_sum = 0;
+    uint64_t items_sum = 0, lam_sum = 0;
+    int filled = 0;
+    for (int i = 0; i < n; ++i) {
+        lam_sum += cfgs[i].lambda;
+        filled += cfgs[i].lambda > 0 ? 1 : 0;
+    }
     L->prune = true;
     for (int i = 0; i < n; ++i) {
         if (cfgs[i].lambda == 0) continue;
         int rc = make_plan(cx, cfgs[i], models[i], n_elites[i], &L->pl[i], 1, tune ? tune->item_cands : 0,
-                           tune ? tune->seg_cands : 0);
+                           tune ? tune->seg_cands : 0, 0, 0, nullptr, false, lam_sum, filled);
         if (rc) return rc;
         items_sum += L->pl[i].items_cap;
         L->prune = L->prune && L->pl[i].prune_ok;
     }
     if (items_sum >= 0xFFFFFFFFull) return CSX_ERR_LIMIT;
-
-    int per_sm = 0;
-    const int cap = tune && tune->ctas_per_sm > 0 ? static_cast<int>(tune->ctas_per_sm) : 3;
-    if (L->prune) {
-        // every island's pruning screen, one after another, each with its own shared memory and up to three CTAs per SM
     for (int i = 0; i < n && L->prune; ++i) {  // one island's lists and elites too large for the pruning kernel
         if (cfgs[i].lambda == 0) continue;
         Plan &pl = L->pl[i];
@@ -471,6 +471,11 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
         pl.smem = prune_smem(pl.sort_n, n_elites[i], cx.num_sms, pl.el_smem);
         L->prune = pl.smem + 1024 <= cx.max_smem;
     }
+
+    int per_sm = 0;
+    const int cap = tune && tune->ctas_per_sm > 0 ? static_cast<int>(tune->ctas_per_sm) : 3;
+    if (L->prune) {
+        // every island's pruning screen, one after another, each with its own shared memory and up to three CTAs per SM
         // (as the single screen); the lists are laid out for the widest grid
         L->smem = 0;
         for (int i = 0; i < n; ++i) {

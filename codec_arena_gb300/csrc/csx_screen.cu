@@ -377,14 +377,43 @@ struct Shard {
 };
 
 // grid_override, item_cands, seg_cands: 0 = automatic (the batched screen
+// Candidates per thread of a three-CTA-per-SM grid from which pruning pays: the
+// threshold then settles early enough, and the pair tables, which grow with
+// the elites, are a small part. A call's ms, pruned / unpruned, on 152 SMs:
+//   sigma 0.12, 153 terms, top 192    1.6e7       3.2e7       4.5e7
+//     64 elites (top 64)            1.87/1.82   2.39/2.57       -
+//     96 elites                     1.96/1.88   2.63/2.62   2.91/3.21
+//     256 elites                    2.08/1.87   2.78/2.62   3.18/3.19
+//   166 terms, 96 elites            2.25/2.29   2.99/3.29   3.42/4.06
+//   sigma 0.03, 256 elites          1.92/2.29   2.50/3.28   2.80/4.06
+// so a line that rises with the elites: 2.3e7 candidates at 64, 4.67e7 at 256.
+// The precision form's other kernel is dearer (64 elites: 1.12/1.28 at 2e6,
+// 1.38/1.66 at 4e6; 256: 1.30/1.24 at 3e6, 1.81/1.93 at 6e6); the full surface
+// has no tables (1.6e7: 2.51/2.43 to 2.23/2.79, 2.4e7: 3.11/3.15, 2.73/3.52). A
+// batch of batch_n > 0 islands counts its mean island, each with a screen of its own
+// instead of one launch for all (20 islands, ms: mean 2e7 19.3/16.7, 4e7
+// 29.2/29.8, 8e7 40.5/51.6).
+uint64_t prune_floor(bool precision, bool full, int batch_n, int ne) {
+    const uint64_t e = static_cast<uint64_t>(ne);
+    if (batch_n > 0) return 400;
+    if (precision) return 12 + e / 8;
+    if (full) return 180;
+    return std::min<uint64_t>(400, 128 + 17 * e / 16);
+}
+
 // passes its own grid and the tuner's sizes). A sharded call sizes its items
 // by a fixed SM count, so that every share's item list is the same whatever
-// GPU it runs on.
+// GPU it runs on. An island of a batch passes the batch's candidates and
+// islands: whether to prune and to take block maps goes by the whole batch
+// (islands' maps of 1e6 to 8e6 candidates cost more than their walks, which
+// overlap, and items of 16 candidates more than the batch kernel gains: a batch
+// that took 12.2 ms with walks took 13.4 with maps).
 constexpr int kItemRefSms = 152;
 
 int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int ne, Plan *pl,
               int grid_override = 0, uint64_t item_cands = 0, uint64_t seg_cands = 0, uint64_t t_begin = 0,
-              uint64_t t_end = 0, const csx_model_full *full = nullptr, bool sharded = false) {
+              uint64_t t_end = 0, const csx_model_full *full = nullptr, bool sharded = false,
+              uint64_t batch_lam = 0, int batch_n = 0) {
     StreamGeom &g = pl->g;
     int src = split_streams(cfg, t_begin, t_end, g);
     if (src) return src;
@@ -398,14 +427,18 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     if (full && tcf) return CSX_ERR_BAD_ARGS;  // the precision form scores the reference surface
     pl->tc = tcf != 0;  // FP64 ranking (pruned, or the unpruned precision kernel)
     pl->fp16 = tcf == CSX_FLAG_TC_FP16;
-    // pruning pays once the generation gives each screen thread a few hundred
-    // candidates (the threshold then settles early; measured against the
-    // unpruned filter kernel: 0.40 against 0.29 ms at 1e6, 0.78 against 0.54
-    // at 1e7, 1.35 against 1.21 at 3e7, 3.14 against 3.45 at 1e8 candidates):
-    // prune from 400 per thread of a three-CTA-per-SM grid
     const uint64_t sms = sharded ? kItemRefSms : static_cast<uint64_t>(cx.num_sms);
-    const uint64_t min_prune = env_u64("CSX_PRUNE_MIN_CANDS", 400ull * 3 * sms * kThreads);
-    pl->prune_ok = pl->prune && lam_range >= min_prune;
+    const uint64_t min_prune = env_u64("CSX_PRUNE_MIN_CANDS", prune_floor(pl->tc, full != nullptr, batch_n, ne) * 3 *
+                                                                  sms * kThreads);
+    pl->prune_ok = pl->prune && std::max(lam_range, batch_lam) / std::max(batch_n, 1) >= min_prune;
+    // Lists and elites too large for the unpruned kernel's shared memory are
+    // taken from 400 candidates per thread on, whatever the floor above.
+    const size_t plain = pl->tc ? static_cast<size_t>(pl->sort_n) * sizeof(Entry) +
+                                      static_cast<size_t>(ne + 1) * kNtot * sizeof(float) + kTcSmemExtra
+                                : screen_smem(pl->sort_n, ne, pl->filter);
+    const bool plain_fits = plain + 1024 <= cx.max_smem;
+    const uint64_t min_large = env_u64("CSX_PRUNE_MIN_CANDS", 400ull * 3 * sms * kThreads);
+    pl->prune_ok = pl->prune_ok && (plain_fits || lam_range >= min_large);
     if (pl->prune_ok) quad_diag(pl->pc.qs, pl->pc.d);
     if (pl->prune_ok && grid_override == 0) {
         // the selection scratch holds one key per CTA: at most 3 CTAs per SM
@@ -416,7 +449,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
         pl->prune = false;
     }
     pl->prune_full = full && grid_override == 0 && pl->fast_delta &&
-                     !(cfg.flags & (CSX_FLAG_NO_PRUNE | CSX_FLAG_EXACT_ALL)) && lam_range >= min_prune &&
+                     !(cfg.flags & (CSX_FLAG_NO_PRUNE | CSX_FLAG_EXACT_ALL)) && lam_range >= min_prune && plain_fits &&
                      make_full_prune(*full, cfg.sigma, &pl->fp);
     if (pl->prune_full) {
         const size_t without = full_prune_smem(pl->sort_n, ne, cx.num_sms, false);
@@ -425,10 +458,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
         pl->smem = pl->el_smem ? with : without;
         pl->prune_full = pl->smem + 1024 <= cx.max_smem;
     }
-    if (!pl->prune && !pl->prune_full)
-        pl->smem = pl->tc ? static_cast<size_t>(pl->sort_n) * sizeof(Entry) +
-                                static_cast<size_t>(ne + 1) * kNtot * sizeof(float) + kTcSmemExtra
-                          : screen_smem(pl->sort_n, ne, pl->filter);
+    if (!pl->prune && !pl->prune_full) pl->smem = plain;
     if (pl->smem + 1024 > cx.max_smem) return CSX_ERR_LIMIT;
     if (grid_override > 0) {
         pl->grid = grid_override;
@@ -495,7 +525,7 @@ int make_plan(const Context &cx, const csx_cfg &cfg, const csx_model &model, int
     segment_geometry(cfg, seg, true, g);
     pl->short_path = my_max <= D;
     pl->dense = false;
-    if (!pl->short_path && lam_range <= kDenseMaxCands && !sized) dense_geometry(cfg, lam_range, pl);
+    if (!pl->short_path && std::max(lam_range, batch_lam) <= kDenseMaxCands && !sized) dense_geometry(cfg, lam_range, pl);
     if (pl->dense) {  // every block of a group is an item, the last group's up to the stream's end
         pl->items_cap = g.n_seg * kDenseGroup;
         return CSX_OK;

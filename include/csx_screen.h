@@ -70,10 +70,12 @@ enum {
                                       reach the top-K.
                                       Results are identical either way; only speed differs.
                                       Without the flag the library prunes generations of at least
-                                      400 candidates per screen thread (3 CTAs x 256 threads per
-                                      SM: 4.67e7 on 152 SMs; below, the unpruned kernel is
-                                      faster); the environment variable CSX_PRUNE_MIN_CANDS sets
-                                      that floor in candidates */
+                                      128 + 17/16 n_elites candidates per screen thread, at most 400
+                                      (3 CTAs x 256 threads per SM: 2.3e7 candidates with 64 elites,
+                                      4.67e7 with 256 on 152 SMs; the precision form 12 + n_elites/8,
+                                      the full surface 180, a batch a mean of 400 per island; below,
+                                      the unpruned kernel is faster); the environment variable
+                                      CSX_PRUNE_MIN_CANDS sets that floor in candidates */
 #define CSX_FLAG_PRUNE_FFMA 0x100u /* the pruning bound's gradient by FP32 FMA: accepted, and what
                                       the library does without it as well */
 
