@@ -14,13 +14,14 @@ T = 4 splitmix64 streams (the reference CI's --threads), sigma 0.12, jump
          integer-issue rates of this GPU (the path is integer-issue bound)
   cpu_baseline  the C restatement of the Zig screen (oracle/) on this host's
          cores, T = 4 as the reference CI, on a bounded prefix sample
-  precision_forms  the same generation with the quadratic block on the tensor
-         cores (BF16, and FP16 with x' = 2g - 1): throughput beside the plain
-         FP32 value, top-256 recall against the FP64 top-256, score errors
+  precision_forms  the same generation ranked by FP64 scores (the BF16 / FP16
+         precision flags; unpruned, their quadratic block runs on the tensor
+         cores): throughput beside the line's value, top-256 recall against
+         the FP64 top-256, score errors
 
 The metric names the BF16 tensor-core form against the plain FP32 form; the
-line's value is the plain FP32 fused screen (the reference's own f32
-semantics, bit-exact), and precision_forms carries the BF16 / FP16 values.
+line's value is the FP32 fused screen with pruning (the reference's own f32
+semantics, bit-exact), and precision_forms carries the other forms' values.
 `--workload precision` prints a line whose value is the BF16 form;
 `--workload islands` the batched-islands workload, `--workload refit` the
 GPU ridge refit and the surrogate's forward / backward kernels (with the full
@@ -65,18 +66,30 @@ def full_synth_ops(tail):
     return 1760.0 - (0.99 * 26 + 0.01 * 13) * 20 - 13 * (5 + 2)
 
 
-# The pruning form per candidate: the header's 4 draws (parents, immigrant
-# test, jump test) + 0.02 jump index draws, the 16 crossover-bit draws of the
-# 0.99 crossover candidates (x 20 lane-ops each), the bound's FP32 work on them
-# (4 x 16 lane-ops beside the tensor core's 16 x 16 MACs, 8 packs), and the
-# full synthesis for the fraction q queued for the reference-order score.
+# A screen that computes every crossover candidate's own bound, per candidate:
+# the header's 4 draws (parents, immigrant test, jump test) + 0.02 jump index
+# draws, the 16 crossover-bit draws of the 0.99 crossover candidates (x 20
+# lane-ops each), the bound's FP32 work on them (4 x 16 lane-ops beside the
+# gradient, 8 packs), and the full synthesis for the fraction q queued for the
+# reference-order score.
 PRUNE_DRAWS = 4.02 + 0.99 * 16
 PRUNE_FIXED_OPS = PRUNE_DRAWS * 20 + 0.99 * (4 * 16 + 8)
-PRUNE_TC_FLOP = 0.99 * 2 * 16 * 16  # tensor-core flops per candidate (the bound's gradient)
 
 
 def prune_ops(q, tail):
     return PRUNE_FIXED_OPS + q * full_synth_ops(tail)
+
+
+# The screen's own count: most candidates go by their parent pair's bound, so
+# what every candidate needs is the header (4.02 draws) and the queued fraction
+# its synthesis. The bits and bounds of the candidates that pass the pair's
+# test (about one in six on the committed surface) are left out: their share
+# is not measured by a run, so the fraction reported is a lower one.
+HEADER_DRAWS = 4.02
+
+
+def pair_prune_ops(q, tail):
+    return HEADER_DRAWS * 20 + q * full_synth_ops(tail)
 
 
 def has_tail(model):
@@ -370,7 +383,7 @@ def _profile_summary() -> dict:
     """ncu figures of the default screen kernel kept under profiles/ (DRAM
     traffic per launch scaled to the full workload, pipe utilisation)."""
     try:
-        with open(os.path.join(ROOT, "profiles", "screen_pt_kernel_ncu.json")) as f:
+        with open(os.path.join(ROOT, "profiles", "screen_p_kernel_ncu.json")) as f:
             return json.load(f)
     except (OSError, ValueError):
         return {}
@@ -414,10 +427,9 @@ def issue_slots(achieved_tops, clocks):
 FORMS = (
     ("fp32_unpruned", "FLAG_NO_PRUNE", "every candidate synthesised and scored (FFMA filter, reference f32 "
                                        "order near the threshold): the plain FP32 form"),
-    ("fp32_prune_ffma", "FLAG_PRUNE_FFMA", "pruning, the bound's gradient by FP32 FMA; reference f32 order"),
-    ("bf16_tc", "FLAG_TC_BF16", "precision form: pruning bound on BF16 tensor cores, queued candidates "
-                                "filtered by FFMA and scored in FP64, survivors the FP64 top-K"),
-    ("fp16_tc", "FLAG_TC_FP16", "precision form as bf16_tc with FP16 tiles"),
+    ("bf16_tc", "FLAG_TC_BF16", "precision form: pruned by the pair, mask and own bounds (FP32), queued "
+                                "candidates filtered by FFMA and scored in FP64, survivors the FP64 top-K"),
+    ("fp16_tc", "FLAG_TC_FP16", "precision form as bf16_tc (the pruned screen has no tiles: the same kernel)"),
     ("bf16_tc_unpruned", "FLAG_TC_BF16|FLAG_NO_PRUNE", "precision form without pruning: the quadratic "
                                                         "block of every candidate on BF16 tensor cores, an "
                                                         "FP64 band"),
@@ -425,10 +437,10 @@ FORMS = (
 
 
 def precision_forms(args, default=None):
-    """The generation in each form beside the default (pruned, FP16 tensor-core
-    bound, reference f32 order): throughput (CUDA events, L2 flushed), screen
-    kernel time, candidates rescored, top-K recall against the FP64 top-K,
-    and the tensor-core scores' errors against FP64."""
+    """The generation in each form beside the default (pruned, reference f32
+    order): throughput (CUDA events, L2 flushed), screen kernel time,
+    candidates rescored, top-K recall against the FP64 top-K, and the
+    tensor-core scores' errors against FP64."""
     import numpy as np
     import torch
 
@@ -441,7 +453,8 @@ def precision_forms(args, default=None):
     out = {}
     forms = list(FORMS)
     if default is None:
-        forms.insert(0, ("fp32_prune_tc", "", "default: pruning, the bound's gradient on FP16 tensor cores"))
+        forms.insert(0, ("fp32_prune", "", "default: pruning by the parent pair's, the mask's and the "
+                                           "candidate's own bound; reference f32 order"))
     for name, flagnames, what in forms:
         flag = 0
         for fn in filter(None, flagnames.split("|")):
@@ -468,20 +481,18 @@ def precision_forms(args, default=None):
                      "ms_per_step": statistics.mean(ms), "screen_kernel_ms": statistics.mean(kms),
                      "rescored": info["exact_evals"], "screen_ctas": info["screen_ctas"],
                      "_surv": screen.survivors_from_bytes(d_out.cpu().numpy(), int(res[0]))}
-        if "TC" in flagnames:
-            # tensor work: pruned forms 2 x 16 x 16 flop per crossover candidate (the bound's
-            # gradient), the unpruned form one 128x16x16 MMA per 128 candidates (512 flop)
-            flop = 512.0 if "NO_PRUNE" in flagnames else PRUNE_TC_FLOP
-            tf = flop * args.lam / (statistics.mean(kms) * 1e-3) / 1e12
+        if "TC" in flagnames and "NO_PRUNE" in flagnames:
+            # tensor work: one 128x16x16 MMA per 128 candidates (512 flop each)
+            tf = 512.0 * args.lam / (statistics.mean(kms) * 1e-3) / 1e12
             pk = _measured_peaks().get("bf16_tflops") or 1900.0
             out[name]["tensor_roofline"] = {"achieved": tf, "peak": pk, "unit": "TFLOP/s", "frac": tf / pk,
                                             "note": "the tensor cores carry a 16x16 product per candidate; "
                                                     "the form stays bound by the integer synthesis"}
     if default is not None:
         v, ms_step, kms_, rescored, surv = default
-        out["fp32_prune_tc"] = {"form": "default: pruning, the bound's gradient on FP16 tensor cores (the line's "
-                                        "value)", "flags": "0", "value": v, "ms_per_step": ms_step,
-                                "screen_kernel_ms": kms_, "rescored": rescored, "_surv": surv}
+        out["fp32_prune"] = {"form": "default: pruning, reference f32 order (the line's value)", "flags": "0",
+                             "value": v, "ms_per_step": ms_step, "screen_kernel_ms": kms_, "rescored": rescored,
+                             "_surv": surv}
     # FP64 ground truth: the exact screen's top 4096 rescored in FP64, certified complete below
     big, _ = screen.screen(screen.Cfg(args.lam, 4096, SEED, threads=args.threads), model, el)
     s64 = _fp64_scores(model, big["g"])
@@ -492,7 +503,7 @@ def precision_forms(args, default=None):
     A = 16 * abs(float(model.w0)) + np.abs(model.w_lin).sum() + np.abs(L).sum()
     e32 = 36 * 2.0 ** -24 * A  # the exact order's FP32 error bound (gamma_35 of the absolute terms)
     certified = bool(float(big["score"][-1]) + e32 < s64[order[K - 1]])
-    ref = out["fp32_prune_tc"]["_surv"].tobytes()
+    ref = out["fp32_prune"]["_surv"].tobytes()
     for name in out:
         sv = out[name].pop("_surv")
         have = {(int(r["stream"]), int(r["index"])) for r in sv}
@@ -517,7 +528,7 @@ def precision_forms(args, default=None):
 
 
 def run_precision(args):
-    """`--workload precision`: the BF16 tensor-core form as the line's value."""
+    """`--workload precision`: the BF16 precision form as the line's value."""
     import torch
 
     torch.cuda.set_device(0)
@@ -530,10 +541,10 @@ def run_precision(args):
             "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": f["bf16_tc"]["ms_per_step"],
             "higher_is_better": True, "scaling": "weak", "vs_baseline": f["bf16_tc"]["value"] / PUBLISHED_CAND_S,
             "vs_baseline_source": PUBLISHED_SOURCE,
-            "dtype": "bf16 tensor cores (pruning bound) + f64 ranking; genes u64/f32", "data": "synthetic (seeded)",
+            "dtype": "f32 pruning bounds + f64 ranking; genes u64/f32", "data": "synthetic (seeded)",
             "config": workload_config(args, 1),
             "bf16_over_fp32": f["bf16_tc"]["value"] / f["fp32_unpruned"]["value"],
-            "bf16_over_fp32_pruned": f["bf16_tc"]["value"] / f["fp32_prune_tc"]["value"],
+            "bf16_over_fp32_pruned": f["bf16_tc"]["value"] / f["fp32_prune"]["value"],
             "clocks": clocks}
     line.update(p)
     print(json.dumps(line), flush=True)
@@ -541,8 +552,9 @@ def run_precision(args):
 
 def run_refit(args):
     """Differentiable refit: ridge refit (alpha 1e-2) of 400,000 rows x 16 genes
-    (seeded quadratic truth + Student-t(3) noise) on the GPU -- FP64 normal
-    equations and FP64 Cholesky -- beside the reference's own numpy FP64 refit
+    (seeded quadratic truth + Student-t(3) noise) on the GPU -- fixed-point
+    normal equations on the tensor cores and an FP64 LDL' solve -- beside the
+    reference's own numpy FP64 refit
     (brain/evolve.py:259-265) on the host cores; the surrogate's forward and
     backward kernels over the same rows."""
     import numpy as np
@@ -594,18 +606,27 @@ def run_refit(args):
     bench.csx_bench_issue_rate.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
     dfma = ctypes.c_double(0)
     bench.csx_bench_issue_rate(4, ctypes.byref(dfma))
-    gram_flop = 2.0 * n * (nf * (nf + 1) / 2 + nf)  # upper triangle + right-hand side, FP64
+    # every entry of the normal equations is a sum over the rows of one of the
+    # 4845 monomials of degree <= 4 in 16 genes (Gram) or of a feature times the
+    # target (right-hand side): the distinct products, each one multiply-add
+    distinct = 4845 + nf
+    gram_flop = 2.0 * n * distinct
     line = {"metric": "ridge refit time (400,000 rows x 16 genes, alpha 1e-2, FP64), 1 GB300", "value": ms_refit,
             "unit": "ms", "n_gpus": 1, "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms_refit,
-            "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "f64 (normal equations, "
-            "Cholesky); f32 genes", "data": "synthetic (seeded quadratic truth + 0.5 * Student-t(3) noise)",
+            "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "f64 (normal equations exact to "
+            "f64 in fixed point on the tensor cores, f64 solve); f32 genes", "data": "synthetic (seeded quadratic truth + 0.5 * Student-t(3) noise)",
             "config": {"workload": "ridge refit toward a zero prior: 400,000 rows of 16 genes, 153 features, alpha 1e-2",
                        "rows": n, "features": nf, "alpha": alpha, "l2": "flushed between steps (256 MiB write)"},
-            "stages_ms": {"normal_equations": ms_gram, "cholesky_solve": ms_solve},
-            "roofline": {"bound": "fp64", "kernel": "sg_gram_kernel", "achieved": gram_flop / (ms_gram * 1e-3) / 1e12,
+            "stages_ms": {"normal_equations": ms_gram, "solve": ms_solve},
+            "roofline": {"bound": "digit making and barriers", "kernel": "sg_gram_mma_kernel",
+                         "achieved": gram_flop / (ms_gram * 1e-3) / 1e12,
                          "peak": 2 * dfma.value / 1e12, "unit": "TFLOP/s",
                          "frac": gram_flop / (ms_gram * 1e-3) / (2 * dfma.value) if dfma.value else None,
-                         "peak_source": "measured: DFMA issue rate of this GPU (csx_bench_issue_rate kind 4)"},
+                         "peak_source": "measured: DFMA issue rate of this GPU (csx_bench_issue_rate kind 4), which "
+                                        "the tensor-core fixed point is not bound by: above 1 is past what the "
+                                        "distinct products would take on the FP64 pipe",
+                         "ops_model": "4845 distinct monomials of degree <= 4 + 153 targets, one multiply-add each "
+                                      "per row"},
             "vs_numpy_fp64": {"max_abs_diff": float(np.abs(w - w_np).max()), "max_abs_w": float(np.abs(w_np).max()),
                               "numpy_seconds": cpu_s, "host_threads": os.cpu_count(),
                               "speedup": cpu_s * 1000 / ms_refit},
@@ -652,8 +673,10 @@ def run_full(args):
     """`--workload full`: the generation workload screened on the full
     quadratic surface (all 29 genes; the committed v3 surrogate moved into the
     465-coefficient layout, new pairs 0): candidates/s by CUDA events, L2
-    flushed between steps, and the issue roofline at its algorithmic work
-    (1235 RNG + 145 gene + 2 x 464 FMA lane-ops per candidate)."""
+    flushed between steps, and the issue roofline: the header's 4.02 draws x 20
+    lane-ops, the 29 crossover bits of the 0.99 crossover candidates x 20 (the
+    bound reads them all), the bound's epilogue (29 x 4), and the full synthesis
+    and score (1235 RNG + 145 gene + 2 x 464 FMA) of the fraction queued."""
     import numpy as np
     import torch
 
@@ -687,7 +710,8 @@ def run_full(args):
         kms.append(screen.last_run_info()["ms_screen"])
     clocks = sampler.stop()
     info = screen.last_run_info()
-    ops = 1235 + 145 + 2 * 464
+    q = info["exact_evals"] / args.lam
+    ops = HEADER_DRAWS * 20 + 0.99 * (29 * 20 + 29 * 4) + q * (1235 + 145 + 2 * 464)
     achieved = args.lam / (statistics.mean(kms) * 1e-3) * ops / 1e12
     line = {"metric": "candidates/sec, full 29-gene quadratic surface, 1 GB300", "value":
             args.lam / (statistics.mean(ms) / 1000), "unit": "candidates/s", "n_gpus": 1, "steps": args.steps,
@@ -695,7 +719,7 @@ def run_full(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "u64/f32", "data": "synthetic (seeded)",
             "config": dict(workload_config(args, 1), surrogate="state/surrogate.txt (v3, 161) in the full "
                            "465-coefficient layout, new pairs 0"),
-            "roofline": dict(issue_slots(achieved, clocks), kernel="csx::screen_kernel<true, FullScreenArgs>",
+            "roofline": dict(issue_slots(achieved, clocks), kernel="csx::screen_ft_kernel", queued_fraction=q,
                              algorithmic_ops_per_candidate=ops, bound="int/fp32-issue"),
             "stages_ms_last_step": {k: round(v, 4) for k, v in info.items() if k.startswith("ms_")},
             "clocks": clocks, "gpu_launches": int(info["launches"]) * args.steps}
@@ -935,23 +959,22 @@ def main():
     cand_s_kernel = args.lam / (ms_screen / 1000.0)
     q = statistics.mean(st["exact_evals"] for st in stage) / args.lam  # queued for the reference order
     tail = has_tail(model)
-    ops = prune_ops(q, tail)
+    ops = pair_prune_ops(q, tail)
     achieved = cand_s_kernel * ops / 1e12
     slots = issue_slots(achieved, clocks)
     prof = _profile_summary()
     traffic = prof.get("bytes_per_launch_full_workload") if args.lam == LAMBDA else None
-    tc_tf = cand_s_kernel * PRUNE_TC_FLOP / 1e12
-    bf16_peak = _measured_peaks().get("bf16_tflops")
     roofline = {
-        "bound": "int-issue", "kernel": prof.get("kernel", "csx::screen_pt_kernel<16, true, false>"),
+        "bound": "int-issue", "kernel": prof.get("kernel", "csx::screen_p_kernel<false, false, false>"),
         "achieved": achieved, "peak": slots["peak"], "unit": "Tlane-op/s", "frac": slots["frac"],
         "peak_source": slots.get("peak_source"),
         "algorithmic_ops_per_candidate": ops,
-        "ops_model": ("pruning form: %.2f draws x 20 lane-ops (4 header draws, 0.02 jump index, 16 crossover "
-                      "bits for the 0.99 crossover candidates) + 0.99 x 72 bound lane-ops + q x %.1f for the "
-                      "fraction q queued for the synthesis and reference-order score (measured q; %s)"
-                      % (PRUNE_DRAWS, full_synth_ops(tail),
+        "ops_model": ("pruning form: %.2f header draws x 20 lane-ops (4 and 0.02 jump indices) + q x %.1f for the "
+                      "fraction q queued for the synthesis and reference-order score (measured q; %s); the bits "
+                      "and bounds of candidates past their pair's bound are not counted"
+                      % (HEADER_DRAWS, full_synth_ops(tail),
                          "genes 0..28" if tail else "genes 0..15: the surface has no linear weight past gene 15")),
+        "ops_with_every_own_bound": prune_ops(q, tail),
         "queued_fraction": q,
         "traffic": traffic,
         "traffic_source": prof.get("traffic_note"),
@@ -959,13 +982,10 @@ def main():
         "ncu": prof.get("ncu"),
         "issue_rates_measured": rates,
         "alu_probe_frac": (achieved / (rates["int_alu"] / 1e12)) if rates.get("int_alu") else None,
-        # the other two ceilings: HBM (the launch's DRAM traffic against the
-        # measured copy bandwidth) and the tensor pipe (the bound's gradient:
-        # 2 x 16 x 16 flop per crossover candidate)
+        # the HBM ceiling: the launch's DRAM traffic against the measured copy
+        # bandwidth (the pruned screen has no tensor work: its bounds are table
+        # reads and FP32 multiply-adds)
         "hbm": hbm_ceiling(traffic, ms_screen),
-        "tensor": {"achieved": tc_tf, "unit": "TFLOP/s", "peak": bf16_peak,
-                   "frac": tc_tf / bf16_peak if bf16_peak else None,
-                   "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst)"},
     }
     line = {"metric": METRIC, "value": value, "unit": "candidates/s",
             "n_gpus": world, "steps": args.steps, "warmup": max(3, args.warmup),
@@ -978,12 +998,12 @@ def main():
             "shape": dict({k: stage[-1][k] for k in ("screen_ctas", "segments", "seg_draws", "item_cands")},
                           items=int(res[3])),
             "exact_evals_last_step": stage[-1]["exact_evals"],
-            "form": "pruning screen: bound's gradient on the FP16 tensor cores, survivors in the reference's "
-                    "f32 order (byte-identical to the unpruned screen)",
+            "form": "pruning screen: parent-pair, mask and own bounds, survivors in the reference's f32 order "
+                    "(byte-identical to the unpruned screen)",
             "wall_s": wall}
     if world == 1 and not args.no_precision:
         # the other forms of the same generation beside this value: unpruned
-        # FP32, the FFMA bound, and the BF16 / FP16 precision forms
+        # FP32 and the BF16 / FP16 precision forms
         line["precision_forms"] = precision_forms(
             args, default=(value, line["ms_per_step"], ms_screen, stage[-1]["exact_evals"],
                            screen.survivors_from_bytes(d_out.cpu().numpy(), int(d_res[0].item()))))

@@ -2,7 +2,11 @@
 // of sm_103a kernels behind the C ABI of include/csx_screen.h. One
 // translation unit; its parts:
 //   csx_pipeline.cuh        types; item building (walk, link, assembly, items)
-//   csx_screen_kernels.cuh  screen kernels, merge tree, regeneration
+//   csx_dense.cuh           items of small generations from block maps
+//   csx_screen_kernels.cuh  unpruned screen kernels, merge tree, regeneration
+//   csx_prune.cuh           the pruning screen and its parent-pair tables
+//   csx_prune_full.cuh      the full surface's pruning screen
+//   csx_ties.cuh            heap replay of exact ties
 //   this file               host orchestration, the single-screen C ABI and
 //                           the allocation-free entry point
 //   csx_batch.cuh           batched islands
@@ -25,16 +29,19 @@
 //             and its stream-local start index (late meetings repaired locally).
 //  4. scan + emit  work items of <= D candidates with known start draw and
 //             stream-local index, in (stream, index) order.
-//  5. screen  persistent CTAs pull items; each thread synthesises and scores
-//             candidates in registers; those that beat the CTA's threshold go
+//  5. screen  persistent CTAs pull items; a candidate is skipped where a
+//             certified bound places it below the K-th score, else synthesised
+//             and scored in registers; those that beat the CTA's threshold go
 //             to a shared-memory buffer that is merged into the CTA's sorted
-//             top-K list (bitonic sort). HBM sees only items and survivors.
-//  6. merge   a tree of bitonic merges reduces the CTA lists.
+//             top-K list. HBM sees only items and survivors.
+//  6. merge   a tree of merges, up to eight lists at a time, reduces the CTA
+//             lists.
 //  7. regen   the K survivors are re-synthesised from (stream, draw) to
 //             recover genes and lineage; the score is re-checked bit for bit.
 //
 // The walk costs two hashes per candidate against ~62 for synthesis. When
-// streams are no longer than one item, steps 1-4 are skipped.
+// streams are no longer than one item, steps 1-4 are skipped; a small
+// generation takes its items from block maps instead.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -370,13 +377,6 @@ void dense_geometry(const csx_cfg &cfg, uint64_t lam, Plan *pl) {
     g.ckcap = kDenseWords;
 }
 
-// A share of one generation's work items (csx_screen_items): every share
-// builds the same item list and screens its part of it.
-struct Shard {
-    uint32_t index = 0, count = 1;
-};
-
-// grid_override, item_cands, seg_cands: 0 = automatic (the batched screen
 // Candidates per thread of a three-CTA-per-SM grid from which pruning pays: the
 // threshold then settles early enough, and the pair tables, which grow with
 // the elites, are a small part. A call's ms, pruned / unpruned, on 152 SMs:
@@ -401,6 +401,13 @@ uint64_t prune_floor(bool precision, bool full, int batch_n, int ne) {
     return std::min<uint64_t>(400, 128 + 17 * e / 16);
 }
 
+// A share of one generation's work items (csx_screen_items): every share
+// builds the same item list and screens its part of it.
+struct Shard {
+    uint32_t index = 0, count = 1;
+};
+
+// grid_override, item_cands, seg_cands: 0 = automatic (the batched screen
 // passes its own grid and the tuner's sizes). A sharded call sizes its items
 // by a fixed SM count, so that every share's item list is the same whatever
 // GPU it runs on. An island of a batch passes the batch's candidates and

@@ -3,7 +3,8 @@ tensor cores (tcgen05, FP32 accumulation) with genes in BF16, or in FP16 with
 the per-gene map x' = 2g - 1 onto [-1, 1]; constant and linear terms in FP32.
 The reference scores in FP32 only (src/screen.zig:97-112); this form exists to
 trade score precision for tensor-core throughput, with its error measured
-against FP64.
+against FP64. The screen uses it with FLAG_TC_* and FLAG_NO_PRUNE; pruned, the
+FLAG_TC_* screens rank by FP64 scores and need no tile.
 """
 from __future__ import annotations
 

@@ -63,7 +63,7 @@ enum {
                                       on the tensor cores and candidates within max(1e-3 relative,
                                       the form's certified error bound) of the K-th score are
                                       rescored in FP64. csx_screen / csx_screen_device */
-#define CSX_FLAG_TC_FP16 0x40u     /* the same with FP16 tiles (unpruned: x' = 2g - 1) */
+#define CSX_FLAG_TC_FP16 0x40u     /* the same; unpruned with FP16 tiles (x' = 2g - 1) */
 #define CSX_FLAG_NO_PRUNE 0x80u    /* score every candidate's full synthesis (the filter form)
                                       instead of skipping, by certified bounds taken from the parent
                                       pair and after the crossover bits, candidates that cannot
@@ -343,7 +343,8 @@ typedef struct csx_model_full {
 
 /* n must be CSX_FULL_NF (else CSX_ERR_BAD_MODEL). */
 int csx_model_full_from_compact(const float *w, int n, csx_model_full *out);
-/* csx_screen / csx_screen_device with the candidates scored on the full
+/* csx_screen / csx_screen_device (pruned from the same floor unless
+ * CSX_FLAG_NO_PRUNE is set, with the same results) with the candidates scored on the full
  * surface. The precision-form flags are refused (CSX_ERR_BAD_ARGS). */
 int csx_screen_full(const csx_cfg *cfg, const csx_model_full *model, const csx_genome *elites, int n_elites,
                     csx_survivor *out, uint64_t out_cap, uint64_t *n_out, uint64_t *screened);

@@ -2,7 +2,7 @@
  * csx_surrogate.h — the quadratic surrogate as a differentiable function on
  * the GPU: batched forward, hand-written backward (d score / d genes and
  * d loss / d coefficients), the ridge refit's normal equations and an FP64
- * Cholesky solve, and a gradient-guided mutation step.
+ * solve, and a gradient-guided mutation step.
  *
  * These replace brain/evolve.py:211-268 (features, refit_surrogate: numpy
  * FP64 `solve((XᵀX + αI), Xᵀy + αw₀)`) and give the screen's surrogate
@@ -74,7 +74,7 @@ int csx_sg_backward_coef_f64(int nf, const float *d_genes, int64_t n, int ldg, c
 int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, const double *d_fit,
                             double *d_gram, double *d_rhs, void *d_work, void *stream);
 
-/* Ridge solve in FP64 by Cholesky on one CTA: w = (G + αI)⁻¹ (rhs + α·prior).
+/* Ridge solve in FP64 (LDL' on a cluster; Cholesky on one CTA for 465): w = (G + αI)⁻¹ (rhs + α·prior).
    d_prior may be NULL (zero prior). d_status (one int) receives 0, or k+1
    when the k-th pivot is not positive. nf <= 166, or 465 (the factor then
    lives in a scratch allocated and freed on `stream`). */
