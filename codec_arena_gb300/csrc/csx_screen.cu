@@ -391,11 +391,11 @@ void dense_geometry(const csx_cfg &cfg, uint64_t lam, Plan *pl) {
 // 1.38/1.66 at 4e6; 256: 1.30/1.24 at 3e6, 1.81/1.93 at 6e6); the full surface
 // has no tables (1.6e7: 2.51/2.43 to 2.23/2.79, 2.4e7: 3.11/3.15, 2.73/3.52). A
 // batch of batch_n > 0 islands counts its mean island, each with a screen of its own
-// instead of one launch for all (20 islands, ms: mean 2e7 19.3/16.7, 4e7
-// 29.2/29.8, 8e7 40.5/51.6).
+// instead of one launch for all (20 islands, ms: mean 1.9e7 18.0/16.8, 3.7e7
+// 28.0/29.7, 7.4e7 38.9/51.6; 5 islands: 5.3/5.4, 6.7/8.2, 12.5/17.0).
 uint64_t prune_floor(bool precision, bool full, int batch_n, int ne) {
     const uint64_t e = static_cast<uint64_t>(ne);
-    if (batch_n > 0) return 400;
+    if (batch_n > 0) return 250;
     if (precision) return 12 + e / 8;
     if (full) return 180;
     return std::min<uint64_t>(400, 128 + 17 * e / 16);

@@ -7,7 +7,7 @@ CUDA-graph launch of one pipeline and returns, per island, exactly what
 `screen.screen` returns for that island alone. The islands' item building runs
 on parallel streams; then, when every island's surrogate admits the pruning
 bound and the islands are on average large enough for pruning to pay (the
-library's pruning floor), each island's pruning screen runs in turn over the whole GPU,
+library's pruning floor), each island's pruning screen runs over the whole GPU as its items are ready,
 else one unpruned persistent screen kernel takes every island's candidates (a
 FLAG_NO_PRUNE island selects that form for its batch). `Tune` holds the pipeline's tunables, which
 change speed only; `autotune` picks them by timing.

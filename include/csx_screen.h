@@ -73,7 +73,7 @@ enum {
                                       128 + 17/16 n_elites candidates per screen thread, at most 400
                                       (3 CTAs x 256 threads per SM: 2.3e7 candidates with 64 elites,
                                       4.67e7 with 256 on 152 SMs; the precision form 12 + n_elites/8,
-                                      the full surface 180, a batch a mean of 400 per island; below,
+                                      the full surface 180, a batch a mean of 250 per island; below,
                                       the unpruned kernel is faster); the environment variable
                                       CSX_PRUNE_MIN_CANDS sets that floor in candidates */
 #define CSX_FLAG_PRUNE_FFMA 0x100u /* the pruning bound's gradient by FP32 FMA: accepted, and what
@@ -256,7 +256,7 @@ int csx_last_run_info(csx_run_info *out);
  * items are built on its own forked stream; then, when every island's
  * surrogate admits the pruning bound and every island is above
  * the pruning floor (CSX_FLAG_NO_PRUNE), each island's pruning screen runs
- * over the whole GPU in turn, else (or when any island carries
+ * over the whole GPU, else (or when any island carries
  * CSX_FLAG_NO_PRUNE) ONE unpruned persistent screen launch consumes all
  * islands' items and keeps a top-K per island; one merge tree and one
  * regeneration launch serve all islands. Results per island equal
