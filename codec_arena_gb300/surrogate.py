@@ -80,15 +80,21 @@ class _Score(torch.autograd.Function):
         genes, coef_c = ctx.saved_tensors
         gout = gout.detach().to(torch.float32).contiguous()
         want_g, want_c = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-        dgenes = torch.empty_like(genes) if want_g else None
+        dgenes = None
+        if want_g:
+            # the kernel writes rows at the stride it reads them, which a column
+            # slice's gradient has no room for
+            if genes.stride(0) != genes.shape[1]:
+                genes = genes.clone(memory_format=torch.contiguous_format)
+            dgenes = torch.empty_like(genes)
         f32 = ctx.coef_dtype == torch.float32  # the kernel rounds its FP64 sums itself
         dcoef = torch.empty(coef_c.numel(), dtype=torch.float32 if f32 else torch.float64,
                             device=genes.device) if want_c else None
         work = workspace(genes.device, coef_c.numel()) if want_c else None
         fn = lib().csx_sg_backward_f32 if f32 else lib().csx_sg_backward
-        check(fn(coef_c.data_ptr(), coef_c.numel(), genes.data_ptr(), genes.shape[0],
-                                    genes.stride(0), ctx.precision, gout.data_ptr(), _ptr(dgenes), _ptr(dcoef),
-                                    _ptr(work), _stream(genes.device)), "sg_backward")
+        check(fn(coef_c.data_ptr(), coef_c.numel(), genes.data_ptr(), genes.shape[0], genes.stride(0),
+                 ctx.precision, gout.data_ptr(), _ptr(dgenes), _ptr(dcoef), _ptr(work), _stream(genes.device)),
+              "sg_backward")
         return dgenes, (dcoef if f32 or not want_c else dcoef.to(ctx.coef_dtype)), None
 
 
