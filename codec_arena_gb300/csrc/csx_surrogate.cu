@@ -592,7 +592,7 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
         }
     }
     int bad = 0;  // thread 0's count is the one reported
-    __syncthreads();
+    cluster.sync();  // own rows are in, and every CTA runs before another writes its shared memory
     for (int k0 = 0, buf = 0; k0 < n; k0 += kSolveNb, buf ^= 1) {
         const int nb = min(kSolveNb, n - k0);
         double *Pb = P + buf * (n + 1) * kSolveNb;
