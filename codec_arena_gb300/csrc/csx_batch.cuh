@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_batch_kernel(const __grid_
     Pend pdef{0u, 0u, 0u};
 
     // merge the buffer into the CTA's sorted list; publishes the island's threshold
-    auto merge = [&]() {
-        cta_merge_top(E, s_kpad, B.sort_n, min(s_buf_n, B.sort_n - s_kpad));
+    auto merge = [&](uint32_t bn) {
+        cta_merge_top(E, s_kpad, B.sort_n, min(bn, B.sort_n - s_kpad));
         if (tid == 0) {
             s_buf_n = 0;
             const Entry kth = E[s_keep - 1];
@@ -161,12 +161,13 @@ __global__ void __launch_bounds__(kThreads, 3) screen_batch_kernel(const __grid_
     for (;;) {
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
+        unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
         const int any = __syncthreads_or(valid || has_def);
         const int any_def = __syncthreads_or(has_def);
         const int cur = s_cur;
         if (kFilter && cur >= 0 && (pn >= kThreads || any_def || (!any && pn > 0))) {
             // a flush appends <= pn + 256 <= 768 entries
-            if (s_buf_n + kPendCap + kThreads > s_buf_cap) merge();
+            if (bn + kPendCap + kThreads > s_buf_cap) merge(bn);
             unsigned long long t1 = s_t1, t2 = s_t2;
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&s_ctrl->gtau);
@@ -181,11 +182,11 @@ __global__ void __launch_bounds__(kThreads, 3) screen_batch_kernel(const __grid_
                 has_def = false;
             }
             __syncthreads();
+            bn = s_buf_n;
             if (tid == 0) s_pend_n = 0;
             __syncthreads();
         }
-        const unsigned int bn = s_buf_n;
-        if (cur >= 0 && (bn >= s_buf_cap / 2 || (!any && bn > 0))) merge();
+        if (cur >= 0 && (bn >= s_buf_cap / 2 || (!any && bn > 0))) merge(bn);
         if (!any) {
             if (cur >= 0) {  // publish this CTA's list and counts for the island it leaves
                 Entry *out = s_lists + static_cast<size_t>(blockIdx.x) * s_kpad;

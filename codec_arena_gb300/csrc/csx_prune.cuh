@@ -123,10 +123,10 @@ __device__ __forceinline__ uint32_t warp_kth_largest(const uint32_t *v, uint32_t
 }
 
 template <class Args>
-__device__ __noinline__ void prune_merge(const Args *A, Entry *E, uint32_t *sel, unsigned int *s_buf_n,
+__device__ __noinline__ void prune_merge(const Args *A, Entry *E, uint32_t *sel, uint32_t bn, unsigned int *s_buf_n,
                                          unsigned long long *s_t1, unsigned long long *s_t2, float *s_ts) {
     const uint32_t tid = threadIdx.x;
-    cta_merge_top(E, A->kpad, A->sort_n, *s_buf_n);
+    cta_merge_top(E, A->kpad, A->sort_n, bn);
     if (tid == 0) {
         *s_buf_n = 0;
         const Entry kth = E[A->keep - 1];
@@ -540,17 +540,18 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         }
     };
 
-    auto merge = [&]() { prune_merge(&A, E, sel, &s_buf_n, &s_t1, &s_t2, &s_ts); };
+    auto merge = [&](uint32_t bn) { prune_merge(&A, E, sel, bn, &s_buf_n, &s_t1, &s_t2, &s_ts); };
 
     for (;;) {
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
+        unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
         const int any = __syncthreads_or(valid || n_def > 0 || n1 + n2 > 0);
         const int any_def = __syncthreads_or(n_def > 0);
         // the queue is evaluated once it can employ every thread (or a thread
         // waits on it, or the work is done); a flush appends <= pn + 2 x 256 <= 1024
         if (pn >= kThreads || any_def || (!any && pn > 0)) {
-            if (s_buf_n + kPendCap + 2 * kThreads > A.buf_cap) merge();  // make room first
+            if (bn + kPendCap + 2 * kThreads > A.buf_cap) merge(bn);  // make room first
             unsigned long long t1 = s_t1, t2 = s_t2;
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
@@ -563,14 +564,14 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
             for (uint32_t i = 0; i < n_def; ++i) rescore(i == 0 ? def[0] : def[1], t1, t2, ts);
             n_def = 0;
             __syncthreads();
+            bn = s_buf_n;
             if (tid == 0) s_pend_n = 0;
             __syncthreads();
         }
         // merge when half full, and every kPruneMergeRounds rounds while the
         // buffer holds anything: the CTA's threshold and published keys then
         // follow the candidates it finds instead of waiting for a full buffer
-        const unsigned int bn = s_buf_n;
-        if (bn >= A.buf_cap / 2 || (bn > 0 && (!any || (round & (kPruneMergeRounds - 1)) == 0))) merge();
+        if (bn >= A.buf_cap / 2 || (bn > 0 && (!any || (round & (kPruneMergeRounds - 1)) == 0))) merge(bn);
         if (!any) break;
         float ts = s_ts;
         const unsigned long long t1 = s_t1;

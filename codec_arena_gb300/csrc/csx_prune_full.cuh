@@ -242,11 +242,12 @@ __global__ void __launch_bounds__(kThreads, 3) screen_ft_kernel(const __grid_con
             buf[atomicAdd(&s_buf_n, 1u)] = Entry{k1, k2};  // score >= ts: ties with the K-th kept
         }
     };
-    auto merge = [&]() { prune_merge(&A, E, sel, &s_buf_n, &s_t1, &s_t2, &s_ts); };
+    auto merge = [&](uint32_t bn) { prune_merge(&A, E, sel, bn, &s_buf_n, &s_t1, &s_t2, &s_ts); };
 
     for (;;) {
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
+        unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
         // a group whose tensor-core wait gave up ends the CTA's screening
         const int stop = (s_gbad[0] | s_gbad[1]) != 0u;
         // the bound left more than half of the last round: off for a round (the
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_ft_kernel(const __grid_con
         const int any_def = __syncthreads_or(has_def);
         if (tid == 0) s_passed = s_seen = 0;
         if (pn >= kThreads || any_def || (!any && pn > 0)) {
-            if (s_buf_n + kPendCap + kThreads > A.buf_cap) merge();  // make room first
+            if (bn + kPendCap + kThreads > A.buf_cap) merge(bn);  // make room first
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
             if ((static_cast<unsigned long long>(g) << 32) > s_t1) ts = okey_score(g);
@@ -279,11 +280,11 @@ __global__ void __launch_bounds__(kThreads, 3) screen_ft_kernel(const __grid_con
                 rescore(q, ts);
             }
             __syncthreads();
+            bn = s_buf_n;
             if (tid == 0) s_pend_n = 0;
             __syncthreads();
         }
-        const unsigned int bn = s_buf_n;
-        if (bn >= A.buf_cap / 2 || (bn > 0 && (!any || (round & 3u) == 0))) merge();
+        if (bn >= A.buf_cap / 2 || (bn > 0 && (!any || (round & 3u) == 0))) merge(bn);
         if (!any) break;
         float ts = s_ts;
         gk = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);

@@ -324,8 +324,8 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
     };
 
     // merge the buffer into the CTA's sorted list; publishes the threshold
-    auto merge = [&]() {
-        cta_merge_top(E, A.kpad, A.sort_n, s_buf_n);
+    auto merge = [&](uint32_t bn) {
+        cta_merge_top(E, A.kpad, A.sort_n, bn);
         if (tid == 0) {
             s_buf_n = 0;
             const Entry kth = E[A.keep - 1];
@@ -343,12 +343,13 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
     for (;;) {
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
+        unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
         const int any = __syncthreads_or(valid || has_def);
         const int any_def = __syncthreads_or(has_def);
         // the queue is evaluated once it can employ every thread (or a thread
         // waits on it, or the work is done); a flush appends <= pn + 256 <= 768
         if (pn >= kThreads || any_def || (!any && pn > 0)) {
-            if (s_buf_n + kPendCap + kThreads > A.buf_cap) merge();  // make room first
+            if (bn + kPendCap + kThreads > A.buf_cap) merge(bn);  // make room first
             unsigned long long t1 = s_t1, t2 = s_t2;
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
@@ -363,11 +364,11 @@ __global__ void __launch_bounds__(kThreads, 2) screen_q_kernel(const __grid_cons
                 has_def = false;
             }
             __syncthreads();
+            bn = s_buf_n;
             if (tid == 0) s_pend_n = 0;
             __syncthreads();
         }
-        const unsigned int bn = s_buf_n;
-        if (bn >= A.buf_cap / 2 || (!any && bn > 0)) merge();
+        if (bn >= A.buf_cap / 2 || (!any && bn > 0)) merge(bn);
         if (!any) break;
         float ts = s_ts;
         const unsigned long long t1 = s_t1;
@@ -681,8 +682,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
     };
 
     // merge the buffer into the CTA's sorted list; publishes the threshold
-    auto merge = [&]() {
-        cta_merge_top(E, A.kpad, A.sort_n, s_buf_n);
+    auto merge = [&](uint32_t bn) {
+        cta_merge_top(E, A.kpad, A.sort_n, bn);
         if (tid == 0) {
             s_buf_n = 0;
             const Entry kth = E[A.keep - 1];
@@ -700,6 +701,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
     for (;;) {
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
+        unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
         // a group whose tensor-core wait gave up ends the CTA's screening
         const int stop = (s_gbad[0] | s_gbad[1]) != 0u;
         const int any = __syncthreads_or((valid || has_def) && !stop);
@@ -707,7 +709,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
         // the queue is scored once it can employ every thread (or a thread
         // waits on it, or the work is done); a flush appends <= pn + 256 <= 768
         if (pn >= kThreads || any_def || (!any && pn > 0)) {
-            if (s_buf_n + kPendCap + kThreads > A.buf_cap) merge();  // make room first
+            if (bn + kPendCap + kThreads > A.buf_cap) merge(bn);  // make room first
             unsigned long long t1 = s_t1, t2 = s_t2;
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
@@ -722,11 +724,11 @@ __global__ void __launch_bounds__(kThreads, 3) screen_tc_kernel(const __grid_con
                 has_def = false;
             }
             __syncthreads();
+            bn = s_buf_n;
             if (tid == 0) s_pend_n = 0;
             __syncthreads();
         }
-        const unsigned int bn = s_buf_n;
-        if (bn >= A.buf_cap / 2 || (!any && bn > 0)) merge();
+        if (bn >= A.buf_cap / 2 || (!any && bn > 0)) merge(bn);
         if (!any) break;
         unsigned long long t1 = s_t1;
         float ts = s_ts;
