@@ -575,7 +575,8 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         if (!any) break;
         float ts = s_ts;
         const unsigned long long t1 = s_t1;
-        gk = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
+        // one lane's reading for the whole warp: the ballots below stand under it
+        gk = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau), 0);
         if ((static_cast<unsigned long long>(gk) << 32) > t1) ts = okey_score(gk);
         const float tlo = __fsub_rd(ts, A.pc.err);
         // rebuild the bitmap: early on at rounds 1, 2, 4, ..., then every bm_period

@@ -116,3 +116,19 @@ def test_batch_prunes_by_its_mean_island(monkeypatch, floor):
         if c.lambda_:
             want, _ = screen.screen(c, m, e)
             assert surv.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("ne", [5, 33, 64, 362])
+def test_thresholds_that_settle_elsewhere(monkeypatch, ne):
+    """Lists longer than a CTA's own finds: its first finite threshold arrives from
+    other CTAs while it screens, at the rounds that rebuild the pair bitmap."""
+    from codec_arena_gb300 import _lib, screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    m = screen.Model.from_compact(np.random.default_rng(ne).normal(0, 1, 153).astype(np.float32))
+    el = wl.seeded_elites(ne, seed=ne)
+    for seed in range(8):
+        for lam, keep in ((900_001, 700), (5_000_003, 1500)):
+            got, n = screen.screen(screen.Cfg(lam, keep, seed, threads=5), m, el)
+            ref, _ = screen.screen(screen.Cfg(lam, keep, seed, threads=5, flags=_lib.FLAG_NO_PRUNE), m, el)
+            assert n == lam and got.tobytes() == ref.tobytes(), (seed, lam)
