@@ -49,6 +49,7 @@ constexpr int kGmThreads = kGmTasks + 32;  // and a warp that issues the MMAs (i
 constexpr int kGmVars = 32;       // variables per row: g_0..g_15, 1, linear-only genes
 constexpr uint32_t kGmA = 128 * kGmRows * 2, kGmB = kGmN * kGmRows * 2;  // bytes of one digit's tiles
 constexpr uint32_t kGmBuf = kDigits * (kGmA + kGmB);
+constexpr size_t kGmPartBytes = static_cast<size_t>(kGmChunks) * kGmBlocks * kGmOutRows * kGmN * sizeof(longlong2);
 constexpr size_t kGmSmem = 1024 + 2 * kGmBuf + kGmRows * (kGmVars - 1) * sizeof(int2) + kGmRows * sizeof(int64_t);
 
 // What the range pass leaves: the largest |value| of each gene (as f32 bits)

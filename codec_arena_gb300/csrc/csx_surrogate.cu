@@ -843,6 +843,8 @@ int gram_parts(int nf) { return is_full(nf) ? kPartBlocksFull : kPartBlocks; }
 size_t part_gram_bytes(int nf) {
     return static_cast<size_t>(gram_parts(nf)) * gram_pairs(nf) * kGramBlk * kGramBlk * sizeof(double);
 }
+static_assert(kGmPartBytes + 15 <= static_cast<size_t>(kPartBlocks) * gram_pairs(kMaxFeat) * kGramBlk * kGramBlk * sizeof(double),
+              "the fixed-point sums end before part_r");
 constexpr size_t kPartCoefBytes = static_cast<size_t>(kPartBlocks) * kFeatCap * sizeof(double);
 size_t gram_smem(int nf) { return static_cast<size_t>(kGramRows) * gram_nb(nf) * kGramBlk * sizeof(double); }
 
@@ -1003,7 +1005,9 @@ int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, co
     GramRange *range = nullptr;
     if (!is_full(nf)) {
         range = reinterpret_cast<GramRange *>(reinterpret_cast<char *>(part_r) + kPartCoefBytes - sizeof(GramRange));
-        auto *part = static_cast<longlong2 *>(d_work);
+        // 16-byte entries in a workspace that is only asked to hold doubles: from
+        // its next such boundary (they take 11 of the 17 MB before part_r)
+        auto *part = reinterpret_cast<longlong2 *>((reinterpret_cast<uintptr_t>(d_work) + 15) & ~uintptr_t{15});
         SG_CUDA(cudaMemsetAsync(range, 0, sizeof(GramRange), s));
         sg_range_kernel<<<static_cast<unsigned>(std::min<int64_t>(n / 64 + 1, 152 * 4)), 256, 0, s>>>(
             ng, d_genes, n, ldg, d_fit, range);

@@ -78,3 +78,29 @@ def test_non_finite_tables_keep_the_fp64_kernel(where):
         want, wrhs = phi.T @ phi, phi.T @ y
     np.testing.assert_allclose(gram, want, rtol=1e-12)
     np.testing.assert_allclose(rhs, wrhs, rtol=1e-9, atol=1e-9)
+
+
+@pytest.mark.parametrize("off", [0, 8, 16, 24])
+@pytest.mark.parametrize("ng", [16, 29])
+def test_workspace_at_any_double(off, ng):
+    """A workspace of the stated size from any 8-byte boundary: the same bits, and
+    nothing written around it."""
+    import torch
+
+    from codec_arena_gb300 import _lib, surrogate
+
+    rng = np.random.default_rng(ng)
+    n, nf = 6401, 1 + ng + 136
+    genes = torch.from_numpy(rng.random((n, ng), dtype=np.float32)).cuda()
+    y = torch.from_numpy(rng.normal(0, 3, n)).cuda()
+    want, wrhs = surrogate.normal_equations(genes, y, nf)
+    size = int(_lib.lib().csx_sg_workspace_bytes(nf))
+    buf = torch.full((size + 64,), 0x5a, dtype=torch.uint8, device="cuda")
+    assert buf.data_ptr() % 16 == 0
+    gram = torch.empty((nf, nf), dtype=torch.float64, device="cuda")
+    rhs = torch.empty(nf, dtype=torch.float64, device="cuda")
+    _lib.check(_lib.lib().csx_sg_normal_equations(nf, genes.data_ptr(), n, ng, y.data_ptr(), gram.data_ptr(),
+                                                  rhs.data_ptr(), buf.data_ptr() + off,
+                                                  torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(gram, want) and torch.equal(rhs, wrhs)
+    assert (buf[:off] == 0x5a).all() and (buf[off + size:] == 0x5a).all()
