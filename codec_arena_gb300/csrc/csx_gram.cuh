@@ -1,5 +1,7 @@
 // csx_gram.cuh — the refit's normal equations ΦᵀΦ and Φᵀy on the tensor
-// cores, in fixed point, exact to 2^-56 of each feature's largest value.
+// cores, in fixed point: each row's products to 8.1 x 2^-56 of the product of
+// their variables' largest values. Tables with an entry for which FP64 sums
+// would be closer are left to the FP64 kernel.
 // Part of csx_surrogate.cu's translation unit (included there); not a
 // standalone header.
 //
@@ -31,6 +33,24 @@
 // two genes a 48-bit integer shifted by both and rounded to 2^-55 of
 // 2^(E_a+E_b). A table with an infinite or NaN entry is left to the FP64
 // kernel.
+//
+// Small entries. The rounding is relative to the scale 2^(E_a+E_b+E_c+E_d) of
+// an entry Σ_r φ φ', not to the entry: two genes that are never large together
+// leave products of 1e-9 with 25 bits, and their squares with eight. The
+// errors of n rows (8.1 x 2^-56 of the scale at most each; by chance their
+// sum's s.d. is about sqrt(n) 2^-57 of it) are below the 2^-54 of the last
+// rounding of an FP64 sum where the entry's magnitude Σ_r |φ φ'| is at least
+// sqrt(n) / 8 of its scale. So every entry is held against that line
+// (kGmSmall): where one of them, or one of Φᵀy by the sum of φ |y| (a row of
+// its own), is below, the FP64 kernel takes the table. A sum whose terms cancel
+// (genes of both signs) can only be taken for small. Largest error over the
+// entries, in units of 2^-53 of the entry, fixed point / FP64 sums, emulated at
+// 4,999 rows: uniform genes 1.0/3.3, a population 1.1/3.3, its genes and 1%
+// immigrants 1.1/3.0; two genes of which one is 100 times smaller in every
+// row 615/3.0, 1e4 times 4e5/3.2. Such a table takes the FP64 kernel's time and
+// the fixed point's: 400,000 rows of 16 genes 9.5 ms instead of 0.69, 4,999 of
+// 29 0.20 instead of 0.054. The check costs the others 2 to 16 us (two launches
+// that leave at once, and from 22 genes on one digit per A tile).
 #pragma once
 
 namespace {
@@ -43,9 +63,10 @@ constexpr int kGmDrain = 4;
 constexpr int kGmN = 64;          // features per column block
 constexpr int kGmBlocks = 3;      // column blocks (166 features at most)
 constexpr int kGmChunks = 50;     // row chunks: 150 CTAs
-constexpr int kGmOutRows = 72;    // pair rows (57) + linear-only genes (13) + y, rounded up
+constexpr int kGmOutRows = 72;    // pair rows (57) + linear-only genes (13) + y + |y|
 constexpr int kGmTasks = 544;     // digit tasks per stage, one per thread: 136 values x 4 groups of 8 rows
 constexpr int kGmThreads = kGmTasks + 32;  // and a warp that issues the MMAs (it waits where their queue is full)
+constexpr double kGmSmall = 0.125;  // an entry's magnitude over sqrt(n) scales from which fixed point is taken
 constexpr int kGmVars = 32;       // variables per row: g_0..g_15, 1, linear-only genes
 constexpr uint32_t kGmA = 128 * kGmRows * 2, kGmB = kGmN * kGmRows * 2;  // bytes of one digit's tiles
 constexpr uint32_t kGmBuf = kDigits * (kGmA + kGmB);
@@ -53,11 +74,13 @@ constexpr size_t kGmPartBytes = static_cast<size_t>(kGmChunks) * kGmBlocks * kGm
 constexpr size_t kGmSmem = 1024 + 2 * kGmBuf + kGmRows * (kGmVars - 1) * sizeof(int2) + kGmRows * sizeof(int64_t);
 
 // What the range pass leaves: the largest |value| of each gene (as f32 bits)
-// and of y (as FP64 bits), and the flag of a wait that gave up.
+// and of y (as FP64 bits); the flag of a wait that gave up, and of a table with
+// an entry too small beside its scale.
 struct GramRange {
     unsigned long long ymax;
     uint32_t gmax[kMaxLin];
     uint32_t err;
+    uint32_t small;
 };
 
 __device__ __forceinline__ bool gram_finite(const GramRange *r, int ng) {
@@ -65,6 +88,9 @@ __device__ __forceinline__ bool gram_finite(const GramRange *r, int ng) {
     for (int k = 0; k < ng; ++k) ok = ok && (r->gmax[k] >> 23) < 255;
     return ok;
 }
+
+// Whether the fixed-point sums stand (known once sg_gram_final_kernel is through).
+__device__ __forceinline__ bool gram_fixed(const GramRange *r, int ng) { return r->small == 0 && gram_finite(r, ng); }
 
 // E with |x| <= 2^E for every |x| whose f32 bits are at most `bits`.
 __device__ __forceinline__ int range_exp(uint32_t bits) {
@@ -129,7 +155,7 @@ __host__ __device__ __forceinline__ int pair_row(int a, int b) {
 constexpr int kPairRows = 57;
 
 // Row q of the A side as a pair of variables (linear-only gene k is variable
-// 17 + k - 16; its partner is the 1); y is (255, 255).
+// 17 + k - 16; its partner is the 1); y is (255, 255), |y| (253, 253).
 __device__ __forceinline__ void gram_row_vars(int q, int ng, int &a, int &b) {
     if (q < kPairRows) {
         const int p = q < 21 ? 0 : q < 42 ? 1 : 2;
@@ -141,7 +167,7 @@ __device__ __forceinline__ void gram_row_vars(int q, int ng, int &a, int &b) {
         a = 17 + q - kPairRows;
         b = 16;
     } else {
-        a = b = 255;
+        a = b = q == kPairRows + ng - 16 ? 255 : 253;
     }
 }
 // Feature f as a pair of variables, in the same numbering.
@@ -192,7 +218,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
     unsigned char *bufs = smem_raw + (base - csx::smem_u32(smem_raw));
     int2 *vars = reinterpret_cast<int2 *>(bufs + 2 * kGmBuf);             // [row][kGmVars - 1]: significand, shift
     int64_t *yint = reinterpret_cast<int64_t *>(vars + kGmRows * (kGmVars - 1));  // y 2^(55 - E_y)
-    const int n_rows = kPairRows + (ng - 16) + 1;                          // A rows in use
+    const int n_rows = kPairRows + (ng - 16) + 2;                          // A rows in use
     const int f0 = blockIdx.y * kGmN, n_feat = min(kGmN, nf - f0);
     for (uint32_t i = tid; i < 2 * kGmBuf / 16; i += kGmThreads) reinterpret_cast<uint4 *>(bufs)[i] = uint4{0, 0, 0, 0};
     if (tid < kGmOutRows + kGmN) {
@@ -278,8 +304,9 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
             for (int e = 0; e < 8; ++e) {
                 const int r = kg * 8 + e;
                 int64_t v;
-                if (a == 255u) {
-                    v = yint[r] + 0x0080808080808080ll;
+                if (a == 255u || a == 253u) {
+                    const int64_t yi = yint[r];
+                    v = (a == 253u && yi < 0 ? -yi : yi) + 0x0080808080808080ll;
                 } else {
                     const int2 va = vars[r * (kGmVars - 1) + a], vb = vars[r * (kGmVars - 1) + b];
                     const int64_t p = static_cast<int64_t>(va.x) * vb.x;  // the product, 10 bits up
@@ -419,98 +446,136 @@ __global__ void __launch_bounds__(kGmThreads, 1) sg_gram_mma_kernel(int ng, int 
     if (warp == 0) csx::tc_dealloc(tmem, 512);
 }
 
-// Entry e of the packed lower triangle of ΦᵀΦ, then of Φᵀy: which row and
-// feature of the MMA it is, the chunks' sums (eight threads per entry), and its
-// scale. With a non-finite table, the FP64 kernel's parts instead.
-__global__ void __launch_bounds__(32 * kSumSplit) sg_gram_final_kernel(int ng, int nf, int chunks,
-                                                                       const GramRange *__restrict__ range,
+// Entry e of the packed lower triangle of ΦᵀΦ (i, j <= i), then of Φᵀy (i).
+struct GramEntry {
+    int i, j;
+    bool live, right;
+};
+__device__ __forceinline__ GramEntry gram_entry(int nf, bool has_rhs) {
+    const int e = blockIdx.x * 32 + threadIdx.x, n_gram = tri(nf);
+    GramEntry r{0, 0, e < n_gram + (has_rhs ? nf : 0), e >= n_gram};
+    if (!r.live) return r;
+    if (r.right) {
+        r.i = e - n_gram;
+        return r;
+    }
+    r.i = static_cast<int>((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
+    while (tri(r.i) > e) --r.i;
+    while (tri(r.i + 1) <= e) ++r.i;
+    r.j = e - tri(r.i);
+    return r;
+}
+__device__ __forceinline__ void gram_store(const GramEntry &e, int nf, double v, double *gram, double *rhs) {
+    if (e.right) {
+        rhs[e.i] = v;
+    } else {
+        gram[static_cast<int64_t>(e.i) * nf + e.j] = v;
+        gram[static_cast<int64_t>(e.j) * nf + e.i] = v;
+    }
+}
+
+// Which row and feature of the MMA an entry is, the chunks' sums (eight threads
+// per entry), its scale, and whether it is too small beside that.
+__global__ void __launch_bounds__(32 * kSumSplit) sg_gram_final_kernel(int ng, int nf, int chunks, double small,
+                                                                       GramRange *__restrict__ range,
                                                                        const longlong2 *__restrict__ part,
-                                                                       const double *__restrict__ part_g,
-                                                                       const double *__restrict__ part_r, int nparts,
                                                                        double *__restrict__ gram,
                                                                        double *__restrict__ rhs) {
-    __shared__ double sp[kSumSplit][32];
     __shared__ long long sh[kSumSplit][32], sl[kSumSplit][32];
-    const int e = blockIdx.x * 32 + threadIdx.x, y = threadIdx.y;
-    const int n_gram = tri(nf), total = n_gram + (rhs ? nf : 0);
-    const bool live = e < total;
-    int i = 0, j = 0;  // entry (i, j <= i), or the right side's i
-    if (live && e < n_gram) {
-        i = static_cast<int>((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
-        while (tri(i) > e) --i;
-        while (tri(i + 1) <= e) ++i;
-        j = e - tri(i);
-    } else if (live) {
-        i = e - n_gram;
+    if (!gram_finite(range, ng)) return;
+    const int y = threadIdx.y;
+    const GramEntry en = gram_entry(nf, rhs != nullptr);
+    int row = 0, col = 0, ex = 0;
+    bool zero = false;  // a factor that is zero throughout: the sum is exact
+    if (en.live) {
+        auto expo = [&](int x) {
+            if (x == 16) return 0;
+            const uint32_t m = range->gmax[x < 16 ? x : x - 1];
+            zero = zero || m == 0;
+            return range_exp(m);
+        };
+        auto feature = [ng](int u, int w) {  // of two variables of the 17
+            const int hi2 = u > w ? u : w, lo2 = u > w ? w : u;
+            return hi2 < 16 ? 1 + ng + tri(hi2) + lo2 : lo2 < 16 ? 1 + lo2 : 0;
+        };
+        int a, b;
+        gram_feature_vars(en.i, ng, a, b);
+        ex = expo(a) + expo(b);
+        if (en.right) {
+            row = kPairRows + ng - 16;
+            col = en.i;
+            ex += range_exp64(range->ymax);
+            zero = zero || range->ymax == 0;
+        } else {
+            int c, d;
+            gram_feature_vars(en.j, ng, c, d);
+            ex += expo(c) + expo(d);
+            auto same = [](int u, int w) { return var_part(u) == var_part(w); };
+            if (a > 16 || b > 16) row = kPairRows + (a > 16 ? a : b) - 17, col = en.j;
+            else if (c > 16 || d > 16) row = kPairRows + (c > 16 ? c : d) - 17, col = en.i;
+            else if (same(a, b)) row = pair_row(a, b), col = en.j;
+            else if (same(c, d)) row = pair_row(c, d), col = en.i;
+            else if (same(a, c)) row = pair_row(a, c), col = feature(b, d);
+            else if (same(a, d)) row = pair_row(a, d), col = feature(b, c);
+            else if (same(b, c)) row = pair_row(b, c), col = feature(a, d);
+            else row = pair_row(b, d), col = feature(a, c);
+        }
     }
-    const bool right = e >= n_gram;
-    double v;
-    if (!gram_finite(range, ng)) {
-        const int bi = i / kGramBlk, bj = j / kGramBlk;
-        const int64_t npairs = gram_pairs(nf);
-        const double *src = right ? part_r + i
-                                  : part_g + (tri(bi) + bj) * (kGramBlk * kGramBlk) + (i % kGramBlk) * kGramBlk + j % kGramBlk;
-        v = sum_parts(src, nparts, right ? kFeatCap : npairs * kGramBlk * kGramBlk, live, sp);
-    } else {
-        int row = 0, col = 0, ex = 0;
-        if (live) {
-            auto expo = [&](int x) { return x == 16 ? 0 : range_exp(range->gmax[x < 16 ? x : x - 1]); };
-            auto feature = [ng](int u, int w) {  // of two variables of the 17
-                const int hi2 = u > w ? u : w, lo2 = u > w ? w : u;
-                return hi2 < 16 ? 1 + ng + tri(hi2) + lo2 : lo2 < 16 ? 1 + lo2 : 0;
-            };
-            int a, b;
-            gram_feature_vars(i, ng, a, b);
-            ex = expo(a) + expo(b);
-            if (right) {
-                row = kPairRows + ng - 16;
-                col = i;
-                ex += range_exp64(range->ymax);
-            } else {
-                int c, d;
-                gram_feature_vars(j, ng, c, d);
-                ex += expo(c) + expo(d);
-                auto same = [](int u, int w) { return var_part(u) == var_part(w); };
-                if (a > 16 || b > 16) row = kPairRows + (a > 16 ? a : b) - 17, col = j;
-                else if (c > 16 || d > 16) row = kPairRows + (c > 16 ? c : d) - 17, col = i;
-                else if (same(a, b)) row = pair_row(a, b), col = j;
-                else if (same(c, d)) row = pair_row(c, d), col = i;
-                else if (same(a, c)) row = pair_row(a, c), col = feature(b, d);
-                else if (same(a, d)) row = pair_row(a, d), col = feature(b, c);
-                else if (same(b, c)) row = pair_row(b, c), col = feature(a, d);
-                else row = pair_row(b, d), col = feature(a, c);
-            }
-        }
-        long long h = 0, l = 0;
-        if (live) {
-            const longlong2 *src = part + (static_cast<int64_t>(col / kGmN) * kGmOutRows + row) * kGmN + col % kGmN;
+    long long h = 0, l = 0, m = 0;  // m: the |y| row's high part
+    if (en.live) {
+        const longlong2 *src = part + (static_cast<int64_t>(col / kGmN) * kGmOutRows + row) * kGmN + col % kGmN;
+        const int64_t step = static_cast<int64_t>(kGmBlocks) * kGmOutRows * kGmN;
 #pragma unroll 4
-            for (int q = y; q < chunks; q += kSumSplit) {
-                const longlong2 x = src[static_cast<int64_t>(q) * kGmBlocks * kGmOutRows * kGmN];
-                h += x.x;
-                l += x.y;
-            }
+        for (int q = y; q < chunks; q += kSumSplit) {
+            const longlong2 x = src[q * step];
+            h += x.x;
+            l += x.y;
         }
-        sh[y][threadIdx.x] = h;
-        sl[y][threadIdx.x] = l;
-        __syncthreads();
-        if (y != 0) return;
+        if (en.right)
+            for (int q = y; q < chunks; q += kSumSplit) m += src[q * step + kGmN].x;
+    }
+    sh[y][threadIdx.x] = h;
+    sl[y][threadIdx.x] = l;
+    __syncthreads();
+    if (y == 0) {
 #pragma unroll
         for (int q = 1; q < kSumSplit; ++q) {
             h += sh[q][threadIdx.x];
             l += sl[q][threadIdx.x];
         }
-        // a scaled feature is Σ_i d_i 2^(-7-8i): the sum is Σ_s v_s 2^(-14-8s)
-        v = scalbn(static_cast<double>(h) + scalbn(static_cast<double>(l), -32), ex - 32 + 2);
-        if (range->err) v = __longlong_as_double(0x7ff8000000000000ll);  // a wait gave up: no result
     }
-    if (!live || y != 0) return;
-    if (right) {
-        rhs[i] = v;
-    } else {
-        gram[static_cast<int64_t>(i) * nf + j] = v;
-        gram[static_cast<int64_t>(j) * nf + i] = v;
-    }
+    __syncthreads();
+    sh[y][threadIdx.x] = m;
+    __syncthreads();
+    if (!en.live || y != 0) return;
+#pragma unroll
+    for (int q = 1; q < kSumSplit; ++q) m += sh[q][threadIdx.x];
+    // a scaled feature is Σ_i d_i 2^(-7-8i): the sum is Σ_s v_s 2^(-14-8s)
+    const double f = (static_cast<double>(h) + scalbn(static_cast<double>(l), -32)) * 0x1p-30;  // in scales
+    const double mag = en.right ? static_cast<double>(m) * 0x1p-30 : f;
+    if (!zero && fabs(mag) < small) range->small = 1u;
+    double v = scalbn(f, ex);
+    if (range->err) v = __longlong_as_double(0x7ff8000000000000ll);  // a wait gave up: no result
+    gram_store(en, nf, v, gram, rhs);
+}
+
+// The same from the FP64 kernel's parts, where the fixed-point sums don't stand.
+__global__ void __launch_bounds__(32 * kSumSplit) sg_gram_fp64_final_kernel(int ng, int nf,
+                                                                            const GramRange *__restrict__ range,
+                                                                            const double *__restrict__ part_g,
+                                                                            const double *__restrict__ part_r,
+                                                                            int nparts, double *__restrict__ gram,
+                                                                            double *__restrict__ rhs) {
+    __shared__ double sp[kSumSplit][32];
+    if (gram_fixed(range, ng)) return;
+    const GramEntry en = gram_entry(nf, rhs != nullptr);
+    const int bi = en.i / kGramBlk, bj = en.j / kGramBlk;
+    const double *src = en.right ? part_r + en.i
+                                 : part_g + (tri(bi) + bj) * (kGramBlk * kGramBlk) + (en.i % kGramBlk) * kGramBlk +
+                                       en.j % kGramBlk;
+    const int64_t npairs = gram_pairs(nf);
+    const double v = sum_parts(src, nparts, en.right ? kFeatCap : npairs * kGramBlk * kGramBlk, en.live, sp);
+    if (en.live && threadIdx.y == 0) gram_store(en, nf, v, gram, rhs);
 }
 
 }  // namespace

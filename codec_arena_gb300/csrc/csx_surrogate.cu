@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 
@@ -375,10 +376,10 @@ __global__ void __launch_bounds__(32 * kSumSplit) sg_sum_parts_kernel(const doub
 }
 
 struct GramRange;
-__device__ __forceinline__ bool gram_finite(const GramRange *r, int ng);
+__device__ __forceinline__ bool gram_fixed(const GramRange *r, int ng);
 
-// Normal equations in FP64 (the full surface, and tables with a non-finite
-// entry; csx_gram.cuh otherwise): thread t of CTA column y owns the 4×4 block number
+// Normal equations in FP64 (the full surface, and the tables that csx_gram.cuh
+// leaves): thread t of CTA column y owns the 4×4 block number
 // y·1024 + t, (bi, bj) with bj <= bi, of ΦᵀΦ; CTA row x accumulates rows of
 // its chunk. Column 0's threads t < nf also accumulate (Φᵀy)_t. Φ for
 // kGramRows rows is staged in shared memory in FP64 (exact: a product of two
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(kGramThreads) sg_gram_kernel(int ng, int nf, c
                                                                double *__restrict__ part_g,
                                                                double *__restrict__ part_r,
                                                                const GramRange *__restrict__ range) {
-    if (range && gram_finite(range, ng)) return;  // sg_gram_mma_kernel's table
+    if (range && gram_fixed(range, ng)) return;  // sg_gram_mma_kernel's table
     extern __shared__ double phi[];  // [kGramRows][featpad]
     __shared__ float gs[kGramRows][kMaxLin + 1];
     __shared__ double ys[kGramRows];
@@ -1014,17 +1015,21 @@ int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, co
         SG_CUDA(cudaGetLastError());
         const int64_t drain = kGmRows * kGmDrain;
         const int chunks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(kGmChunks, (n + drain - 1) / drain)));
-        const bool stack = kPairRows + ng - 16 + 1 <= 64;
+        const bool stack = kPairRows + ng - 16 + 2 <= 64;
         (stack ? sg_gram_mma_kernel<true> : sg_gram_mma_kernel<false>)<<<dim3(chunks, kGmBlocks), kGmThreads, kGmSmem, s>>>(
             ng, nf, d_genes, n, ldg, d_fit, range, part);
         SG_CUDA(cudaGetLastError());
+        const int total = tri(nf) + (d_fit ? nf : 0);
+        double *rhs = d_fit ? d_rhs : nullptr;
+        sg_gram_final_kernel<<<(total + 31) / 32, dim3(32, kSumSplit), 0, s>>>(
+            ng, nf, chunks, kGmSmall * std::sqrt(static_cast<double>(n)), range, part, d_gram, rhs);
+        SG_CUDA(cudaGetLastError());
+        // these two leave at once where the fixed-point sums stand
         sg_gram_kernel<<<dim3(grid, ycols), threads, gram_smem(nf), s>>>(ng, nf, d_genes, n, ldg, d_fit, part_g, part_r,
                                                                         range);
         SG_CUDA(cudaGetLastError());
-        const int total = tri(nf) + (d_fit ? nf : 0);
-        sg_gram_final_kernel<<<(total + 31) / 32, dim3(32, kSumSplit), 0, s>>>(ng, nf, chunks, range, part, part_g,
-                                                                              part_r, grid, d_gram,
-                                                                              d_fit ? d_rhs : nullptr);
+        sg_gram_fp64_final_kernel<<<(total + 31) / 32, dim3(32, kSumSplit), 0, s>>>(ng, nf, range, part_g, part_r, grid,
+                                                                                   d_gram, rhs);
         SG_CUDA(cudaGetLastError());
         return CSX_OK;
     }

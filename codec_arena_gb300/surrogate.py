@@ -120,7 +120,9 @@ def score_f64(genes: torch.Tensor, coef: torch.Tensor) -> torch.Tensor:
 
 
 def normal_equations(genes: torch.Tensor, fit: Optional[torch.Tensor], nf: int):
-    """(ΦᵀΦ, Φᵀy) in FP64 on the GPU (fixed summation order)."""
+    """(ΦᵀΦ, Φᵀy) on the GPU, FP64: summed in fixed point on the tensor cores
+    where every entry's magnitude keeps that as close as FP64 sums, else in FP64
+    (fixed summation order)."""
     genes = _genes(genes)
     _ng(nf)
     dev = genes.device

@@ -70,7 +70,11 @@ int csx_sg_backward_coef_f64(int nf, const float *d_genes, int64_t n, int ldg, c
                              double *d_dcoef, void *d_work, void *stream);
 
 /* Normal equations of the ridge refit, FP64: d_gram (nf×nf, row-major, full
-   symmetric) = ΦᵀΦ, d_rhs (nf) = Φᵀy. d_fit may be NULL (rhs not written). */
+   symmetric) = ΦᵀΦ, d_rhs (nf) = Φᵀy. d_fit may be NULL (rhs not written).
+   nf <= 166: summed in fixed point on the tensor cores where every entry's
+   magnitude Σ|φ φ'| is at least sqrt(n) / 8 of the product of its variables'
+   largest values (and no entry of the table is infinite or NaN), by FP64 sums
+   otherwise: decided on the device. */
 int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, const double *d_fit,
                             double *d_gram, double *d_rhs, void *d_work, void *stream);
 

@@ -104,3 +104,70 @@ def test_workspace_at_any_double(off, ng):
                                                   torch.cuda.current_stream().cuda_stream))
     assert torch.equal(gram, want) and torch.equal(rhs, wrhs)
     assert (buf[:off] == 0x5a).all() and (buf[off + size:] == 0x5a).all()
+
+
+def _table(kind, n, ng, rng):
+    import os
+
+    from codec_arena_gb300 import genome, workloads as wl
+
+    g = rng.random((n, ng), dtype=np.float32)
+    if kind.startswith("pop"):
+        pop = genome.load_elites(os.path.join(wl.GOLDEN_DIR, "pop_seed_96.txt"), v6_fix=True)["g"]
+        p = np.clip(pop[rng.integers(0, len(pop), n), :ng] + 0.24 * (rng.random((n, ng)) - 0.5), 0, 1)
+        g = np.where(rng.random((n, 1)) < 0.05, g, p)
+    y = _phi(g.astype(np.float64), ng) @ rng.normal(0, 1, 1 + ng + 136) + 0.5 * rng.standard_t(3, n)
+    if kind.startswith("apart"):  # two genes (of two parts, of one, a linear-only one) never large together
+        small = np.float32(float(kind.split()[1]))
+        k = rng.random(n) < 0.5
+        for a, b in ((3, 9), (4, 5), (2, ng - 1)):
+            g[:, a] = np.where(k, g[:, a], g[:, a] * small)
+            g[:, b] = np.where(k, g[:, b] * small, g[:, b])
+    if kind == "rare":            # one row carries a column's largest value and the targets'
+        g[1:, 7] *= np.float32(1e-7)
+        y[0] = 1e9
+        g[0, 11] = np.float32(1e-8)
+    if kind == "disjoint":        # genes that are never nonzero together
+        k = rng.random(n) < 0.5
+        g[:, 3] = np.where(k, g[:, 3], 0)
+        g[:, 9] = np.where(k, 0, g[:, 9])
+    if kind == "zero":
+        g[:, 3] = 0
+        y = np.zeros(n)
+    if kind.endswith("4 decimals"):
+        g = np.round(g, 4)
+    return np.ascontiguousarray(g, np.float32), y
+
+
+@pytest.mark.parametrize("ng", [16, 22, 29])
+@pytest.mark.parametrize("n", [1, 33, 1500])
+@pytest.mark.parametrize("kind", ["uniform", "uniform 4 decimals", "pop 4 decimals", "apart 1e-2", "apart 1e-4",
+                                  "apart 1e-6", "apart 1e-9", "apart 1e-30", "rare", "disjoint", "zero"])
+def test_normal_equations_entry_by_entry(kind, n, ng):
+    """Each entry against its own magnitude sum_r |phi_i phi_j|, whatever the
+    columns' largest values. FP64 sums are within 2^-53 of it per rounding: the
+    rows of a part (32 at a time dealt to 152), 19 parts per thread, 8 threads, the
+    product. Fixed-point sums are taken only where the magnitude is at least
+    sqrt(n) / 8 of the scale, of which a row is within 8.1 x 2^-56: 8.1 sqrt(n) x
+    2^-53 of the magnitude, and two roundings at the end."""
+    _entry_by_entry(kind, n, ng)
+
+
+@pytest.mark.parametrize("ng", [16, 29])
+@pytest.mark.parametrize("n", [31, 32, 127, 128, 129, 255, 257, 6400, 6401, 9001])
+def test_fixed_point_entries_at_stage_edges(n, ng):
+    """The same where the rows end around a stage, a drain and a chunk."""
+    _entry_by_entry("uniform", n, ng)
+
+
+def _entry_by_entry(kind, n, ng):
+    g, y = _table(kind, n, ng, np.random.default_rng(n + ng))
+    gram, rhs = _run(g, y, 1 + ng + 136)
+    phi = _phi(g.astype(np.longdouble), ng)
+    yl = y.astype(np.longdouble)
+    mag, mrhs = np.abs(phi).T @ np.abs(phi), np.abs(phi).T @ np.abs(yl)
+    want, wrhs = (mag, phi.T @ yl) if g.min() >= 0 else (phi.T @ phi, phi.T @ yl)
+    rows = 32 * -(-(-(-n // 32)) // 152)
+    tol = (max(8.1 * np.sqrt(n), rows + 28) + 2) * 2.0 ** -53
+    assert np.all(np.abs(gram - want) <= tol * mag)
+    assert np.all(np.abs(rhs - wrhs) <= tol * mrhs)
