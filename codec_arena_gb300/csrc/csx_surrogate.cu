@@ -502,10 +502,21 @@ __host__ __device__ constexpr int solve_rows(int n, int r) {  // rows r, r + 8, 
 }
 // Doubles before local row q (global row r + 8 q, r + 8 q + 1 long).
 __host__ __device__ constexpr int solve_off(int r, int q) { return q * (r + 1) + kSolveCtas * (q * (q - 1) / 2); }
-constexpr size_t solve_smem(int n) {  // the largest CTA's rows, two column buffers, L's columns, the copy for n <= 166
+constexpr size_t solve_smem(int n) {  // the largest CTA's rows, two column buffers, L's columns, the scales, the copy for n <= 166
     return (static_cast<size_t>(solve_off(kSolveCtas - 1, solve_rows(n, 0))) + 2ull * (n + 1) * kSolveNb +
-            static_cast<size_t>(n + 1) * kSolveNb + 3ull * (kFullFeat + 1) + 2 + (n <= kMaxFeat ? static_cast<size_t>(tri(n)) : 0u)) *
+            static_cast<size_t>(n + 1) * kSolveNb + 4ull * (kFullFeat + 1) + 2 + (n <= kMaxFeat ? static_cast<size_t>(tri(n)) : 0u)) *
            sizeof(double);
+}
+
+// The power of two that brings a diagonal entry d into [1, 4) when it
+// multiplies its row and its column. Rows and columns scaled by powers of two
+// leave every rounding as it is, and no product of two entries of a panel can
+// overflow or vanish (unscaled, u_ak u_bk of a matrix of 1e-170 was 0).
+__device__ __forceinline__ double solve_scale(double d) {
+    const int64_t bits = __double_as_longlong(d);
+    const int64_t e = bits >> 52;  // sign and biased exponent
+    if (e < 0 || e == 2047 || bits == 0) return 1.0;  // not positive definite: reported below
+    return __longlong_as_double((1023 - ((e - 1023) >> 1)) << 52);
 }
 
 // 1 / d for a pivot: a float reciprocal of the significand's leading bits and
@@ -531,9 +542,11 @@ __device__ __forceinline__ double pivot_rcp(double d) {
 // Lᵀ w = z by one CTA, 32 unknowns at a time from the last: within a block one
 // warp takes an unknown per step, one FMA for all 32 lanes; then every warp
 // takes the block's unknowns off the ones before it, a warp per 32 of them and
-// half of the block. `row(i)` is L's row i; y has n entries in shared memory.
+// half of the block. `row(i)` is L's row i; y and the scales sc have n entries in
+// shared memory.
 template <class RowFn>
-__device__ void back_substitute(int n, double *y, double (*half)[kFullFeat + 1], RowFn row, double *__restrict__ w) {
+__device__ void back_substitute(int n, double *y, double (*half)[kFullFeat + 1], const double *sc, RowFn row,
+                                double *__restrict__ w) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i0 = (n - 1) & ~31; i0 >= 0; i0 -= 32) {
         const int cnt = min(32, n - i0);
@@ -548,7 +561,7 @@ __device__ void back_substitute(int n, double *y, double (*half)[kFullFeat + 1],
             }
             if (lane < cnt) {
                 y[i0 + lane] = z;
-                w[i0 + lane] = z;
+                w[i0 + lane] = z * sc[i0 + lane];
             }
         }
         __syncthreads();
@@ -581,14 +594,17 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
     double *Lc = P + 2 * (n + 1) * kSolveNb;                     // the step's columns of L, all rows
     double *zs = Lc + (n + 1) * kSolveNb;                        // the last solve's unknowns
     auto *half = reinterpret_cast<double(*)[kFullFeat + 1]>(zs + kFullFeat + 1);
-    double *Lfull = zs + 3 * (kFullFeat + 1);                    // n <= 166: L in one CTA for the last solve
+    double *sc = zs + 3 * (kFullFeat + 1);                       // the rows' scales
+    double *Lfull = zs + 4 * (kFullFeat + 1);                    // n <= 166: L in one CTA for the last solve
+    for (int j = tid; j < n; j += kSolveThreads) sc[j] = solve_scale(gram[static_cast<int64_t>(j) * n + j] + alpha);
+    __syncthreads();
     for (int q = warp; q < nrows; q += kSolveThreads / 32) {
         const int i = r + kSolveCtas * q;
         double *row = A + solve_off(r, q);
         for (int j = lane; j <= i; j += 32) {
             double v;
-            if (i < n) v = gram[static_cast<int64_t>(i) * n + j] + (i == j ? alpha : 0.0);
-            else v = j < n ? rhs[j] + (prior ? alpha * prior[j] : 0.0) : 0.0;
+            if (i < n) v = (gram[static_cast<int64_t>(i) * n + j] + (i == j ? alpha : 0.0)) * sc[i] * sc[j];
+            else v = j < n ? (rhs[j] + (prior ? alpha * prior[j] : 0.0)) * sc[j] : 0.0;
             row[j] = v;
         }
     }
@@ -677,11 +693,11 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
                 for (int j = lane; j < i; j += 32) Lfull[tri(i) + j] = src[j];
             }
             __syncthreads();
-            back_substitute(n, zs, half, [&](int i) { return Lfull + tri(i); }, w);
+            back_substitute(n, zs, half, sc, [&](int i) { return Lfull + tri(i); }, w);
         } else {
             __syncthreads();
             back_substitute(
-                n, zs, half,
+                n, zs, half, sc,
                 [&](int i) {
                     return cluster.map_shared_rank(A, i % kSolveCtas) + solve_off(i % kSolveCtas, i / kSolveCtas);
                 },

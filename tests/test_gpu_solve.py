@@ -67,3 +67,23 @@ def test_solves_in_a_row(n):
     assert not status.any()
     for i, (a, b, _) in enumerate(sys):
         _close(out[i].cpu().numpy(), a, b, n)
+
+
+@pytest.mark.parametrize("n", [1, 4, 33, 153, 166, 465])
+@pytest.mark.parametrize("lo,hi", [(-500, -500), (500, 500), (-480, 480), (-535, -530)])
+def test_rows_of_any_exponent(n, lo, hi):
+    """Rows and columns multiplied by powers of two: the unscaled system's bits,
+    scaled back (down to a diagonal of subnormals, where the matrix is diagonal)."""
+    import torch
+
+    from codec_arena_gb300 import surrogate
+
+    a, b, _ = _system(n, n + 1)
+    if lo < -500:
+        a = np.diag(2.0 ** np.random.default_rng(n).integers(0, 20, n))
+    s = np.random.default_rng(n).integers(lo, hi + 1, n)
+    scaled = np.ldexp(np.ldexp(a, s[:, None]), s[None, :])
+    w0 = surrogate.ridge_solve(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), 0.0).cpu().numpy()
+    w = surrogate.ridge_solve(torch.from_numpy(scaled).cuda(), torch.from_numpy(np.ldexp(b, s)).cuda(), 0.0)
+    assert np.isfinite(w0).all()
+    np.testing.assert_array_equal(w.cpu().numpy(), np.ldexp(w0, -s))
