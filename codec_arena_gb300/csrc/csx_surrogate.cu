@@ -685,6 +685,8 @@ __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThrea
     }
     cluster.sync();  // every row of L is final
     if (r == 0) {
+        if (__syncthreads_or(bad))  // no weights from a factorisation that failed
+            for (int j = tid; j < n; j += kSolveThreads) sc[j] = __longlong_as_double(0x7ff8000000000000ll);
         const double *zrow = cluster.map_shared_rank(A, n % kSolveCtas) + solve_off(n % kSolveCtas, n / kSolveCtas);
         for (int j = tid; j < n; j += kSolveThreads) zs[j] = zrow[j];
         if (n <= kMaxFeat) {  // L into this CTA, then the solve on local rows

@@ -78,10 +78,9 @@ int csx_sg_backward_coef_f64(int nf, const float *d_genes, int64_t n, int ldg, c
 int csx_sg_normal_equations(int nf, const float *d_genes, int64_t n, int ldg, const double *d_fit,
                             double *d_gram, double *d_rhs, void *d_work, void *stream);
 
-/* Ridge solve in FP64 (LDL' on a cluster; Cholesky on one CTA for 465): w = (G + αI)⁻¹ (rhs + α·prior).
+/* Ridge solve in FP64 (LDL' on a cluster of eight CTAs): w = (G + αI)⁻¹ (rhs + α·prior).
    d_prior may be NULL (zero prior). d_status (one int) receives 0, or k+1
-   when the k-th pivot is not positive. nf <= 166, or 465 (the factor then
-   lives in a scratch allocated and freed on `stream`). */
+   when the k-th pivot is not positive (d_w is NaN then). nf <= 166, or 465. */
 int csx_sg_ridge_solve(int nf, const double *d_gram, const double *d_rhs, double alpha, const double *d_prior,
                        double *d_w, int *d_status, void *stream);
 

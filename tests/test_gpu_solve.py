@@ -87,3 +87,21 @@ def test_rows_of_any_exponent(n, lo, hi):
     w = surrogate.ridge_solve(torch.from_numpy(scaled).cuda(), torch.from_numpy(np.ldexp(b, s)).cuda(), 0.0)
     assert np.isfinite(w0).all()
     np.testing.assert_array_equal(w.cpu().numpy(), np.ldexp(w0, -s))
+
+
+@pytest.mark.parametrize("n", [1, 9, 166, 465])
+@pytest.mark.parametrize("pivot", [0.0, -1.0, float("nan")])
+def test_a_failed_factorisation_leaves_no_weights(n, pivot):
+    import torch
+
+    from codec_arena_gb300 import _lib
+
+    k = n // 2
+    a = np.eye(n)
+    a[k, k] = pivot
+    g, b = torch.from_numpy(a).cuda(), torch.ones(n, dtype=torch.float64, device="cuda")
+    w = torch.zeros(n, dtype=torch.float64, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().csx_sg_ridge_solve(n, g.data_ptr(), b.data_ptr(), 0.0, None, w.data_ptr(),
+                                             status.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert status.item() == k + 1 and w.isnan().all()
