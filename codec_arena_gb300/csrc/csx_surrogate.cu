@@ -583,7 +583,7 @@ __device__ void back_substitute(int n, double *y, double (*half)[kFullFeat + 1],
 __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(kSolveThreads)
     sg_ridge_solve_kernel(int n, const double *__restrict__ gram, const double *__restrict__ rhs, double alpha,
                           const double *__restrict__ prior, double *__restrict__ w, int *status) {
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];  // the panels are written as double2
     __shared__ double s_l[kSolveNb][kSolveNb], s_r[kSolveNb];
     cg::cluster_group cluster = cg::this_cluster();
     const int r = static_cast<int>(cluster.block_rank());
