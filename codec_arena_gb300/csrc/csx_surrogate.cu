@@ -521,9 +521,9 @@ __device__ __forceinline__ double solve_scale(double d) {
 
 // 1 / d for a pivot: a float reciprocal of the significand's leading bits and
 // two Newton steps x += x (1 - m x), then the exponent: four dependent FP64
-// operations of 64 cycles each, where the division takes 565 cycles. Within an
-// ulp or two of 1 / d for the exponents a normal equation's pivot can have; the
-// division otherwise (zero, negative, subnormal, infinite, NaN, or a reciprocal
+// operations of 64 cycles each, where the division takes 565 cycles. Within
+// 2^-52 of 1 / d (the two steps square the seed's 2^-22 twice, which leaves the
+// last one's rounding); the division otherwise (zero, negative, subnormal, infinite, NaN, or a reciprocal
 // near underflow). The float parts are read off and put back by integer
 // operations: the conversions run on the FP64 pipe too.
 __device__ __forceinline__ double pivot_rcp(double d) {

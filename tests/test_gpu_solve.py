@@ -105,3 +105,22 @@ def test_a_failed_factorisation_leaves_no_weights(n, pivot):
     _lib.check(_lib.lib().csx_sg_ridge_solve(n, g.data_ptr(), b.data_ptr(), 0.0, None, w.data_ptr(),
                                              status.data_ptr(), torch.cuda.current_stream().cuda_stream))
     assert status.item() == k + 1 and w.isnan().all()
+
+
+def test_pivot_reciprocal():
+    """1 / d of a diagonal matrix's pivots, over significands (ones next to powers
+    of two among them) and exponents. Two Newton steps square the seed's 2^-22
+    twice, so the last step's rounding is what is left: at most one unit of 2^-52
+    of the result (a half, and room for the residual's)."""
+    import torch
+
+    from codec_arena_gb300 import surrogate
+
+    rng = np.random.default_rng(1)
+    for rep in range(40):
+        m = 1.0 + rng.random(465)
+        m[:8] = [1.0, 1 + 2.0 ** -52, 2 - 2.0 ** -52, 1 + 2.0 ** -23, 2 - 2.0 ** -23, 1.5, 4 / 3, 1 + 2.0 ** -29]
+        d = np.ldexp(m, rng.integers(-1021, 1022, 465))
+        w = surrogate.ridge_solve(torch.from_numpy(np.diag(d)).cuda(), torch.ones(465, dtype=torch.float64).cuda(), 0.0)
+        want = 1.0 / d
+        assert np.all(np.abs(w.cpu().numpy() - want) <= 2.0 ** -52 * want)
