@@ -750,9 +750,10 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
     cx.timed = (cfg.flags & CSX_FLAG_STAGE_TIMES) != 0;
     cx.info = csx_run_info{};
     cx.info.screen_ctas = static_cast<uint32_t>(pl.grid);
-    cx.info.segments = pl.short_path ? 0 : g.n_seg;
-    cx.info.seg_draws = pl.short_path ? 0 : g.L;
-    cx.info.item_cands = 1ull << g.d_log2;
+    const bool walked = !pl.short_path && !pl.dense;
+    cx.info.segments = walked ? g.n_seg : 0;
+    cx.info.seg_draws = walked ? g.L : 0;
+    cx.info.item_cands = pl.dense ? (1ull << pl.dg.b_log2) / 62 : 1ull << g.d_log2;  // a block's candidates
     uint32_t launches = 0;
     auto mark = [&](int i) -> cudaError_t { return cx.timed ? cudaEventRecord(cx.ev[i], st) : cudaSuccess; };
     CSX_CUDA(mark(0));

@@ -235,9 +235,10 @@ int csx_limits(uint64_t *max_keep, uint64_t *max_elites);
 typedef struct csx_run_info {
     uint32_t launches;      /* kernels the call enqueued */
     uint32_t screen_ctas;   /* persistent screen CTAs */
-    uint64_t segments;      /* walk segments (0 when streams fit one item) */
-    uint64_t seg_draws;     /* draws per walk segment */
-    uint64_t item_cands;    /* candidates per work item (D) */
+    uint64_t segments;      /* walk segments (0 when streams fit one item, or where small
+                               generations take their items from block maps) */
+    uint64_t seg_draws;     /* draws per walk segment (0 likewise) */
+    uint64_t item_cands;    /* candidates per work item (D; of a block of draws, 62 each) */
     uint64_t items;         /* work items the screen consumed */
     float ms_prep;          /* elite table */
     float ms_items;         /* walk, assemble, scan, emit */

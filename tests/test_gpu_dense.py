@@ -33,3 +33,25 @@ def test_dense_items_equal_the_walks(monkeypatch, lam, T, imm, jump):
     b, nb = screen.screen(cfg, m, el)
     assert na == nb == lam == sum(n for _, n in shards)
     assert a.tobytes() == b.tobytes()
+
+
+@pytest.mark.parametrize("lam,T,cands", [(2_000, 1000, 64), (200_000, 4, 8), (500_001, 4, 16), (8_000_000, 7, 16),
+                                         (8_000_001, 7, 64)])
+def test_run_info_describes_the_items(monkeypatch, lam, T, cands):
+    """Streams of one item, block maps of both sizes, and the walk past them."""
+    from codec_arena_gb300 import screen, workloads as wl
+
+    for name in ("CSX_SEG_CANDS", "CSX_ITEM_CANDS"):
+        monkeypatch.delenv(name, raising=False)
+    screen.screen(screen.Cfg(lam, 100, 11, threads=T), screen.Model.from_compact(wl.surrogate_161()),
+                  wl.seeded_elites(24, seed=3))
+    info = screen.last_run_info()
+    assert info["item_cands"] == cands
+    if lam <= 8_000_000:
+        assert info["segments"] == info["seg_draws"] == 0
+    else:
+        assert info["segments"] >= T and info["seg_draws"] > 0
+    if T > 500:
+        assert info["items"] == T
+    else:  # all but the streams' and the segments' ends hold that many
+        assert 0.95 * cands <= lam / info["items"] <= 1.1 * cands
