@@ -193,7 +193,7 @@ def ascend(genes: torch.Tensor, coef: torch.Tensor, eta: float, steps: int):
     sc = torch.empty(src.shape[0], dtype=torch.float32, device=src.device)
     # the kernel reads src and writes the copy, unless the clone has a place of
     # its own (in a graph, a dual number's) or src's rows overlap
-    if (type(src) is torch.Tensor and not src.requires_grad and _fwd._current_level < 0
+    if (type(src) is torch.Tensor and not src.requires_grad and _fwd.unpack_dual(src).tangent is None
             and src.stride(0) >= src.shape[1]):
         out = torch.empty_like(src)
         check(lib().csx_sg_ascend_to(coef.data_ptr(), nf, src.data_ptr(), src.shape[0], src.stride(0), src.shape[1],

@@ -66,3 +66,20 @@ def test_clones_with_a_place_of_their_own():
     one = rows[:1].expand(5, 29)                                # rows that overlap
     new, sc = surrogate.ascend(one, coef, 0.01, 3)
     assert torch.equal(new, want[:1].expand(5, 29)) and new.is_contiguous()
+
+
+def test_dual_numbers_keep_their_tangent():
+    import torch
+    import torch.autograd.forward_ad as fwd
+
+    from codec_arena_gb300 import surrogate
+
+    rows, t = torch.rand(40, 29, device="cuda"), torch.rand(40, 29, device="cuda")
+    coef = torch.randn(166, device="cuda")
+    want, ws = surrogate.ascend(rows, coef, 0.01, 3)
+    with fwd.dual_level():
+        new, sc = surrogate.ascend(fwd.make_dual(rows, t), coef, 0.01, 3)
+        primal, tangent = fwd.unpack_dual(new)
+        assert torch.equal(primal, want) and torch.equal(tangent, t) and torch.equal(sc, ws)
+        new, sc = surrogate.ascend(rows, coef, 0.01, 3)
+        assert torch.equal(new, want) and fwd.unpack_dual(new).tangent is None
