@@ -591,8 +591,7 @@ int batch_prepare(Context &cx, int n, const csx_cfg *cfgs, const csx_model *mode
             const IslandBufs &b = L->b[i];
             L->pargs[i] = prune_args(screen_args(cfgs[i], models[i], make_synth(cfgs[i], n_elites[i]), pl, b.tab,
                                                  b.items, b.ctrl, b.la),
-                                     models[i], pl, b.pairs, L->pub + static_cast<size_t>(kPruneMs) * nl * i,
-                                     cx.num_sms);
+                                     models[i], pl, b.pairs, L->pub + static_cast<size_t>(kPruneMs) * nl * i);
         }
     }
     return CSX_OK;

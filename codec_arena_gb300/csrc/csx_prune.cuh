@@ -78,7 +78,6 @@ struct PruneArgs : ScreenArgs {
     uint32_t k1;
     const float *tmax;    // ne x ne: the linear tail's largest value over a pair (null without a tail)
     uint32_t *pub;        // kPruneMs x gridDim.x: okey of each CTA's 1st / 2nd / 4th best entry
-    uint32_t sel_cap;     // entries of the selection scratch in shared memory (>= gridDim.x)
     uint32_t el_smem;     // 1: the elite table is copied to shared memory (prune_el_smem)
     uint32_t bm_words;    // words of the pair bitmap in shared memory (0: the pair table is read directly)
     uint32_t bm_period;   // rounds (outer) between its rebuilds, a power of two
@@ -527,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         }
     };
 
-    auto rescore = [&](const Pend &q, unsigned long long t1, unsigned long long t2, float ts) {
+    auto rescore = [&](const Pend &q, float ts) {
         const Item it = A.items[q.item];
         const float s = prune_rescore<kFp64>(&A, el, stream_seed(A.seed, it.stream), it.draw0 + q.ddraw,
                                              __fsub_rd(ts, A.err));
@@ -552,16 +551,11 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         // waits on it, or the work is done); a flush appends <= pn + 2 x 256 <= 1024
         if (pn >= kThreads || any_def || (!any && pn > 0)) {
             if (bn + kPendCap + 2 * kThreads > A.buf_cap) merge(bn);  // make room first
-            unsigned long long t1 = s_t1, t2 = s_t2;
             float ts = s_ts;
             const unsigned int g = *reinterpret_cast<volatile unsigned int *>(&A.ctrl->gtau);
-            if ((static_cast<unsigned long long>(g) << 32) > t1) {
-                t1 = static_cast<unsigned long long>(g) << 32;
-                t2 = 0;
-                ts = okey_score(g);
-            }
-            for (uint32_t i = tid; i < pn; i += kThreads) rescore(pend[i], t1, t2, ts);
-            for (uint32_t i = 0; i < n_def; ++i) rescore(i == 0 ? def[0] : def[1], t1, t2, ts);
+            if ((static_cast<unsigned long long>(g) << 32) > s_t1) ts = okey_score(g);
+            for (uint32_t i = tid; i < pn; i += kThreads) rescore(pend[i], ts);
+            for (uint32_t i = 0; i < n_def; ++i) rescore(i == 0 ? def[0] : def[1], ts);
             n_def = 0;
             __syncthreads();
             bn = s_buf_n;
@@ -837,7 +831,8 @@ inline bool prune_el_smem(uint32_t sort_n, int ne, int num_sms, size_t max_smem)
 
 // Masks the pair table enumerates per pair: 2^n_enum. One mask costs about 45
 // instructions against some 150 per candidate of the screen, so the table is
-// given one mask per eight candidates: 3-4% of the screen. All 16 genes at
+// given one mask per eight candidates (at least five genes' masks, whatever the
+// budget): 3-4% of the screen. All 16 genes at
 // 2.65e9 candidates and 64 elites (2080 pairs); fewer genes loosen the bound
 // (pairs left at the final threshold, committed surface: 8% with 16 genes
 // enumerated, 10% with 10, 11% with 8, 14% with 6).
@@ -849,7 +844,9 @@ inline int pair_enum(uint64_t lambda, int ne) {
 }
 
 // Genes of the mask table: the enumerated ones but four (a pair's group of
-// threads shares those), at most eight, fewer where the table would pass 64 MB.
+// threads shares those), at most eight, fewer where the table would pass 64 MB,
+// down to the five of a thread's Gray walk: 151 MB at the 1,536 elites that the
+// library takes at most.
 inline int pair_k1(int n_enum, int ne) {
     const uint64_t pairs = static_cast<uint64_t>(ne) * (ne + 1) / 2;
     int k = std::min(kMaxMaskGenes, std::max(kPairGray, n_enum - 4));

@@ -53,6 +53,7 @@
 #include <map>
 #include <mutex>
 #include <set>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/csx_screen.h"
@@ -691,8 +692,7 @@ int enqueue_pairs(const csx_model &m, const PruneConst &pc, int ne, bool tail, c
 }
 
 // The pruning screen's arguments past the plain screen's.
-PruneArgs prune_args(const ScreenArgs &A, const csx_model &m, const Plan &pl, const PairBufs &b, uint32_t *pub,
-                     int num_sms) {
+PruneArgs prune_args(const ScreenArgs &A, const csx_model &m, const Plan &pl, const PairBufs &b, uint32_t *pub) {
     PruneArgs P{};
     static_cast<ScreenArgs &>(P) = A;
     uint8_t perm[16];
@@ -705,7 +705,6 @@ PruneArgs prune_args(const ScreenArgs &A, const csx_model &m, const Plan &pl, co
     P.u0 = b.u0;
     P.tmax = b.tmax;
     P.pub = pub;
-    P.sel_cap = 3u * static_cast<uint32_t>(num_sms);
     P.el_smem = pl.el_smem ? 1u : 0u;
     P.bm_words = prune_bm_words(static_cast<int>(A.sc.ne));
     // a rebuild reads the whole table once per CTA: every 2 outer rounds for 64
@@ -803,7 +802,7 @@ int enqueue_screen(Context &cx, const csx_cfg &cfg, const csx_model &model, cons
 
     const ScreenArgs A = screen_args(cfg, model, sc, pl, tab, items, ctrl, static_cast<Entry *>(cx.lists_a.p));
     if (pl.prune) {
-        const PruneArgs P = prune_args(A, model, pl, pairs, static_cast<uint32_t *>(cx.pub.p), cx.num_sms);
+        const PruneArgs P = prune_args(A, model, pl, pairs, static_cast<uint32_t *>(cx.pub.p));
         screen_p_fn(pl.tail, pl.tc, prune_bx_smem(pl.sort_n, ne))<<<pl.grid, kThreads, pl.smem, st>>>(P);
     } else if (pl.tc) {
         TcScreenArgs P;
@@ -1108,7 +1107,7 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
             CSX_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));
             const uint32_t ts = static_cast<uint32_t>(t);
             if (!all && bufs.pairs.box && pl.prune_ok) {
-                tie_collect_pruned_kernel<<<blocks, 256, 0, st>>>(prune_args(A, model, pl, bufs.pairs, nullptr, cx.num_sms),
+                tie_collect_pruned_kernel<<<blocks, 256, 0, st>>>(prune_args(A, model, pl, bufs.pairs, nullptr),
                                                                   n_items, ts, lo, hi, thr, d_hits, d_count, cap);
             } else if (full) {
                 if (pl.fast_delta)

@@ -127,7 +127,7 @@ __device__ __noinline__ float exact_score_at(const ScreenArgs *__restrict__ A, c
 // FullScreenArgs, every candidate scored on the full surface.
 template <bool kFastDelta, class Args = ScreenArgs>
 __global__ void __launch_bounds__(kThreads, 3) screen_kernel(const __grid_constant__ Args A) {
-    constexpr bool kFull = sizeof(Args) == sizeof(FullScreenArgs);
+    constexpr bool kFull = std::is_same<Args, FullScreenArgs>::value;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Entry *E = reinterpret_cast<Entry *>(smem_raw);
     float *el = reinterpret_cast<float *>(E + A.sort_n);
