@@ -48,7 +48,7 @@
 
 namespace csx {
 
-constexpr int kPruneMs = 3;  // order statistics each CTA publishes: its 1st, 2nd and 4th best
+constexpr int kPruneMs = 3;  // order statistics each CTA publishes (publish_first)
 // Candidates per thread between the CTA's barriers, and outer rounds between
 // merges of a non-empty buffer.
 constexpr int kPruneRounds = 64;
@@ -77,7 +77,7 @@ struct PruneArgs : ScreenArgs {
     uint64_t goff[8];     // draw offset (x kGolden) of those genes' crossover bits
     uint32_t k1;
     const float *tmax;    // ne x ne: the linear tail's largest value over a pair (null without a tail)
-    uint32_t *pub;        // kPruneMs x gridDim.x: okey of each CTA's 1st / 2nd / 4th best entry
+    uint32_t *pub;        // kPruneMs x gridDim.x: okey of each CTA's m-th, 2m-th and 4m-th best entry
     uint32_t el_smem;     // 1: the elite table is copied to shared memory (prune_el_smem)
     uint32_t bm_words;    // words of the pair bitmap in shared memory (0: the pair table is read directly)
     uint32_t bm_period;   // rounds (outer) between its rebuilds, a power of two
@@ -121,6 +121,18 @@ __device__ __forceinline__ uint32_t warp_kth_largest(const uint32_t *v, uint32_t
     return prefix;
 }
 
+// The first of the list positions m, 2m, 4m that each CTA publishes: the
+// smallest power of two of which the grid's CTAs can cover K (1 up to one
+// survivor per CTA: the 1st, 2nd and 4th best; past four survivors per CTA m
+// alone). With the 1st, 2nd and 4th whatever K, lists past four survivors per
+// CTA had only a CTA's own threshold: 2,047 of 5e7 candidates scored 41% of them
+// in 4.4 ms instead of 5% in 1.2 (full surface: 97% in 7.1, 16% in 3.5).
+__device__ __forceinline__ uint32_t publish_first(uint32_t keep) {
+    uint32_t m = 1;
+    while (static_cast<uint64_t>(m) * gridDim.x < keep) m <<= 1;
+    return m;
+}
+
 template <class Args>
 __device__ __noinline__ void prune_merge(const Args *A, Entry *E, uint32_t *sel, uint32_t bn, unsigned int *s_buf_n,
                                          unsigned long long *s_t1, unsigned long long *s_t2, float *s_ts) {
@@ -137,16 +149,17 @@ __device__ __noinline__ void prune_merge(const Args *A, Entry *E, uint32_t *sel,
             atomicMax(&A->ctrl->gtau, ok);
         }
     }
-    if (tid < kPruneMs && (1u << tid) <= A->keep) {
-        const unsigned int ok = static_cast<unsigned int>(E[(1u << tid) - 1].k1 >> 32);
+    const uint32_t m0 = publish_first(A->keep);
+    if (tid < kPruneMs && (m0 << tid) <= A->keep) {
+        const unsigned int ok = static_cast<unsigned int>(E[(m0 << tid) - 1].k1 >> 32);
         if (ok != 0u) atomicMax(&A->pub[tid * gridDim.x + blockIdx.x], ok);
     }
     __syncthreads();
     if (tid < 32) {
         uint32_t best = 0;
         for (int mi = 0; mi < kPruneMs; ++mi) {
-            const uint32_t jm = (A->keep + (1u << mi) - 1) >> mi;
-            if ((1u << mi) > A->keep || jm > gridDim.x) continue;
+            const uint32_t m = m0 << mi, jm = (A->keep + m - 1) / m;
+            if (m > A->keep || (mi > 0 && m > 4)) continue;
             const volatile uint32_t *src = A->pub + mi * gridDim.x;
             for (uint32_t i = tid; i < gridDim.x; i += 32) sel[i] = src[i];
             __syncwarp();
@@ -436,7 +449,7 @@ __device__ __forceinline__ float prune_bound(const PruneArgs &A, const uint32_t 
 // is rebuilt as the threshold rises (a bit of an older threshold only passes
 // more).
 // Global threshold: besides the best CTA K-th score (Ctrl::gtau), every CTA
-// publishes the keys of its m-th best entry, m = 1, 2, 4. If ceil(K / m) CTAs
+// publishes the keys of its m-th best entry, for three m (publish_first). If ceil(K / m) CTAs
 // have published keys >= x, at least K distinct screened candidates score at
 // least x, so the generation's K-th score is >= x; each published key only
 // grows, so a stale read gives a lower, still valid, threshold. After each

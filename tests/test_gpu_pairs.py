@@ -132,3 +132,21 @@ def test_thresholds_that_settle_elsewhere(monkeypatch, ne):
             got, n = screen.screen(screen.Cfg(lam, keep, seed, threads=5), m, el)
             ref, _ = screen.screen(screen.Cfg(lam, keep, seed, threads=5, flags=_lib.FLAG_NO_PRUNE), m, el)
             assert n == lam and got.tobytes() == ref.tobytes(), (seed, lam)
+
+
+@pytest.mark.parametrize("keep,nf", [(700, 161), (2047, 161), (4096, 161), (2047, 465)])
+def test_long_lists_share_a_threshold(monkeypatch, keep, nf):
+    """Lists longer than four survivors per CTA: the published positions still
+    cover K, so that a small part of 5e7 candidates is scored in full (the
+    threshold of 4,096 of them lies 3.8 s.d. up, a CTA's own 4,096 of 330,000 2.2)."""
+    from codec_arena_gb300 import _lib, screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    m = (screen.ModelFull.from_compact(wl.seeded_normal_model(seed=3, n=465)) if nf == 465
+         else screen.Model.from_compact(wl.surrogate_161()))
+    el = wl.seeded_elites(64, seed=2)
+    got, n = screen.screen(screen.Cfg(50_000_000, keep, 3, threads=4, flags=_lib.FLAG_STAGE_TIMES), m, el)
+    evals = screen.last_run_info()["exact_evals"]
+    ref, _ = screen.screen(screen.Cfg(50_000_000, keep, 3, threads=4, flags=_lib.FLAG_NO_PRUNE), m, el)
+    assert n == 50_000_000 and got.tobytes() == ref.tobytes()
+    assert evals < 0.2 * n, evals / n
