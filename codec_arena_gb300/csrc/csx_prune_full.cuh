@@ -19,9 +19,16 @@
 // Qs yh is a 29 x 29 product per candidate, 841 FMAs: each 128-thread group
 // writes its candidates' yh as FP16 rows of a shared-memory tile and one thread
 // issues tcgen05.mma (M 128, N 32, K 32, FP32 accumulation); every thread reads
-// its own row back. Where the bound leaves more than half of the candidates (a
-// mutation as wide as the genes' range, a threshold not yet settled), a CTA
-// passes everything on for a while instead of paying for both.
+// its own row back. Where the bound leaves more than half of a round's candidates
+// (elites that are alike and near the top, as survivors screened again are; a
+// threshold not yet settled), a CTA scores the next ones without it and tries
+// again, after four such rounds in a row at growing distances. A round that tries
+// again takes a quarter of the candidates: its queue is full within two or three
+// per thread. 2.65e8 candidates whose elites are the survivors of a screen: 28.0
+// ms with every candidate queued and fetched back, 19.6 so (16.5 unpruned: the
+// coefficients come from shared memory here, and with them as constants in this
+// kernel its other rounds spill, 11.9 ms instead of 11.3 on uniform elites); 5e7:
+// 6.6 ms, 4.5 so, 3.5 unpruned.
 //
 // What bounds it is the instruction issue, 33 hashes first. 2.65e8 candidates
 // of 64 uniform elites, a seeded N(0, 0.1) surface, sigma 0.12, top 256: 16.5
@@ -76,10 +83,9 @@ constexpr int kFtCoef = ft_row(kNtot);
 // through the kernel's arguments each coefficient was a load of its own: a
 // screen that scored every candidate took 26.7 and 30.3 ms at 2.65e8 where the
 // unpruned kernel takes 16.5.
-__device__ __noinline__ float full_score_at(const SynthConst *__restrict__ C, float w0, uint32_t coef, const float *el,
-                                            uint64_t seed_t, uint64_t p) {
-    const CandHead h = cand_head(*C, seed_t, p);
-    GeneSource S = gene_source(*C, el, seed_t, p, h);
+__device__ __forceinline__ float full_score(const SynthConst &C, float w0, uint32_t coef, const float *el,
+                                            uint64_t seed_t, uint64_t p, const CandHead &h) {
+    GeneSource S = gene_source(C, el, seed_t, p, h);
     float G[kNtot];
     float R = w0;
 #pragma unroll
@@ -104,6 +110,60 @@ __device__ __noinline__ float full_score_at(const SynthConst *__restrict__ C, fl
         R = __fmaf_rn(g, t, R);
     }
     return R;
+}
+__device__ __noinline__ float full_score_at(const SynthConst *__restrict__ C, float w0, uint32_t coef, const float *el,
+                                            uint64_t seed_t, uint64_t p) {
+    const CandHead h = cand_head(*C, seed_t, p);
+    return full_score(*C, w0, coef, el, seed_t, p, h);
+}
+
+// A round without the bound, out of line: kFtRounds candidates of the thread's
+// items scored, the ones at the threshold ts or above to the CTA's queue.
+struct DirectRound {  // a thread's place among its items, and the candidate the full queue did not take
+    uint64_t st;
+    uint32_t item, left, n_it, screened, exact, n_def;
+    bool valid;
+    Pend def;
+};
+__device__ __noinline__ void full_direct(const FullPruneArgs *__restrict__ A, const float *el, uint32_t coef,
+                                         Pend *pend, unsigned int *s_pend_n, float ts, DirectRound *place) {
+    if (!place->valid) return;
+    const uint32_t n_items = A->ctrl->n_items;
+    DirectRound d = *place;
+    Item it = A->items[d.item];
+    uint64_t seed_t = stream_seed(A->seed, it.stream);
+    uint64_t p = (d.st - seed_t) * kGoldenInv - 1;
+#pragma unroll 1
+    for (int r = 0; r < kFtRounds && d.n_def == 0; ++r) {
+        const CandHead h = cand_head(A->sc, seed_t, p);
+        ++d.exact;
+        if (full_score(A->sc, A->fm.w0, coef, el, seed_t, p, h) >= ts) {
+            const Pend q{d.item, d.n_it - d.left, static_cast<uint32_t>(p - it.draw0)};
+            const unsigned int slot = atomicAdd(s_pend_n, 1u);
+            if (slot < kPendCap) {
+                pend[slot] = q;
+            } else {
+                d.def = q;
+                d.n_def = 1;
+            }
+        }
+        p += h.len;
+        if (--d.left == 0) {
+            d.item = gridDim.x * kThreads + atomicAdd(&A->ctrl->next_item, 1u);
+            d.n_it = 0;
+            d.valid = d.item < n_items;
+            if (!d.valid) break;
+            it = A->items[d.item];
+            seed_t = stream_seed(A->seed, it.stream);
+            p = it.draw0;
+            d.n_it = d.left = it.n;
+            d.screened += it.n;
+            d.valid = it.n > 0;
+            if (!d.valid) break;
+        }
+    }
+    d.st = seed_t + (p + 1) * kGolden;
+    *place = d;
 }
 
 // One round of a 128-thread group: row `row` of its tile <- pk (32 halfs), one
@@ -251,10 +311,10 @@ __global__ void __launch_bounds__(kThreads, 3) screen_ft_kernel(const __grid_con
         // a group whose tensor-core wait gave up ends the CTA's screening
         const int stop = (s_gbad[0] | s_gbad[1]) != 0u;
         // the bound left more than half of the last round: off for a round (the
-        // threshold has yet to settle), after the sixteenth time for ever longer
+        // threshold has yet to settle), after the fourth time in a row for ever longer
         if (s_passed * 2 > s_seen) {
             ++fails;
-            off_until = round + (fails <= 16 ? 1u : min(1u << (fails - 16), kFtProbe));
+            off_until = round + (fails <= 4 ? 1u : min(1u << (fails - 4), kFtProbe));
             fails = min(fails, 24u);
         } else if (s_seen > 0) {
             fails = 0;
@@ -295,9 +355,25 @@ __global__ void __launch_bounds__(kThreads, 3) screen_ft_kernel(const __grid_con
         const bool settled = __syncthreads_or(ts > -INFINITY) != 0;
         const bool on = settled && round >= off_until;
         ++round;
+        // tried again, a short round
+        const int r0 = on && fails > 1 ? kFtRounds - kFtRounds / 4 : 0;
+        if (!on && settled) {
+            DirectRound d{st, item, left, n_it, screened, exact, 0u, valid, {0u, 0u, 0u}};
+            full_direct(&A, el, smem_u32(coef), pend, &s_pend_n, ts, &d);
+            st = d.st;
+            item = d.item;
+            left = d.left;
+            n_it = d.n_it;
+            screened = d.screened;
+            exact = d.exact;
+            valid = d.valid;
+            has_def = d.n_def != 0u;
+            def = d.def;
+            continue;
+        }
         uint32_t passed = 0, seen = 0;
 #pragma unroll 1
-        for (int r = 0; r < kFtRounds; ++r) {
+        for (int r = r0; r < kFtRounds; ++r) {
             const bool act = valid && !has_def;
             const uint64_t s0 = st;
             const PairHead h = pair_head(A.sc, pow2, s0);

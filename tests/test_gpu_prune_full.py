@@ -61,3 +61,25 @@ def test_full_prune_ties_and_stream_ranges(monkeypatch):
     for k in ([0, 1], [1, 3]):
         _both(monkeypatch, w * 0 + rng.normal(0, 1, 465).astype(np.float32), el, 600_001, 80, streams=tuple(k))
     _both(monkeypatch, np.zeros(465, np.float32), el, 100_001, 30)
+
+
+@pytest.mark.parametrize("ne", [2, 40])
+def test_full_prune_backs_off(monkeypatch, ne):
+    """A surface that the bound is used for (its slack is within the limit of
+    its spread over uniform genes), elites that are alike, and nothing but
+    crossover and mutation: the bound of every candidate is the elites' score
+    and the slack, above every score there is, so each round that computes it
+    leaves everything. 1.5e8 candidates are some 80 rounds of 456 CTAs: past the
+    sixteenth that leaves more than half, and into the longer pauses."""
+    from codec_arena_gb300 import _lib, screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    m = screen.ModelFull.from_compact(wl.seeded_normal_model(seed=3, n=465))
+    el = wl.seeded_elites(ne, seed=4)
+    el["g"] = el["g"][0]
+    lam, kw = 150_000_001, dict(threads=3, imm_p=0.0, jump_p=0.0)
+    got, n = screen.screen(screen.Cfg(lam, 60, 11, flags=_lib.FLAG_STAGE_TIMES, **kw), m, el)
+    evals = screen.last_run_info()["exact_evals"]  # the unpruned kernel counts none
+    ref, nr = screen.screen(screen.Cfg(lam, 60, 11, flags=_lib.FLAG_NO_PRUNE, **kw), m, el)
+    assert n == nr == lam and got.tobytes() == ref.tobytes()
+    assert evals > 0.99 * lam
