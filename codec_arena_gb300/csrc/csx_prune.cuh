@@ -53,6 +53,11 @@ constexpr int kPruneMs = 3;  // order statistics each CTA publishes (publish_fir
 // merges of a non-empty buffer.
 constexpr int kPruneRounds = 64;
 constexpr uint32_t kPruneMergeRounds = 4;
+// Rounds without the bounds (screen_p_kernel): a warp whose CTA's queue is full
+// within kPruneQuick candidates per thread was left a third or more of them; a
+// round without is 2^1 .. 2^(kPruneDirect - 1) candidates per thread.
+constexpr int kPruneQuick = 6;
+constexpr uint32_t kPruneDirect = 8;
 // kGolden's inverse modulo 2^64: a draw offset back from its state.
 constexpr uint64_t golden_inverse() {
     uint64_t x = kGolden;  // correct to 3 bits; each Newton step doubles them
@@ -104,6 +109,14 @@ __device__ __forceinline__ float prune_rescore(const ScreenArgs *__restrict__ A,
                                                uint64_t p, float tlo) {
     if (!kFp64) return exact_score_at<true>(A, el, seed_t, p);
     return prune_rescore64(A, el, seed_t, p, tlo);
+}
+
+// The filter's score of one candidate, its jump applied (within ScreenArgs::err of
+// the real score), out of line: for the rounds that score without the bounds.
+__device__ __noinline__ float filter_score_at(const ScreenArgs *__restrict__ A, const float *el, uint64_t seed_t,
+                                              uint64_t p) {
+    const CandHead h = cand_head(A->sc, seed_t, p);
+    return synth_score<true, false, false, DevModel, true>(A->m, A->sc, el, seed_t, p, h, nullptr);
 }
 
 // The j-th largest (1-based) of v[0..n), by one warp (every lane calls):
@@ -459,6 +472,18 @@ __device__ __forceinline__ float prune_bound(const PruneArgs &A, const uint32_t 
 // covers the rounding of those scores too) -- instead of the reference's f32
 // order.
 // kFar: the box table stays in global memory (prune_bx_smem).
+// Rounds without the bounds. Elites that are alike and score near the top (a run
+// that screens its own survivors) leave the bounds little to rule out: every
+// crossover of theirs lies within its mutation box of the threshold. The f32
+// order's form then costs the bounds and the queue, 117 ms of 1e9 candidates
+// where the unpruned kernel takes 32. So where most of a CTA's warps fill the
+// queue at once (kPruneQuick) in two rounds in a row, each such round is followed
+// by one that scores by the filter alone and queues what may reach the threshold, up to
+// 128 candidates per thread: 46 ms (bounds that leave a third: 88 -> 46; 3e7
+// candidates 4.2 -> 2.05). On elites of full spread nothing changed (2.65e9 22.3
+// ms, 1e8 1.36). The FP64 form keeps its queue (the bounds cost it less beside its
+// scores: 35 ms of 3e8 where its unpruned kernel takes 17 to 29; with these rounds
+// 14, but 11.0 ms instead of 10.7 at 1e9 on elites of full spread).
 template <bool kTail, bool kFp64, bool kFar>
 __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_constant__ PruneArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -473,6 +498,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     uint32_t *bm = bx + (kFar ? 0u : A.sc.ne * 17);
     uint32_t *sel = bm + A.bm_words;
     __shared__ unsigned int s_buf_n, s_pend_n;
+    __shared__ uint32_t s_quick, s_fails, s_direct;
     __shared__ unsigned long long s_t1, s_t2;
     __shared__ float s_ts;
 
@@ -487,6 +513,7 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
     if (tid == 0) {
         s_buf_n = 0;
         s_pend_n = 0;
+        s_quick = s_fails = s_direct = 0;
         s_t1 = 0;
         s_t2 = 0;
         s_ts = -INFINITY;
@@ -558,6 +585,16 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
         __syncthreads();
         const unsigned int pn = min(s_pend_n, kPendCap);
         unsigned int bn = s_buf_n;  // nobody appends until after the next barrier
+        if (!kFp64 && tid == 0) {  // whether the next round scores without the bounds (read behind the barriers below)
+            const bool fail = s_quick > kThreads / 64 && (s_t1 != 0ull || gk != 0u);
+            if (s_direct != 0u) {
+                s_direct = 0;  // never two in a row: the rounds with the bounds drain the warps' queues
+            } else {
+                s_fails = fail ? min(s_fails + 1u, kPruneDirect) : 0u;
+                s_direct = s_fails >= 2u ? 1u << (s_fails - 1u) : 0u;
+            }
+            s_quick = 0;
+        }
         const int any = __syncthreads_or(valid || n_def > 0 || n1 + n2 > 0);
         const int any_def = __syncthreads_or(n_def > 0);
         // the queue is evaluated once it can employ every thread (or a thread
@@ -597,6 +634,30 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
             __syncwarp();
         }
         ++round;
+        if (const uint32_t cnt = kFp64 ? 0u : s_direct; cnt != 0u && ts > -INFINITY) {
+            const float td = __fsub_rd(ts, A.err);
+#pragma unroll 1
+            for (uint32_t i = 0; i < cnt && valid && n_def == 0; ++i) {
+                const Item it = A.items[item];
+                const uint64_t seed_t = stream_seed(A.seed, it.stream);
+                const uint64_t p = (st - seed_t) * kGoldenInv - 1;
+                if (!(filter_score_at(&A, el, seed_t, p) < td)) {
+                    const Pend q{item, n_it - left, static_cast<uint32_t>(p - it.draw0)};
+                    const unsigned int ps = atomicAdd(&s_pend_n, 1u);
+                    if (ps < kPendCap) {
+                        pend[ps] = q;
+                    } else {
+                        def[0] = q;
+                        n_def = 1;
+                    }
+                }
+                const bool imm = (draw_vh(st + 2 * kGolden) >> 8) < A.sc.imm_thr;
+                const uint64_t sj = st + (imm ? 32u : 61u) * kGolden;
+                st = sj + (((draw_vh(sj) >> 8) < A.sc.jump_thr) ? 3u : 1u) * kGolden;
+                if (--left == 0) next_item();
+            }
+            continue;
+        }
 #pragma unroll 1
         for (int rr = 0; rr < kPruneRounds; ++rr) {
             const uint64_t s0 = st;
@@ -652,7 +713,10 @@ __global__ void __launch_bounds__(kThreads, 3) screen_p_kernel(const __grid_cons
                     if (!(f < tlo)) push(q, wq.i2[n2 + lane]);  // NaN: scored
                 }
             }
-            if (__any_sync(0xffffffffu, n_def > 0)) break;
+            if (__any_sync(0xffffffffu, n_def > 0)) {
+                if (!kFp64 && lane == 0 && rr < kPruneQuick) atomicAdd(&s_quick, 1u);
+                break;
+            }
         }
     }
     Entry *out = A.lists + static_cast<size_t>(blockIdx.x) * A.kpad;

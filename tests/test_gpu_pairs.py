@@ -150,3 +150,28 @@ def test_long_lists_share_a_threshold(monkeypatch, keep, nf):
     ref, _ = screen.screen(screen.Cfg(50_000_000, keep, 3, threads=4, flags=_lib.FLAG_NO_PRUNE), m, el)
     assert n == 50_000_000 and got.tobytes() == ref.tobytes()
     assert evals < 0.2 * n, evals / n
+
+
+@pytest.mark.parametrize("nf,ne,kw", [(161, 64, {}), (161, 2, {"imm_p": 0.0, "jump_p": 1.0}), (166, 33, {"imm_p": 0.0}),
+                                      (153, 300, {"imm_p": 0.5}), (161, 40, {"imm_p": 1.0})])
+@pytest.mark.parametrize("lam,keep", [(400_001, 7), (30_000_001, 192)])
+def test_bounds_that_rule_out_nothing(monkeypatch, nf, ne, kw, lam, keep):
+    """Elites that are alike and at the top (and candidates that are always
+    scored): most rounds score without the bounds, each candidate once, instead of
+    queueing nearly all of them."""
+    from codec_arena_gb300 import _lib, screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    m = screen.Model.from_compact(wl.surrogate_161() if nf == 161 else wl.seeded_normal_model(seed=8, n=nf))
+    el = wl.seeded_elites(max(ne, 64), seed=2)
+    for gen in range(3):
+        top, _ = screen.screen(screen.Cfg(2_000_000, 64, gen, threads=4), m, el)
+        el["g"][:64] = top["g"]
+    el = el[:ne].copy()
+    el["g"] = top["g"][0] + 0.01 * np.random.default_rng(1).random((ne, 29), dtype=np.float32)
+    got, n = screen.screen(screen.Cfg(lam, keep, 3, threads=3, sigma=0.07, flags=_lib.FLAG_STAGE_TIMES, **kw), m, el)
+    evals = screen.last_run_info()["exact_evals"]
+    ref, _ = screen.screen(screen.Cfg(lam, keep, 3, threads=3, sigma=0.07, flags=_lib.FLAG_NO_PRUNE, **kw), m, el)
+    assert n == lam and got.tobytes() == ref.tobytes()
+    if lam > 1e7:
+        assert evals < 0.3 * n, evals / n
