@@ -1089,7 +1089,7 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
     if (full) F.fm = make_full_model(*full);
     const unsigned int cap = 1u << 20;
     CSX_CUDA(cx.tie_hits.ensure(static_cast<size_t>(cap) * sizeof(TieHit)));
-    CSX_CUDA(cx.tie_count.ensure(sizeof(unsigned int)));
+    CSX_CUDA(cx.tie_count.ensure(2 * sizeof(unsigned int)));
     auto *d_hits = static_cast<TieHit *>(cx.tie_hits.p);
     auto *d_count = static_cast<unsigned int *>(cx.tie_count.p);
     const int blocks = static_cast<int>(std::min<uint64_t>((n_items + 255) / 256, 32ull * cx.num_sms));
@@ -1100,13 +1100,13 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
         const uint64_t n_t = (t == g.T - 1) ? g.my_last : g.per;
         std::vector<TieHit> &h = heaps[t];
         uint64_t lo = 0, size = std::max<uint64_t>(4 * K, 1024);
-        bool all = true;
+        bool all = true, tables = bufs.pairs.box && pl.prune_ok;
         float thr = -INFINITY;
         while (lo < n_t) {
             const uint64_t hi = std::min(n_t, lo + size);
-            CSX_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));
+            CSX_CUDA(cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned int), st));
             const uint32_t ts = static_cast<uint32_t>(t);
-            if (!all && bufs.pairs.box && pl.prune_ok) {
+            if (!all && tables) {
                 tie_collect_pruned_kernel<<<blocks, 256, 0, st>>>(prune_args(A, model, pl, bufs.pairs, nullptr),
                                                                   n_items, ts, lo, hi, thr, d_hits, d_count, cap);
             } else if (full) {
@@ -1121,9 +1121,10 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
                     tie_collect_kernel<false><<<blocks, 256, 0, st>>>(A, n_items, ts, lo, hi, thr, all, d_hits, d_count, cap);
             }
             CSX_CUDA(cudaGetLastError());
-            unsigned int n = 0;
-            CSX_CUDA(cudaMemcpyAsync(&n, d_count, sizeof(n), cudaMemcpyDeviceToHost, st));
+            unsigned int got[2] = {0, 0};
+            CSX_CUDA(cudaMemcpyAsync(got, d_count, sizeof(got), cudaMemcpyDeviceToHost, st));
             CSX_CUDA(cudaStreamSynchronize(st));
+            const unsigned int n = got[0];
             if (n > cap) {  // too many above the root in this chunk: read it in halves
                 size = std::max<uint64_t>(1, (hi - lo) / 2);
                 continue;
@@ -1139,6 +1140,8 @@ int fix_ties(Context &cx, const csx_cfg &cfg, const csx_model &model, const csx_
                 all = false;
                 thr = h[0].score;
             }
+            // a chunk whose root has settled and of which the tables left most: the others without them
+            if (hi - lo >= (1u << 18) && 2ull * got[1] > hi - lo) tables = false;
             lo = hi;
             size *= 2;
         }

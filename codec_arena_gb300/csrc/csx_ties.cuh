@@ -57,7 +57,10 @@ __global__ void tie_collect_kernel(const __grid_constant__ Args A, uint64_t n_it
 // The same for a generation the pruning screen ran, whose pair tables are still
 // there: only candidates that the pair's and the mask's bounds leave a chance
 // above thr are scored, a warp's worth at a time. Scoring every candidate of a
-// stream took 12.3 ms where a 2.65e9 generation held one tie.
+// stream took 12.3 ms where a 2.65e9 generation held one tie. count[0]: hits;
+// count[1]: candidates scored (where that is most of a chunk, the host goes on
+// without the tables: elites that are alike and near the top, 1e9 candidates
+// replayed in 97 ms with them throughout, 72 so).
 constexpr uint32_t kTieQueue = 64;
 
 __global__ void __launch_bounds__(256) tie_collect_pruned_kernel(const __grid_constant__ PruneArgs A, uint64_t n_items,
@@ -71,9 +74,11 @@ __global__ void __launch_bounds__(256) tie_collect_pruned_kernel(const __grid_co
     const bool pow2 = (A.sc.ne & (A.sc.ne - 1)) == 0;
     const float tlo = __fsub_rd(thr, A.pc.err);
     uint32_t n1 = 0, n2 = 0;  // queued after the pair's test (q), after the mask's (r)
+    uint32_t scored = 0;      // by this lane
     auto score = [&](uint64_t st, uint64_t idx) {
         const uint64_t p = (st - seed_t) * kGoldenInv - 1;
         const float s = exact_score_at<true>(&A, A.el, seed_t, p);
+        ++scored;
         if (s > thr) {
             const unsigned int slot = atomicAdd(count, 1u);
             if (slot < cap) out[slot] = TieHit{idx, p, s, 0u};
@@ -144,6 +149,8 @@ __global__ void __launch_bounds__(256) tie_collect_pruned_kernel(const __grid_co
         }
     }
     drain(true);
+    scored = __reduce_add_sync(0xffffffffu, scored);
+    if (lane == 0 && scored) atomicAdd(count + 1, scored);
 }
 
 // Survivor records of the candidates at (stream, draw, index): genes and

@@ -175,3 +175,27 @@ def test_bounds_that_rule_out_nothing(monkeypatch, nf, ne, kw, lam, keep):
     assert n == lam and got.tobytes() == ref.tobytes()
     if lam > 1e7:
         assert evals < 0.3 * n, evals / n
+
+
+@pytest.mark.parametrize("nf", [161, 465])
+def test_tie_replay_where_the_tables_rule_out_nothing(orc, monkeypatch, nf):
+    """Elites of one genome at 0 and 1 and no mutation: every crossover candidate
+    ties with the best, so that the replay's tables leave whole chunks and the later
+    ones are read without them (a stream of 1e6 has chunks past 2^18)."""
+    import os
+
+    from codec_arena_gb300 import _lib, screen, workloads as wl
+
+    monkeypatch.setenv("CSX_PRUNE_MIN_CANDS", "0")
+    w = np.random.default_rng(4).integers(-2, 3, nf).astype(np.float32)
+    el = wl.seeded_elites(12, seed=2)
+    el["g"] = np.round(el["g"][0])
+    kw = dict(threads=2, sigma=0.0, jump_p=0.1, imm_p=0.05)
+    m = (screen.ModelFull if nf == 465 else screen.Model).from_compact(w)
+    got, n = screen.screen(screen.Cfg(2_000_001, 50, 9, **kw), m, el)
+    ref, _ = screen.screen(screen.Cfg(2_000_001, 50, 9, flags=_lib.FLAG_NO_PRUNE, **kw), m, el)
+    assert n == 2_000_001 and got.tobytes() == ref.tobytes()
+    if nf == 161:
+        want, _ = orc.screen(orc.cfg(2_000_001, 50, 9, **kw), orc.model_from_compact(w), el,
+                             cpu_threads=os.cpu_count() or 4)
+        assert got.tobytes() == want.tobytes()
