@@ -660,7 +660,7 @@ def refit_full(args, timed, dfma):
     cpu_s = time.perf_counter() - t0
     gram_flop = 2.0 * n * (nf * (nf + 1) / 2 + nf)
     return {"rows": n, "features": nf, "alpha": alpha, "ms": ms_refit,
-            "stages_ms": {"normal_equations": ms_gram, "cholesky_solve": ms_solve},
+            "stages_ms": {"normal_equations": ms_gram, "solve": ms_solve},
             "roofline": {"bound": "fp64", "kernel": "sg_gram_kernel", "achieved": gram_flop / (ms_gram * 1e-3) / 1e12,
                          "peak": 2 * dfma / 1e12, "unit": "TFLOP/s",
                          "frac": gram_flop / (ms_gram * 1e-3) / (2 * dfma) if dfma else None},

@@ -1,5 +1,5 @@
 // The quadratic surrogate as a differentiable function: forward, backward,
-// the ridge refit's normal equations, an FP64 solve (LDL' or Cholesky) and a
+// the ridge refit's normal equations, an FP64 solve (LDL') and a
 // gradient-ascent mutation step (include/csx_surrogate.h).
 //
 // Reference: brain/evolve.py:211-220 (features: [1 | genes | g_i g_j, j <= i
@@ -7,10 +7,10 @@
 // solve); src/screen.zig:97-112 (the screen's score of the same features).
 //
 // Work sizes are small next to the screen: a refit table of 400,000 rows of
-// 16 genes is 25.6 MB. The normal equations (nf(nf+1)/2 products per row, to
-// FP64) run on the tensor cores in exact fixed point (csx_gram.cuh), those of
-// the full surface on the FP64 pipe; everything else is a few hundred FP32
-// FMAs per row.
+// 16 genes is 25.6 MB. The normal equations (nf(nf+1)/2 products per row) run on
+// the tensor cores in fixed point (csx_gram.cuh), those of the full surface, and
+// of tables for which FP64 sums are closer, on the FP64 pipe; everything else is
+// a few hundred FP32 FMAs per row.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -5,9 +5,9 @@ ridge refit (include/csx_surrogate.h).
 hand-written kernels: d score / d genes (for gradient-guided mutation) and
 d loss / d coefficients (FP64 accumulation). `refit` replaces
 brain/evolve.py:250-268 (`refit_surrogate`): it forms the normal equations
-ΦᵀΦ and Φᵀy in FP64 on the GPU (in exact fixed point on the tensor cores, or
-FP64 sums) and solves (ΦᵀΦ + αI) w = Φᵀy + α w₀ by an FP64 LDLᵀ factorisation
-on a cluster of CTAs (Cholesky on one for 465 coefficients). `ridge_grad` is the ridge loss
+ΦᵀΦ and Φᵀy in FP64 on the GPU (in fixed point on the tensor cores where that
+is as close as FP64 sums, else by those) and solves (ΦᵀΦ + αI) w = Φᵀy + α w₀ by
+an FP64 LDLᵀ factorisation on a cluster of CTAs. `ridge_grad` is the ridge loss
 gradient 2Φᵀ(Φw − y) + 2α(w − w₀) from the backward kernel, which vanishes
 at the solution.
 
@@ -137,8 +137,8 @@ def normal_equations(genes: torch.Tensor, fit: Optional[torch.Tensor], nf: int):
 
 
 def ridge_solve(gram: torch.Tensor, rhs: torch.Tensor, alpha: float, prior: Optional[torch.Tensor] = None):
-    """w = (G + αI)⁻¹ (rhs + α·prior) in FP64: LDLᵀ on a cluster of CTAs up to
-    166 coefficients, Cholesky on one CTA (the factor in a global scratch) for 465."""
+    """w = (G + αI)⁻¹ (rhs + α·prior) in FP64: LDLᵀ on a cluster of
+    eight CTAs, its rows in their shared memory (every layout)."""
     nf = gram.shape[0]
     dev = gram.device
     gram = gram.to(torch.float64).contiguous()

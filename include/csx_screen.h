@@ -246,7 +246,7 @@ typedef struct csx_run_info {
     float ms_merge;         /* top-K merge tree */
     float ms_regen;         /* survivor regeneration */
     float ms_total;
-    uint64_t exact_evals;   /* candidates scored in the reference order (filter mode) */
+    uint64_t exact_evals;   /* candidates scored in the reference order (filter mode, pruning screens) */
 } csx_run_info;
 int csx_last_run_info(csx_run_info *out);
 
@@ -255,7 +255,7 @@ int csx_last_run_info(csx_run_info *out);
  * running brain/evolve.py with its own seed, elites and surrogate,
  * .github/workflows/arena.yml:56-92) in one pipeline: every island's work
  * items are built on its own forked stream; then, when every island's
- * surrogate admits the pruning bound and every island is above
+ * surrogate admits the pruning bound and their mean budget is above
  * the pruning floor (CSX_FLAG_NO_PRUNE), each island's pruning screen runs
  * over the whole GPU, else (or when any island carries
  * CSX_FLAG_NO_PRUNE) ONE unpruned persistent screen launch consumes all
